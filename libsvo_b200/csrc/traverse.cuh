@@ -19,9 +19,8 @@
 //     push it was set to the pushed child's tcMax, which is the child frame's
 //     tMax and never changes afterwards; so on a pop tMin := popped tMax;
 //   - node centres are exact dyadic numbers (-0.5 + (2i+1) 2^-(k+1) for a
-//     depth-k node with lattice coordinate i): a child's centre is its
-//     parent's +- half the child size, so a pop recovers the parent's centre
-//     exactly from the child's and the low bit of the lattice coordinate.
+//     depth-k node with lattice coordinate i), so any ancestor's centre is a
+//     prefix of the bits of a node's own (ancestor_center).
 // The stack lives in shared memory, one 8-byte word per level per thread,
 // laid out [level][thread] so a warp's accesses are contiguous.
 #pragma once
@@ -51,6 +50,7 @@ struct RayHit {
   // SampleResult.nodeCenter: the hit child's centre, or the current node's
   // when the watchdog ends the ray (shadow rays start there)
   float cx, cy, cz;
+  float t_enter, t_exit;  // the root box (both 0 when the ray misses it)
 };
 
 __device__ __forceinline__ float cl_max(float a, float b) { return (a < b) ? b : a; }
@@ -110,105 +110,226 @@ struct StagedFetch {
   }
 };
 
-// A saved traversal state for the cycle search of very long rays (descend):
-// frame node, scale and tMin bits, the stacked frames, and the loop and fetch
-// counts when it was saved.  Lives in local memory (volatile, so the hot
-// loop's registers are not spent on it); only rays that run kCycleFrom
-// iterations or more touch it -- on the 1080p icosphere frame the 8 rays the
-// watchdog stops, which otherwise run alone for 980 iterations after the rest
-// of the frame is done (a search from iteration 64 or 256 made the many long
-// rays below 512 pay for the checks and the frame slower).
-constexpr uint32_t kCycleFrom = 512;
+// A saved traversal state for the cycle search of rays that do not advance
+// (descend_general): frame node, size and tMin bits, the stacked frames, and
+// the loop and fetch counts when it was saved.  Lives in local memory
+// (volatile, so no registers are spent on it).
+constexpr uint32_t kSearchFrom = 128;  // rays that run descend_general from the root
+constexpr uint32_t kFirstGap = 32;
 struct CycleMark {
-  uint32_t node, scale, tmin, loops, fetches, next_save;
+  uint32_t node, size, tmin, loops, fetches, next_save, gap;
   uint32_t stack[2 * kMaxStack];
 };
 
-// The descent loop.  kFlat selects the CpuRaycasterSingleRay3 rules; S is
-// the stack size (treelet) or the octree depth (flat).  `stack` points at
-// this thread's column of the shared-memory stack, `stride` words apart.
-//
-// Per frame (set on push and pop) the registers hold the node, its tMin and
-// tMax, its centre, the child size sx2 and half of it, and the node record,
-// which is loaded as soon as the node is known so the load overlaps the
-// entry-point arithmetic of the next iteration.
-//
-// kSigned: the reference orders each child's slab distances with a compare
-// and swap (tx0 > tx1).  When the reciprocal r is finite, rounding is
-// monotone, so the swap happens exactly when r < 0 (equal values swap to
-// themselves): the near face is lo when r > 0 and hi when r < 0.  A child's
-// two faces along an axis are the parent's mid plane c and its outer face
-// c +- sx2 (exact dyadic numbers, the values the reference's childCenter +-
-// childSizeHalf produce), so each axis costs the distance to the mid plane,
-// the distance to the outer face and the max of the two (the far face); the
-// min (the near face) is taken only for a valid child, the one case that
-// reads tcMin.  Rays with an infinite or NaN reciprocal (a direction
-// component of exactly zero) or a -0 origin coordinate (see cast_ray) take
-// kSigned = false, the literal compare and swap.
-template <bool kFlat, bool kSigned, class Fetch>
-__device__ __forceinline__ void descend(const Fetch& fetch, uint64_t num_nodes,
-                                        const float o[3], float dx, float dy, float dz, float rx,
-                                        float px, float ry, float py, float rz, float pz,
-                                        float t_min, float t_max, float tsr, int S, uint2* stack,
-                                        int stride, RayHit& h, uint32_t loop_cap) {
+// Bit 31 set exactly when pos > c.  The sign of c - pos says so: with
+// subnormals the difference rounds to zero only when the two are equal, x - x
+// is +0, and a NaN the hardware produces is positive (the comparison is false).
+__device__ __forceinline__ uint32_t above(float pos, float c) {
+#if defined(__CUDACC__)
+  return __float_as_uint(__fsub_rn(c, pos));
+#else
+  return pos > c ? 0x80000000u : 0u;
+#endif
+}
+
+// v with the sign that `above` gives: v where bit 31 is set, else -v.  v > 0.
+__device__ __forceinline__ float with_side(uint32_t side, float v) {
+  return __uint_as_float((~side & 0x80000000u) | __float_as_uint(v));
+}
+
+// (acc << 1) | bit 31 of side: one funnel shift.
+__device__ __forceinline__ uint32_t shift_in(uint32_t acc, uint32_t side) {
+#if defined(__CUDACC__)
+  return __funnelshift_l(side, acc, 1);
+#else
+  return (acc << 1) | (side >> 31);
+#endif
+}
+
+// The centre coordinate of the ancestor at the level whose child size is sx2,
+// from a descendant's: as c + 1.5, in [1, 2), the coordinate's fraction is the
+// lattice coordinate in fixed point, so the ancestor's is its leading bits with
+// the bit of weight sx2 set (one = the bits of 1 + sx2, keep = the mask of the
+// bits above).  The sum is rounded down: the one centre that needs 24 bits
+// (depth 23) then loses a bit below those that are kept.
+__device__ __forceinline__ float ancestor_center(float c, uint32_t one, uint32_t keep) {
+#if defined(__CUDACC__)
+  const uint32_t x = __float_as_uint(__fadd_rz(c, 1.5f));
+#else
+  const uint32_t x = 0x3f800000u | (uint32_t)(int32_t)(((double)c + 0.5) * 8388608.0);
+#endif
+  return __fadd_rn(__uint_as_float((x & keep) | one), -1.5f);
+}
+
+// Where a ray stands between two iterations of the reference: its frame (node,
+// interval, centre, child size: 2^-(k+1) at depth k) and what it has counted.
+struct RayState {
+  uint32_t node;
+  float tmin, tmax, cx, cy, cz, sx2;
+  uint32_t loops, fetches;
+};
+
+// The ray against the root box, set up once per ray.
+struct Ray {
+  float ox, oy, oz, dx, dy, dz;  // origin, clamped direction
+  float rx, ry, rz, px, py, pz;  // 1 / d and -o / d
+  float t_max, tsr;              // exit from the root box, tScaleRatio
+};
+
+// The frame's level counted as the reference's S - scale: 1 at the root.
+__device__ __forceinline__ uint32_t level_of(float sx2) {
+  return 127u - (__float_as_uint(sx2) >> 23);
+}
+
+// The reference's pop test.
+template <bool kFlat>
+__device__ __forceinline__ bool interval_done(float tmin, float tmax) {
+  const float eps = 0.00001f;
+  if (kFlat) return (tmax < 0.0f) || (fabsf(__fsub_rn(tmin, tmax)) < eps) || !(tmin < tmax);
+  return (tmax < 0.0f) || !(fabsf(__fsub_rn(tmin, tmax)) > eps);
+}
+
+// The child size at which the treelet rules stop (the reference's scale 1) or,
+// in a flat pool, below which no child may be an inner node (scale 0).
+template <bool kFlat>
+__device__ __forceinline__ float last_size(int S) {
+  return pow2i(kFlat ? -S : 1 - S);
+}
+
+__device__ __forceinline__ void ray_missed(bool flat, const Ray& r, uint32_t loops,
+                                           uint32_t fetches, RayHit& h) {
+  h.hit = 0u;
+  h.node = 0u;
+  h.depth = 0u;
+  h.t = flat ? 0.0f : r.t_max;
+  h.loops = loops;
+  h.fetches = fetches;
+}
+
+// The reference's loop as it is written, from any state on: every frame is
+// stacked, a child's slab distances are compared and swapped, and the watchdog
+// is looked at in every iteration.  Rays that `descend` cannot take (an
+// infinite reciprocal, an origin that is not finite, or -0: see cast_ray) run it from
+// the root, and those that stop advancing or come near the watchdog finish in
+// it.  A pass is one child test and the pops that follow it.
+template <bool kFlat, class Fetch>
+__device__ __forceinline__ void descend_general(const Fetch& fetch, uint64_t num_nodes,
+                                                const Ray& r, int S, uint2* stack, int stride,
+                                                const RayState& from, RayHit& h,
+                                                uint32_t loop_cap) {
   const float eps = 0.00001f;
   // the reference's watchdog, or the caller's smaller cap (cost estimates)
   const uint32_t watchdog = (uint32_t)((S + 1) * (S + 1) * 5);
   const uint32_t max_loops = loop_cap && loop_cap < watchdog ? loop_cap : watchdog;
-  int scale = S - 1;
+  const float sx2_last = last_size<kFlat>(S);
+  const uint32_t last_node = num_nodes ? (uint32_t)(num_nodes - 1u) : 0u;
   uint32_t node = 0u;
-  float tmin = t_min, tmax = t_max;
-  uint32_t ix = 0u, iy = 0u, iz = 0u;  // lattice coordinate at depth S-1-scale
+  float tmin = from.tmin, tmax = r.t_max;
   float cx = 0.0f, cy = 0.0f, cz = 0.0f;
-  float sx2 = 0.5f, half = 0.25f;
+  float sx2 = 0.5f;
+  uint32_t loops = from.loops, fetches = from.fetches;
+  uint2* sp = stack;  // the next free stack word
   bool in_pool = num_nodes > 0u;
   uint2 nd = in_pool ? fetch(0u) : make_uint2(0u, 0u);
-  uint32_t loops = 0u, fetches = 0u;
-  // pools hold at most 2^32 nodes, so the in-pool test of a 32-bit index is
-  // one 32-bit compare against the last index
-  const uint32_t last_node = num_nodes ? (uint32_t)(num_nodes - 1u) : 0u;
-  uint2* sp = stack;  // the next free stack word: level S-1-scale
-  uint32_t check_at = max_loops < kCycleFrom ? max_loops : kCycleFrom;
+  // the first iteration of the cycle search
+  const uint32_t search_from = from.loops ? from.loops + 1u : kSearchFrom;
+  uint32_t check_at = max_loops < search_from ? max_loops : search_from;
   volatile CycleMark mark;
+  mark.loops = 0u;  // none saved
+  mark.next_save = search_from;
+  mark.gap = kFirstGap;
+
+  uint32_t ci = 0u;            // the child on the given side of the centre,
+  float tc_min, tc_max, half;  // its slab and half size
+  auto slab = [&](uint32_t bx, uint32_t by, uint32_t bz) {
+    ci = shift_in(shift_in(bx >> 31, by), bz);
+    half = __fmul_rn(sx2, 0.5f);
+    // child centre (-0.5 + b) * sx2 + c = c +- half; faces ccx -+ half
+    const float ccx = __fadd_rn(with_side(bx, half), cx);
+    const float ccy = __fadd_rn(with_side(by, half), cy);
+    const float ccz = __fadd_rn(with_side(bz, half), cz);
+    float tx0 = __fadd_rn(__fmul_rn(r.rx, __fsub_rn(ccx, half)), r.px);
+    float tx1 = __fadd_rn(__fmul_rn(r.rx, __fadd_rn(ccx, half)), r.px);
+    if (tx0 > tx1) {
+      const float s = tx0;
+      tx0 = tx1;
+      tx1 = s;
+    }
+    float ty0 = __fadd_rn(__fmul_rn(r.ry, __fsub_rn(ccy, half)), r.py);
+    float ty1 = __fadd_rn(__fmul_rn(r.ry, __fadd_rn(ccy, half)), r.py);
+    if (ty0 > ty1) {
+      const float s = ty0;
+      ty0 = ty1;
+      ty1 = s;
+    }
+    float tz0 = __fadd_rn(__fmul_rn(r.rz, __fsub_rn(ccz, half)), r.pz);
+    float tz1 = __fadd_rn(__fmul_rn(r.rz, __fadd_rn(ccz, half)), r.pz);
+    if (tz0 > tz1) {
+      const float s = tz0;
+      tz0 = tz1;
+      tz1 = s;
+    }
+    tc_min = cl_max(tx0, cl_max(ty0, tz0));
+    tc_max = cl_min(tx1, cl_min(ty1, tz1));
+  };
+  auto push = [&](uint32_t bx, uint32_t by, uint32_t bz) {
+    *sp = make_uint2(node, __float_as_uint(tmax));
+    sp += stride;
+    node = (kFlat ? 0u : node) + nd.x + __popc(nd.y & ((0x100u << ci) - 0x100u));
+    in_pool = node <= last_node;
+    if (in_pool) nd = fetch(node);
+    tmax = tc_max;
+    cx = __fadd_rn(with_side(bx, half), cx);
+    cy = __fadd_rn(with_side(by, half), cy);
+    cz = __fadd_rn(with_side(bz, half), cz);
+    sx2 = half;
+  };
+  // the frames above the given one: a frame's interval end depends only on its
+  // box and the ray, so they are pushed again from the root
+  while (sx2 != from.sx2) {
+    const uint32_t bx = above(from.cx, cx), by = above(from.cy, cy), bz = above(from.cz, cz);
+    slab(bx, by, bz);
+    push(bx, by, bz);
+  }
+
   auto capped = [&]() {
     h.flags = SVO_HITFLAG_CAPPED;
     h.loops = loops;
     h.fetches = fetches;
+    h.tc_min = tmin;
     if (!kFlat) {  // sample() reports the current node as a hit (:268-277)
       h.hit = 1u;
       h.node = node;
-      h.depth = (uint32_t)(S - scale);
+      h.depth = level_of(sx2);
       h.t = tmin;
       h.cx = cx;
       h.cy = cy;
       h.cz = cz;
       // quality = scale_exp2 - tScaleRatio * tMin, as for a leaf
-      h.tc_min = tmin;
       h.sx2 = sx2;
       h.leaf = 1u;
     }
   };
 
-  for (;;) {  // ends by a return, or by a pop above the root
+  bool pop = interval_done<kFlat>(tmin, tmax);  // whether the next iteration pops
+  for (;;) {                                    // ends by a return
     ++loops;
     if (loops >= check_at) {
-      if (loops == max_loops) {
+      if (loops >= max_loops) {
         capped();
         return;
       }
-      // Cold path (rays past kCycleFrom iterations only).  The state at the
-      // start of an iteration is the frame's node, scale and tMin and the
-      // stacked frames: a frame's tMax depends only on its box and the ray,
-      // and the box on the nodes stacked above it.  Once that state recurs,
-      // the ray repeats the same iterations with period p until the
-      // watchdog, so whole periods are skipped (loop and fetch counts
-      // advanced by them) and the iterations left run as usual: the watchdog
-      // then stops the ray in the state, and with the counts, the reference
-      // reaches.  States are saved at iterations kCycleFrom, 2 kCycleFrom, ...
-      // (Brent's cycle search) and compared with every later iteration.
-      check_at = loops + 1u;
-      const uint32_t depth = (uint32_t)(S - 1 - scale);
-      bool same = loops > kCycleFrom && mark.node == node && mark.scale == (uint32_t)scale &&
+      // The state at the start of an iteration is the frame's node, size and
+      // tMin and the stacked frames.  Once that state recurs, the ray repeats
+      // the same iterations with period p until the watchdog, so whole periods
+      // are skipped (loop and fetch counts advanced by them) and the
+      // iterations left run as usual: the watchdog then stops the ray in the
+      // state, and with the counts, the reference reaches.  Every iteration is
+      // compared with a saved state, which is replaced after 32, 64, 128, ...
+      // of them (Brent's cycle search); check_at = loops + 1 keeps a pass to one
+      // iteration meanwhile.
+      const uint32_t depth = level_of(sx2) - 1u;
+      bool same = mark.loops != 0u && mark.node == node && mark.size == __float_as_uint(sx2) &&
                   mark.tmin == __float_as_uint(tmin);
       for (uint32_t j = 0; same && j < depth; ++j) {
         const uint2 a = stack[j * stride];
@@ -224,183 +345,284 @@ __device__ __forceinline__ void descend(const Fetch& fetch, uint64_t num_nodes,
           capped();
           return;
         }
-      } else if (loops == kCycleFrom || loops == mark.next_save) {
-        mark.node = node;
-        mark.scale = (uint32_t)scale;
-        mark.tmin = __float_as_uint(tmin);
-        mark.loops = loops;
-        mark.fetches = fetches;
-        mark.next_save = 2u * loops;
-        for (uint32_t j = 0; j < depth; ++j) {
-          const uint2 a = stack[j * stride];
-          mark.stack[2 * j] = a.x;
-          mark.stack[2 * j + 1] = a.y;
+      } else {
+        if (loops >= mark.next_save) {
+          mark.node = node;
+          mark.size = __float_as_uint(sx2);
+          mark.tmin = __float_as_uint(tmin);
+          mark.loops = loops;
+          mark.fetches = fetches;
+          mark.next_save = loops + mark.gap;
+          mark.gap = 2u * mark.gap;
+          for (uint32_t j = 0; j < depth; ++j) {
+            const uint2 a = stack[j * stride];
+            mark.stack[2 * j] = a.x;
+            mark.stack[2 * j + 1] = a.y;
+          }
         }
+        check_at = loops + 1u;
       }
     }
-    bool pop;
-    if (kFlat)
-      pop = (tmax < 0.0f) || (fabsf(__fsub_rn(tmin, tmax)) < eps) || !(tmin < tmax);
-    else
-      pop = (tmax < 0.0f) || !(fabsf(__fsub_rn(tmin, tmax)) > eps);
-    if (pop) {
-      ++scale;
-      if (scale >= S) break;
-      sp -= stride;
-      const uint2 e = *sp;
-      tmin = tmax;
-      node = e.x;
-      tmax = __uint_as_float(e.y);
-      // a stacked node passed the in-pool test before its children were
-      // tested, so the popped one is in the pool
-      in_pool = true;
-      nd = fetch(node);
-      // parent centre = child centre -+ the child's sx2 (exact)
-      cx = __fadd_rn(cx, (ix & 1u) ? -sx2 : sx2);
-      cy = __fadd_rn(cy, (iy & 1u) ? -sx2 : sx2);
-      cz = __fadd_rn(cz, (iz & 1u) ? -sx2 : sx2);
-      ix >>= 1;
-      iy >>= 1;
-      iz >>= 1;
-      half = sx2;  // the parent's half child size is the child's size (exact)
-      sx2 = __fmul_rn(sx2, 2.0f);
-      continue;
-    }
-    // childEntryPoint = (o + (tMin + eps) d) - centre and its sign test: in
-    // IEEE arithmetic with subnormals, a - b > 0 exactly when a > b (a - b
-    // rounds to 0 only when a == b), so the subtraction is left out
-    const float te = __fadd_rn(tmin, eps);
-    const bool bxp = __fadd_rn(o[0], __fmul_rn(te, dx)) > cx;
-    const bool byp = __fadd_rn(o[1], __fmul_rn(te, dy)) > cy;
-    const bool bzp = __fadd_rn(o[2], __fmul_rn(te, dz)) > cz;
-    float tx0, tx1, ty0, ty1, tz0, tz1;
-    float mx = 0.0f, my = 0.0f, mz = 0.0f, ox = 0.0f, oy = 0.0f, oz = 0.0f;
-    if (kSigned) {
-      // The child's faces are the mid plane c and its outer face c +- sx2;
-      // the far one is the farther (the near ones, needed only for a valid
-      // child, are taken there).  No NaN and no -0 here, so the hardware
-      // min/max give the reference's order bit for bit.
-      mx = __fadd_rn(__fmul_rn(rx, cx), px);
-      my = __fadd_rn(__fmul_rn(ry, cy), py);
-      mz = __fadd_rn(__fmul_rn(rz, cz), pz);
-      ox = __fadd_rn(__fmul_rn(rx, __fadd_rn(cx, bxp ? sx2 : -sx2)), px);
-      oy = __fadd_rn(__fmul_rn(ry, __fadd_rn(cy, byp ? sx2 : -sx2)), py);
-      oz = __fadd_rn(__fmul_rn(rz, __fadd_rn(cz, bzp ? sx2 : -sx2)), pz);
-      tx0 = ty0 = tz0 = 0.0f;
-      tx1 = fmaxf(mx, ox);
-      ty1 = fmaxf(my, oy);
-      tz1 = fmaxf(mz, oz);
-    } else {
-      // child centre (-0.5 + b) * sx2 + c = c +- half; faces ccx -+ half
-      const float ccx = __fadd_rn(bxp ? half : -half, cx);
-      const float ccy = __fadd_rn(byp ? half : -half, cy);
-      const float ccz = __fadd_rn(bzp ? half : -half, cz);
-      tx0 = __fadd_rn(__fmul_rn(rx, __fsub_rn(ccx, half)), px);
-      tx1 = __fadd_rn(__fmul_rn(rx, __fadd_rn(ccx, half)), px);
-      if (tx0 > tx1) {
-        const float s = tx0;
-        tx0 = tx1;
-        tx1 = s;
-      }
-      ty0 = __fadd_rn(__fmul_rn(ry, __fsub_rn(ccy, half)), py);
-      ty1 = __fadd_rn(__fmul_rn(ry, __fadd_rn(ccy, half)), py);
-      if (ty0 > ty1) {
-        const float s = ty0;
-        ty0 = ty1;
-        ty1 = s;
-      }
-      tz0 = __fadd_rn(__fmul_rn(rz, __fsub_rn(ccz, half)), pz);
-      tz1 = __fadd_rn(__fmul_rn(rz, __fadd_rn(ccz, half)), pz);
-      if (tz0 > tz1) {
-        const float s = tz0;
-        tz0 = tz1;
-        tz1 = s;
-      }
-    }
-    // kSigned: no NaN and no -0 among the distances (see cast_ray), so the
-    // hardware min/max equal the reference's max/min bit for bit
-    const float tc_max = kSigned ? fminf(tx1, fminf(ty1, tz1)) : cl_min(tx1, cl_min(ty1, tz1));
-    auto near_max = [&]() {
-      return kSigned ? fmaxf(fminf(mx, ox), fmaxf(fminf(my, oy), fminf(mz, oz)))
-                     : cl_max(tx0, cl_max(ty0, tz0));
-    };
-
-    if (!in_pool) {
-      h.flags = SVO_HITFLAG_BOUNDS;
-      h.loops = loops;
-      h.fetches = fetches;
-      return;
-    }
-    ++fetches;
-    const uint32_t bx = bxp, by = byp, bz = bzp;
-    const uint32_t ci = (bx << 2) | (by << 1) | bz;
-    const uint32_t masks = nd.y;
-    const uint32_t sh = masks >> ci;  // bit 8: valid, bit 0: leaf
-    if (sh & 0x100u) {
-      const float tc_min = near_max();
-      const uint32_t below = __popc(masks & ((0x100u << ci) - 0x100u));
-      const uint32_t child = (kFlat ? 0u : node) + nd.x + below;
-      const bool leaf = sh & 1u;
-      const bool lod = kFlat ? (__fmul_rn(tsr, tc_max) > sx2)
-                             : (__fmul_rn(tsr, tc_min) > sx2 || scale == 1);
-      if (leaf || lod) {
-        h.hit = 1u;
-        h.node = child;
-        h.depth = (uint32_t)((leaf || kFlat) ? (S - scale) : (S - scale + 1));
-        h.t = tmin;
-        h.loops = loops;
-        h.fetches = fetches;
-        h.tc_min = tc_min;
-        h.sx2 = sx2;
-        h.leaf = leaf ? 1u : 0u;
-        h.cx = __fadd_rn(bxp ? half : -half, cx);
-        h.cy = __fadd_rn(byp ? half : -half, cy);
-        h.cz = __fadd_rn(bzp ? half : -half, cz);
-        return;
-      }
-      if (kFlat && scale == 0) {  // non-leaf below the octree's depth: corrupt pool
+    if (!pop) {
+      // childEntryPoint = (o + (tMin + eps) d) - centre and its sign test
+      const float te = __fadd_rn(tmin, eps);
+      const uint32_t bx = above(__fadd_rn(r.ox, __fmul_rn(te, r.dx)), cx);
+      const uint32_t by = above(__fadd_rn(r.oy, __fmul_rn(te, r.dy)), cy);
+      const uint32_t bz = above(__fadd_rn(r.oz, __fmul_rn(te, r.dz)), cz);
+      slab(bx, by, bz);
+      if (!in_pool) {
         h.flags = SVO_HITFLAG_BOUNDS;
         h.loops = loops;
         h.fetches = fetches;
         return;
       }
-      // push: the current frame's tMin becomes tc_max (recovered on pop)
-      *sp = make_uint2(node, __float_as_uint(tmax));
-      sp += stride;
-      --scale;
-      node = child;
-      in_pool = node <= last_node;
-      if (in_pool) nd = fetch(node);
-      tmin = tc_min;
-      tmax = tc_max;
-      ix = (ix << 1) | bx;
-      iy = (iy << 1) | by;
-      iz = (iz << 1) | bz;
-      cx = __fadd_rn(bx ? half : -half, cx);
-      cy = __fadd_rn(by ? half : -half, cy);
-      cz = __fadd_rn(bz ? half : -half, cz);
-      sx2 = half;
-      half = __fmul_rn(half, 0.5f);
-      continue;
+      ++fetches;
+      const uint32_t sh = nd.y >> ci;  // bit 8: valid, bit 0: leaf
+      if (sh & 0x100u) {
+        const bool leaf = sh & 1u;
+        const bool lod = kFlat ? (__fmul_rn(r.tsr, tc_max) > sx2)
+                               : (__fmul_rn(r.tsr, tc_min) > sx2 || sx2 == sx2_last);
+        if (leaf || lod) {
+          h.hit = 1u;
+          h.node = (kFlat ? 0u : node) + nd.x + __popc(nd.y & ((0x100u << ci) - 0x100u));
+          h.depth = (leaf || kFlat) ? level_of(sx2) : level_of(sx2) + 1u;
+          h.t = tmin;
+          h.loops = loops;
+          h.fetches = fetches;
+          h.tc_min = tc_min;
+          h.sx2 = sx2;
+          h.leaf = leaf ? 1u : 0u;
+          h.cx = __fadd_rn(with_side(bx, half), cx);
+          h.cy = __fadd_rn(with_side(by, half), cy);
+          h.cz = __fadd_rn(with_side(bz, half), cz);
+          return;
+        }
+        if (kFlat && sx2 == sx2_last) {  // non-leaf below the octree's depth: corrupt pool
+          h.flags = SVO_HITFLAG_BOUNDS;
+          h.loops = loops;
+          h.fetches = fetches;
+          return;
+        }
+        // the current frame's tMin becomes tc_max (recovered on pop)
+        push(bx, by, bz);
+        tmin = tc_min;
+      } else {
+        tmin = tc_max;  // advance to the next sibling
+      }
+      pop = interval_done<kFlat>(tmin, tmax);
+      if (!pop || loops + 1u >= check_at) continue;
+      ++loops;
     }
-    tmin = tc_max;  // advance to the next sibling
+    for (;;) {  // one level a turn; each is one iteration of the reference
+      if (sx2 == 0.5f) {  // above the root: the ray leaves the octree
+        ray_missed(kFlat, r, loops, fetches, h);
+        return;
+      }
+      sp -= stride;
+      tmin = tmax;
+      tmax = __uint_as_float(sp->y);
+      sx2 = __fmul_rn(sx2, 2.0f);
+      pop = interval_done<kFlat>(tmin, tmax);
+      if (!pop || loops + 1u >= check_at) break;
+      ++loops;
+    }
+    // a stacked node passed the in-pool test before its children were tested
+    node = sp->x;
+    in_pool = true;
+    nd = fetch(node);
+    const uint32_t one = __float_as_uint(__fadd_rn(1.0f, sx2));
+    const uint32_t keep = 0x7f000000u - 2u * one;
+    cx = ancestor_center(cx, one, keep);
+    cy = ancestor_center(cy, one, keep);
+    cz = ancestor_center(cz, one, keep);
   }
-  h.hit = 0u;
-  h.node = 0u;
-  h.depth = 0u;
-  h.t = kFlat ? 0.0f : t_max;
-  h.loops = loops;
-  h.fetches = fetches;
 }
 
-// One ray: root box test, direction clamp, then the descent.  loop_cap > 0
-// stops the ray after that many iterations instead of the watchdog's (S+1)^2*5
-// (used only to estimate costs; results under a cap are not the reference's).
+// The descent of a ray with finite reciprocals, until it ends (true), or until
+// it has run `limit` passes or is seen not to advance (false: `st` holds where
+// it stands).
+// kFlat selects the CpuRaycasterSingleRay3 rules; S is the stack size
+// (treelet) or the octree depth (flat).  `stack` points at this thread's column
+// of the shared-memory stack, `stride` words apart.
+//
+// A pass of the loop is one child test of the reference and every pop that
+// follows it.  A warp whose lanes each spend a pass on a single pop runs the
+// test for the other lanes beside it: on the 1080p icosphere frame 21 of 32
+// lanes took part in an average test and 11 in an average pop, and a pop took
+// 1.8 turns.  With the pops behind the test the frame takes 1.35 M warp passes
+// instead of 1.91 M, and 27 lanes take part in a test.  The loop is bound by
+// instruction issue where warps fill the GPU (a 3840x2160 primary + shadow frame
+// 1738 -> 1248 us, a million explicit rays 573 -> 446 us against one event a
+// pass) and by the chain of its longest ray elsewhere (a 1920x1080 frame 283 ->
+// 225 us, 641x479 with hit records 82 -> 55 us).  What the loop keeps per level
+// was chosen for few instructions and 48 registers (10 blocks of 128 threads an
+// SM; 55 and 9 before): no lattice coordinates, no test counter beside the pass
+// counter, no in-pool flag.
+//
+// A child that ends where its parent does -- it leaves through the same plane,
+// so the two tMax have the same bits -- is popped together with it, so the
+// parent is not stacked: popping the child goes to the nearest ancestor that
+// ends later, in one stack read.  `open` has the bit of weight sx2 set for each
+// stacked frame (over the exponent bits of 1.0f, so that a bit and those are
+// the float 1 + sx2); the level it names gives the size, the centre
+// (ancestor_center) and the number of iterations the pops count as.
+//
+// A few rays of a frame never end: they advance in place, or repeat a short
+// cycle of pushes and pops, until the watchdog stops them at (S+1)^2*5
+// iterations.  tMin grows along every other ray, so a ray whose tMin has not
+// grown over kProgressPasses passes leaves for descend_general, which looks for
+// the cycle and skips it.  (The lanes of a warp begin together and a pass is
+// one test for each, so they all look in the same pass.)
+//
+// The reference orders each child's slab distances with a compare and swap
+// (tx0 > tx1).  When the reciprocal r is finite, rounding is monotone, so the
+// swap happens exactly when r < 0 (equal values swap to themselves): the near
+// face is lo when r > 0 and hi when r < 0.  A child's two faces along an axis
+// are the parent's mid plane c and its outer face c +- sx2 (exact dyadic
+// numbers, the values the reference's childCenter +- childSizeHalf produce), so
+// each axis costs the distance to the mid plane, the distance to the outer
+// face and the max of the two (the far face); the min (the near face) is taken
+// only for a valid child, the one case that reads tcMin.  There is no NaN and
+// no -0 among the distances (see cast_ray), so the hardware min/max give the
+// reference's order bit for bit.
+constexpr uint32_t kProgressPasses = 32;
+template <bool kFlat, class Fetch>
+__device__ __forceinline__ bool descend(const Fetch& fetch, uint64_t num_nodes, const Ray& r,
+                                        int S, uint2* stack, int stride, uint32_t limit,
+                                        RayState& st, RayHit& h) {
+  const float eps = 0.00001f;
+  const float sx2_last = last_size<kFlat>(S);
+  // Pools hold at most 2^32 nodes, so the in-pool test of a 32-bit index is one
+  // compare against the last index.  A node outside gets a record of valid
+  // leaves only: its test then ends the ray, where the index is looked at again.
+  const uint32_t last_node = num_nodes ? (uint32_t)(num_nodes - 1u) : 0u;
+  constexpr uint32_t kOne = 0x3f800000u;
+  uint32_t node = 0u;
+  float tmin = st.tmin, tmax = r.t_max;
+  float cx = 0.0f, cy = 0.0f, cz = 0.0f;
+  float sx2 = 0.5f;
+  uint2 nd = num_nodes ? fetch(0u) : make_uint2(0u, 0xFFFFu);
+  uint32_t passes = 0u, pops = 0u;  // tests (the reference's fetches) and popped levels
+  uint32_t check_at = kProgressPasses < limit ? kProgressPasses : limit;
+  float seen = tmin;  // tMin when it was last looked at
+  uint32_t open = kOne;
+  uint2* sp = stack;  // the next free stack word
+  if (interval_done<kFlat>(tmin, tmax)) {
+    ray_missed(kFlat, r, 1u, 0u, h);
+    return true;
+  }
+  for (;;) {
+    if (passes == check_at) {
+      if (passes == limit || tmin <= seen) break;
+      seen = tmin;
+      check_at = check_at + kProgressPasses < limit ? check_at + kProgressPasses : limit;
+    }
+    ++passes;
+    // childEntryPoint = (o + (tMin + eps) d) - centre and its sign test
+    const float te = __fadd_rn(tmin, eps);
+    const uint32_t bx = above(__fadd_rn(r.ox, __fmul_rn(te, r.dx)), cx);
+    const uint32_t by = above(__fadd_rn(r.oy, __fmul_rn(te, r.dy)), cy);
+    const uint32_t bz = above(__fadd_rn(r.oz, __fmul_rn(te, r.dz)), cz);
+    const float mx = __fadd_rn(__fmul_rn(r.rx, cx), r.px);
+    const float my = __fadd_rn(__fmul_rn(r.ry, cy), r.py);
+    const float mz = __fadd_rn(__fmul_rn(r.rz, cz), r.pz);
+    const float ox = __fadd_rn(__fmul_rn(r.rx, __fadd_rn(cx, with_side(bx, sx2))), r.px);
+    const float oy = __fadd_rn(__fmul_rn(r.ry, __fadd_rn(cy, with_side(by, sx2))), r.py);
+    const float oz = __fadd_rn(__fmul_rn(r.rz, __fadd_rn(cz, with_side(bz, sx2))), r.pz);
+    const float tc_max = fminf(fmaxf(mx, ox), fminf(fmaxf(my, oy), fmaxf(mz, oz)));
+    const uint32_t ci = shift_in(shift_in(bx >> 31, by), bz);
+    const uint32_t masks = nd.y;
+    const uint32_t sh = masks >> ci;  // bit 8: valid, bit 0: leaf
+    if (sh & 0x100u) {
+      const float tc_min = fmaxf(fminf(mx, ox), fmaxf(fminf(my, oy), fminf(mz, oz)));
+      const float half = __fmul_rn(sx2, 0.5f);
+      const uint32_t below = __popc(masks & ((0x100u << ci) - 0x100u));
+      const uint32_t child = (kFlat ? 0u : node) + nd.x + below;
+      const bool leaf = sh & 1u;
+      const bool lod = kFlat ? (__fmul_rn(r.tsr, tc_max) > sx2)
+                             : (__fmul_rn(r.tsr, tc_min) > sx2 || sx2 == sx2_last);
+      if (leaf || lod || (kFlat && sx2 == sx2_last)) {
+        h.loops = passes + pops;
+        h.fetches = passes;
+        if (node > last_node || num_nodes == 0u) {  // the frame's node is outside the pool
+          h.flags = SVO_HITFLAG_BOUNDS;
+          h.fetches = passes - 1u;
+          return true;
+        }
+        if (kFlat && !leaf && !lod) {  // non-leaf below the octree's depth: corrupt pool
+          h.flags = SVO_HITFLAG_BOUNDS;
+          return true;
+        }
+        h.hit = 1u;
+        h.node = child;
+        h.depth = (leaf || kFlat) ? level_of(sx2) : level_of(sx2) + 1u;
+        h.t = tmin;
+        h.tc_min = tc_min;
+        h.sx2 = sx2;
+        h.leaf = leaf ? 1u : 0u;
+        h.cx = __fadd_rn(with_side(bx, half), cx);
+        h.cy = __fadd_rn(with_side(by, half), cy);
+        h.cz = __fadd_rn(with_side(bz, half), cz);
+        return true;
+      }
+      // push: the current frame's tMin becomes tc_max (recovered on pop)
+      if (tc_max != tmax) {
+        *sp = make_uint2(node, __float_as_uint(tmax));
+        sp += stride;
+        open |= __float_as_uint(__fadd_rn(1.0f, sx2));
+      }
+      node = child;
+      nd = make_uint2(0u, 0xFFFFu);
+      if (node <= last_node) nd = fetch(node);
+      tmin = tc_min;
+      tmax = tc_max;
+      cx = __fadd_rn(with_side(bx, half), cx);
+      cy = __fadd_rn(with_side(by, half), cy);
+      cz = __fadd_rn(with_side(bz, half), cz);
+      sx2 = half;
+    } else {
+      tmin = tc_max;  // advance to the next sibling
+    }
+    if (interval_done<kFlat>(tmin, tmax)) {
+      uint32_t bit;
+      do {
+        if (open == kOne) {  // above the root: the ray leaves the octree
+          ray_missed(kFlat, r, passes + pops + level_of(sx2), passes, h);
+          return true;
+        }
+        sp -= stride;
+        const uint2 e = *sp;
+        tmin = tmax;
+        node = e.x;
+        tmax = __uint_as_float(e.y);
+        bit = open & (0u - open);
+        open ^= bit;
+      } while (interval_done<kFlat>(tmin, tmax));
+      // a stacked node passed the in-pool test before its children were tested
+      nd = fetch(node);
+      const uint32_t one = kOne | bit;
+      const uint32_t keep = 0u - 2u * bit;
+      cx = ancestor_center(cx, one, keep);
+      cy = ancestor_center(cy, one, keep);
+      cz = ancestor_center(cz, one, keep);
+      const float size = __fadd_rn(__uint_as_float(one), -1.0f);
+      pops += (__float_as_uint(size) - __float_as_uint(sx2)) >> 23;
+      sx2 = size;
+    }
+  }
+  st = RayState{node, tmin, tmax, cx, cy, cz, sx2, passes + pops, passes};
+  return false;
+}
+
+// One ray: root box test, direction clamp, then the descent.  pass_cap > 0
+// stops the ray after that many child tests instead of the watchdog's
+// (S+1)^2*5 iterations (used only to estimate costs; results under a cap are
+// not the reference's: h.tc_min is how far the ray has come).
 template <bool kFlat, class Fetch>
 __device__ __forceinline__ RayHit cast_ray(const Fetch& fetch, uint64_t num_nodes,
                                            const float o[3], float dx, float dy, float dz,
                                            float tsr, int S, uint2* stack, int stride,
-                                           uint32_t loop_cap = 0u) {
+                                           uint32_t pass_cap = 0u) {
   RayHit h;
   h.node = 0u;
   h.t = 0.0f;
@@ -415,6 +637,8 @@ __device__ __forceinline__ RayHit cast_ray(const Fetch& fetch, uint64_t num_node
   h.cx = 0.0f;
   h.cy = 0.0f;
   h.cz = 0.0f;
+  h.t_enter = 0.0f;
+  h.t_exit = 0.0f;
 
   float t_min, t_max;
   {
@@ -424,6 +648,8 @@ __device__ __forceinline__ RayHit cast_ray(const Fetch& fetch, uint64_t num_node
       return h;
     }
   }
+  h.t_enter = t_min;
+  h.t_exit = t_max;
   // Direction clamp: sample() replaces |d| < 1e-4 by 1e-4 * sign(d)
   // (:231-239); traversSvo replaces |d| < 1e-5 by 1e-5 * sign(d) * 10 (:184-186).
   if (kFlat) {
@@ -437,22 +663,45 @@ __device__ __forceinline__ RayHit cast_ray(const Fetch& fetch, uint64_t num_node
     if (fabsf(dy) < mn) dy = __fmul_rn(mn, cl_sign(dy));
     if (fabsf(dz) < mn) dz = __fmul_rn(mn, cl_sign(dz));
   }
-  const float rx = __frcp_rn(dx), px = __fmul_rn(-o[0], rx);
-  const float ry = __frcp_rn(dy), py = __fmul_rn(-o[1], ry);
-  const float rz = __frcp_rn(dz), pz = __fmul_rn(-o[2], rz);
-  // kSigned needs finite reciprocals.  It also takes the hardware min/max:
-  // with finite r, a slab distance r * plane + p is -0 only for the plane at
-  // 0 when the origin coordinate is -0 and r < 0 (x + (-x) rounds to +0), so
-  // rays with a -0 origin coordinate keep the reference's compare/select.
+  Ray r;
+  r.ox = o[0];
+  r.oy = o[1];
+  r.oz = o[2];
+  r.dx = dx;
+  r.dy = dy;
+  r.dz = dz;
+  r.rx = __frcp_rn(dx);
+  r.ry = __frcp_rn(dy);
+  r.rz = __frcp_rn(dz);
+  r.px = __fmul_rn(-o[0], r.rx);
+  r.py = __fmul_rn(-o[1], r.ry);
+  r.pz = __fmul_rn(-o[2], r.rz);
+  r.t_max = t_max;
+  r.tsr = tsr;
+  // `descend` needs finite 1 / d and -o / d (the second is finite only with the
+  // first, and with a finite origin), so that no slab distance is a NaN.  It
+  // also takes the hardware min/max: a distance r * plane + p is -0 only for
+  // the plane at 0 when the origin coordinate is -0 and r < 0 (x + (-x) rounds
+  // to +0), so rays with a -0 origin coordinate keep the compare/select.
   const bool neg_zero = __float_as_uint(o[0]) == 0x80000000u ||
                         __float_as_uint(o[1]) == 0x80000000u ||
                         __float_as_uint(o[2]) == 0x80000000u;
-  if (isfinite(rx) && isfinite(ry) && isfinite(rz) && !neg_zero)
-    descend<kFlat, true>(fetch, num_nodes, o, dx, dy, dz, rx, px, ry, py, rz, pz, t_min, t_max,
-                         tsr, S, stack, stride, h, loop_cap);
-  else
-    descend<kFlat, false>(fetch, num_nodes, o, dx, dy, dz, rx, px, ry, py, rz, pz, t_min, t_max,
-                          tsr, S, stack, stride, h, loop_cap);
+  RayState st = {0u, t_min, t_max, 0.0f, 0.0f, 0.0f, 0.5f, 0u, 0u};
+  if (isfinite(r.px) && isfinite(r.py) && isfinite(r.pz) && !neg_zero) {
+    // n passes are n tests, at most as many pushes, and so at most n plus the
+    // root's pops: below this many passes no ray comes to the watchdog
+    const uint32_t limit = ((uint32_t)((S + 1) * (S + 1) * 5) - 2u) / 2u;
+    if (pass_cap) {
+      if (!descend<kFlat>(fetch, num_nodes, r, S, stack, stride, pass_cap, st, h)) {
+        h.flags = SVO_HITFLAG_CAPPED;
+        h.loops = st.loops;
+        h.tc_min = st.tmin;
+      }
+      return h;
+    }
+    if (descend<kFlat>(fetch, num_nodes, r, S, stack, stride, limit, st, h)) return h;
+  }
+  descend_general<kFlat>(fetch, num_nodes, r, S, stack, stride, st, h, pass_cap);
   return h;
 }
 
