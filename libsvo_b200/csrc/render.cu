@@ -27,24 +27,32 @@ constexpr int kThreads = kBlockW * kBlockH;
 // A frame's blocks differ in cost by two orders of magnitude (rays that graze
 // a surface run hundreds of iterations, most rays a dozen), and raster order
 // starts some of the longest blocks last, where they run on after the other
-// SMs are done.  Large frames therefore estimate each 16x8 block's cost first
-// (its two 8x8 cells' centre rays, cut off at kCostCap iterations) and
-// append the block to the list of its cost bucket; block r of the frame
-// kernel then casts the r-th block of the buckets taken costliest first.
-// Every pixel is still cast by the same code: only the order the blocks
-// start in changes.  On the 1920x1080 icosphere frame the ordered frame
-// kernel takes 254 us against 311 us in raster order, about the 246 us of
-// its longest block alone.  The estimate is a chain of dependent node reads
-// per ray, so its time grows with the cap, and a low cap ranks the blocks
-// worse: frames took 0.2910, 0.2900 and 0.2965 ms with caps 40, 48 and 63.
-// The cells' centre rays rank them better than their top-left rays (0.2827
-// against 0.2873 ms); four samples a block (one per warp tile) cost more in
-// the estimate than they gained (0.297 ms).
-constexpr uint32_t kCostCap = 48;
-constexpr uint32_t kCostBuckets = kCostCap + 1;
+// SMs are done.  Frames of one to four million pixels therefore estimate each
+// 16x8 block's cost first (its two 8x8 cells' centre rays) and append the block
+// to the list of its cost bucket; block r of the frame kernel then casts the
+// r-th block of the buckets taken costliest first.  Every pixel is still cast by
+// the same code: only the order the blocks start in changes.
+//
+// The estimate is a chain of dependent node reads per ray, so its time grows
+// with the cap on its passes.  A ray at the cap counts for what its progress
+// says about the rest of its way through the root box, so that the long blocks
+// are told from one another: 1920x1080 icosphere frames took 226 us with 48
+// passes so extended, 255 us with the 48 counted as they are, 243 us with 32,
+// 233 us with 64 passes, 235 us with one sample a block, and 256 us in raster
+// order.  Sixteen of a warp's lanes cast samples: with all 32 the paths of more
+// cells diverge in each of a warp's passes (248 against 241 us).
+//
+// The line: the tail that the order removes is a few long rays, so it does not
+// grow with the frame, while the estimate is a share of it.  At 1280x720 the two
+// are equal (107 us); at 3840x2160 an icosphere takes 761 us either way and a
+// terrain 857 us ordered, 801 us in raster order.
+constexpr uint32_t kCostCap = 48;  // passes of an estimate ray
+constexpr uint32_t kCostBuckets = 49;
+constexpr uint32_t kCostTop = kCostBuckets - 1;
 constexpr uint32_t kCostSamples = kBlockW / 8;  // one ray per 8x8 cell of a block
+constexpr uint32_t kCostLanes = 16;             // lanes of a warp that cast a sample
 constexpr uint64_t kOrderMinPixels = 1ull << 20;
-constexpr uint32_t kOrderMaxBlocks = 1u << 20;
+constexpr uint64_t kOrderMaxPixels = 1ull << 22;
 static_assert(kCostSamples == 2, "a block's cost is the larger of two adjacent lanes' samples");
 static_assert(kCostBuckets > 32 && kCostBuckets <= 64, "one warp scans the buckets, two per lane");
 
@@ -69,14 +77,14 @@ __device__ __forceinline__ uint32_t same_key_lanes(uint32_t k) {
   return peers;
 }
 
-// The r-th block in cost order (buckets kCostCap down to 0, each in the
+// The r-th block in cost order (buckets kCostTop down to 0, each in the
 // order its blocks were appended).  Called by one whole warp; every lane
 // returns the block.
 __device__ __forceinline__ uint32_t ordered_block(const BlockOrder& o, uint32_t r, uint32_t lane) {
-  const uint32_t k1 = lane + 32 < kCostBuckets ? kCostCap - 32 - lane : 0u;
-  const uint32_t c0 = __ldg(o.count + (kCostCap - lane));
+  const uint32_t k1 = lane + 32 < kCostBuckets ? kCostTop - 32 - lane : 0u;
+  const uint32_t c0 = __ldg(o.count + (kCostTop - lane));
   const uint32_t c1 = lane + 32 < kCostBuckets ? __ldg(o.count + k1) : 0u;
-  uint32_t p0 = c0, p1 = c1;  // inclusive prefix sums, bucket kCostCap first
+  uint32_t p0 = c0, p1 = c1;  // inclusive prefix sums, bucket kCostTop first
   for (uint32_t d = 1; d < 32; d <<= 1) {
     const uint32_t y0 = __shfl_up_sync(0xFFFFFFFFu, p0, d);
     const uint32_t y1 = __shfl_up_sync(0xFFFFFFFFu, p1, d);
@@ -90,13 +98,13 @@ __device__ __forceinline__ uint32_t ordered_block(const BlockOrder& o, uint32_t 
   uint32_t bucket, before;
   if (m != 0u) {
     const int l = __ffs(m) - 1;
-    bucket = kCostCap - (uint32_t)l;
+    bucket = kCostTop - (uint32_t)l;
     before = __shfl_sync(0xFFFFFFFFu, p0 - c0, l);
   } else {
     m = __ballot_sync(0xFFFFFFFFu, p1 > r);
     if (m == 0u) return r;  // not reached: the buckets hold every block once
     const int l = __ffs(m) - 1;
-    bucket = kCostCap - 32 - (uint32_t)l;
+    bucket = kCostTop - 32 - (uint32_t)l;
     before = __shfl_sync(0xFFFFFFFFu, p1 - c1, l);
   }
   return __ldg(o.list + (uint64_t)bucket * o.nblocks + (r - before));
@@ -144,9 +152,20 @@ __global__ void __launch_bounds__(kThreads) render_frame_kernel(
   count_stats(stats, h);
 }
 
+// The bucket of a sample ray: six to a doubling of its expected iterations.
+__device__ __forceinline__ uint32_t cost_bucket(const RayHit& h) {
+  float n = (float)h.loops;
+  if (h.flags == SVO_HITFLAG_CAPPED) {
+    const float enter = fmaxf(h.t_enter, 0.0f);
+    const float done = __fdividef(h.tc_min - enter, h.t_exit - enter);
+    n = __fdividef(n, fminf(fmaxf(done, 0.02f), 1.0f));
+  }
+  return min((uint32_t)(__log2f(fmaxf(n, 1.0f)) * 6.0f), kCostBuckets - 1u);
+}
+
 // The cost estimate: one thread per sample ray, the two samples of block b
-// in lanes 2b and 2b+1 of a warp.  The block's cost (the larger sample,
-// capped) picks its bucket, and the block is appended to that bucket's list
+// in adjacent lanes.  The larger of its two buckets is the block's, and the
+// block is appended to that bucket's list
 // (one atomic per bucket and warp, so neighbouring blocks of a bucket stay
 // together).
 template <bool kFlat>
@@ -154,26 +173,26 @@ __global__ void __launch_bounds__(kThreads) block_cost_kernel(
     const uint2* __restrict__ nodes, uint64_t num_nodes, const svo_frame_params p, int S,
     uint32_t gx, uint32_t nblocks, uint32_t* __restrict__ count, uint32_t* __restrict__ list) {
   extern __shared__ uint2 stack_smem[];
-  const uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
   const uint32_t lane = threadIdx.x % 32;
+  const uint64_t i = ((uint64_t)blockIdx.x * (kThreads / 32) + threadIdx.x / 32) * kCostLanes + lane;
   // the frame kernel may be scheduled once every block of this grid has
   // started (it waits for this grid's completion before reading the lists)
   asm volatile("griddepcontrol.launch_dependents;");
-  const bool live = i < (uint64_t)nblocks * kCostSamples;
+  const bool live = lane < kCostLanes && i < (uint64_t)nblocks * kCostSamples;
   const uint32_t b = (uint32_t)(i / kCostSamples), c = (uint32_t)(i % kCostSamples);
   // the cell's centre pixel (pixel 4, 4 of the 8x8 cell; clamped to the
   // frame in cells cut by its edge)
   const uint32_t x0 = (b % gx) * kBlockW + c * 8, y0 = (b / gx) * kBlockH;
   const uint32_t x = min(x0 + 4u, p.width - 1u), y = min(y0 + 4u, p.height - 1u);
-  uint32_t loops = 0u;
+  uint32_t cost = 0u;
   if (live && x0 < p.width && y0 < p.height) {
     float o[3], dx, dy, dz;
     pixel_ray(p, x, y, o, dx, dy, dz);
-    loops = cast_ray<kFlat>(GlobalFetch{nodes}, num_nodes, o, dx, dy, dz, p.t_scale_ratio, S,
-                            stack_smem + threadIdx.x, kThreads, kCostCap)
-                .loops;
+    const RayHit h = cast_ray<kFlat>(GlobalFetch{nodes}, num_nodes, o, dx, dy, dz, p.t_scale_ratio,
+                                     S, stack_smem + threadIdx.x, kThreads, kCostCap);
+    cost = cost_bucket(h);
   }
-  const uint32_t cost = min(max(loops, __shfl_xor_sync(0xFFFFFFFFu, loops, 1)), kCostCap);
+  cost = max(cost, __shfl_xor_sync(0xFFFFFFFFu, cost, 1));
   const bool appends = live && c == 0;
   const uint32_t peers = same_key_lanes(appends ? cost : kCostBuckets) & 0x55555555u;
   if (appends) {
@@ -294,11 +313,12 @@ cudaMemPool_t order_pool() {
 
 // Longest-first order of the frame's blocks into *order (stream-ordered
 // scratch the caller frees with cudaFreeAsync(order->count)); false when the
-// frame is small or scratch is not available, and the raster launch is used
+// frame is too small or too large for it or scratch is not available, and the raster launch is used
 // instead.
 bool order_blocks(const uint2* nodes, uint64_t num_nodes, const svo_frame_params& p, int S,
                   bool flat, uint32_t gx, uint32_t nblocks, cudaStream_t stream, BlockOrder* order) {
-  if ((uint64_t)p.width * p.height < kOrderMinPixels || nblocks > kOrderMaxBlocks) return false;
+  const uint64_t pixels = (uint64_t)p.width * p.height;
+  if (pixels < kOrderMinPixels || pixels > kOrderMaxPixels) return false;
   cudaMemPool_t pool = order_pool();
   if (!pool) {
     cudaGetLastError();
@@ -315,7 +335,8 @@ bool order_blocks(const uint2* nodes, uint64_t num_nodes, const svo_frame_params
   }
   uint32_t* list = scratch + kCountBytes / sizeof(uint32_t);
   const uint64_t samples = (uint64_t)nblocks * kCostSamples;
-  const unsigned grid = (unsigned)((samples + kThreads - 1) / kThreads);
+  constexpr uint32_t kPerBlock = kThreads / 32 * kCostLanes;
+  const unsigned grid = (unsigned)((samples + kPerBlock - 1) / kPerBlock);
   const size_t smem = render_smem_bytes(S);
   bool ok = cudaMemsetAsync(scratch, 0, kCountBytes, stream) == cudaSuccess;
   if (ok) {
