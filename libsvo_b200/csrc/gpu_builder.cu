@@ -12,24 +12,37 @@
 // TreeletMemoryManager (src/TreeletMemoryManager.cpp:518-545).
 //
 // Pipeline, all in device memory:
-//  1. face normals, one thread per triangle;
-//  2. voxelisation per spatial chunk (the top octree level(s)): a count pass
-//     and an emit pass, one thread per triangle, walking columns along the
-//     dominant normal axis exactly like the host builder, with the
-//     separating-axis triangle/box test; each overlap is a 64-bit key
-//     (code within the chunk << tri_bits | triangle);
-//  3. radix sort of the keys (CUB), so equal codes are grouped with their
-//     triangles ascending, then one thread per run sums the face normals in
-//     that order -> leaf codes and attributes;
-//  4. octree levels bottom-up: one thread per parent over its <= 8 children
-//     (valid mask, first child, averaged attributes as the host does);
-//  5. the treelet cut in closed form: treelet boundaries sit on fixed levels
+//  1. per-triangle records: what a leaf needs of a triangle that does not depend
+//     on the voxel (the interpolation's vectors, or the face normal);
+//  2. voxelisation: one thread per column of voxels along a triangle's dominant
+//     normal axis, walked exactly like the host builder with the separating-axis
+//     triangle/box test; the columns of all triangles are numbered one after
+//     another, so a triangle of two voxels and one of a thousand fill the GPU
+//     alike.  A first pass keeps each column's hits as a mask, a second writes
+//     the overlaps as 64-bit keys (code << tri_bits | triangle), triangles
+//     ascending;
+//  3. a stable radix sort of the keys by code (CUB), so equal codes are grouped
+//     with their triangles ascending;
+//  4. the octree from the sorted keys in two passes: where a key differs from the
+//     one before it says which levels begin a node there, so one count per block
+//     and level, and one pass that writes every level's first children and each
+//     leaf's attributes (summed over its triangles in order, as the host does);
+//  5. attributes of the inner levels bottom-up, one thread per parent over its
+//     <= 8 children;
+//  6. the treelet cut in closed form: treelet boundaries sit on fixed levels
 //     (stop_level), each treelet is the breadth-first fill of its root's
 //     subtree down to the next boundary, so its nodes at a level are one
 //     contiguous range of that level, its local positions are range offsets,
 //     and the treelet ids are range offsets of the boundary levels; one block
 //     per treelet writes its slot, with every sub-treelet root patched into
 //     its parent's leaf as insert_all does.
+// Octrees whose keys would not fit 64 bits, or whose columns number more than
+// kMaxColumns, run 2 to 4 once per spatial chunk (a cell of a top level).
+//
+// Scratch comes from a stream-ordered memory pool of the library's own; the host
+// waits four times a chunk for a size.  An 81,920-triangle icosphere at depth 11
+// (13 M leaves, 17.3 M nodes, a 628 MB pool) takes 4.1 ms (69.7 before), a 131,072-triangle
+// terrain at depth 9 0.96 ms (22.7), the 5.2 M-triangle depth-14 octree 0.67 s (1.61).
 //
 // FP32 arithmetic uses explicit round-to-nearest intrinsics in the host
 // builder's operation order (the library is built with -fmad=false), so the
@@ -41,6 +54,8 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <mutex>
+#include <utility>
 #include <vector>
 
 #include "../../include/libsvo_b200.h"
@@ -80,11 +95,6 @@ __device__ __forceinline__ uint32_t pack_color(float r, float g, float b) {
 __device__ __forceinline__ uint32_t pack_normal(float x, float y, float z) {
   return pack_color(__fadd_rn(__fmul_rn(x, 0.5f), 0.5f), __fadd_rn(__fmul_rn(y, 0.5f), 0.5f),
                     __fadd_rn(__fmul_rn(z, 0.5f), 0.5f));
-}
-__device__ __forceinline__ void unpack_color(uint32_t v, float rgb[3]) {
-  rgb[0] = __fdiv_rn((float)(v >> 24), 255.0f);
-  rgb[1] = __fdiv_rn((float)((v >> 16) & 255u), 255.0f);
-  rgb[2] = __fdiv_rn((float)((v >> 8) & 255u), 255.0f);
 }
 __device__ __forceinline__ float len3(float x, float y, float z) {
   return __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z)));
@@ -151,31 +161,89 @@ __device__ bool tri_box_overlap(const float bc[3], float h, const float a[3], co
   return __fadd_rn(dot3(n[0], n[1], n[2], vmax), d) >= 0.0f;
 }
 
-// ---- 1. face normals ---------------------------------------------------------
+// ---- 1. triangle records -------------------------------------------------------
+
+__device__ __forceinline__ void face_normal(const float* a, const float* b, const float* c,
+                                            float n[3]) {
+  n[0] = __fsub_rn(__fmul_rn(__fsub_rn(b[1], a[1]), __fsub_rn(c[2], a[2])),
+                   __fmul_rn(__fsub_rn(b[2], a[2]), __fsub_rn(c[1], a[1])));
+  n[1] = __fsub_rn(__fmul_rn(__fsub_rn(b[2], a[2]), __fsub_rn(c[0], a[0])),
+                   __fmul_rn(__fsub_rn(b[0], a[0]), __fsub_rn(c[2], a[2])));
+  n[2] = __fsub_rn(__fmul_rn(__fsub_rn(b[0], a[0]), __fsub_rn(c[1], a[1])),
+                   __fmul_rn(__fsub_rn(b[1], a[1]), __fsub_rn(c[0], a[0])));
+}
 
 __global__ void face_normals_kernel(const float* __restrict__ V, const uint32_t* __restrict__ T,
                                     uint64_t nt, float* __restrict__ fn) {
   const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nt) return;
-  const float* a = V + 3 * (uint64_t)T[3 * t];
-  const float* b = V + 3 * (uint64_t)T[3 * t + 1];
-  const float* c = V + 3 * (uint64_t)T[3 * t + 2];
-  const float n0 = __fsub_rn(__fmul_rn(__fsub_rn(b[1], a[1]), __fsub_rn(c[2], a[2])),
-                             __fmul_rn(__fsub_rn(b[2], a[2]), __fsub_rn(c[1], a[1])));
-  const float n1 = __fsub_rn(__fmul_rn(__fsub_rn(b[2], a[2]), __fsub_rn(c[0], a[0])),
-                             __fmul_rn(__fsub_rn(b[0], a[0]), __fsub_rn(c[2], a[2])));
-  const float n2 = __fsub_rn(__fmul_rn(__fsub_rn(b[0], a[0]), __fsub_rn(c[1], a[1])),
-                             __fmul_rn(__fsub_rn(b[1], a[1]), __fsub_rn(c[0], a[0])));
-  const float len = len3(n0, n1, n2);
+  float n[3];
+  face_normal(V + 3 * (uint64_t)T[3 * t], V + 3 * (uint64_t)T[3 * t + 1],
+              V + 3 * (uint64_t)T[3 * t + 2], n);
+  const float len = len3(n[0], n[1], n[2]);
   if (len > 0.0f) {
-    fn[3 * t] = __fdiv_rn(n0, len);
-    fn[3 * t + 1] = __fdiv_rn(n1, len);
-    fn[3 * t + 2] = __fdiv_rn(n2, len);
+    fn[3 * t] = __fdiv_rn(n[0], len);
+    fn[3 * t + 1] = __fdiv_rn(n[1], len);
+    fn[3 * t + 2] = __fdiv_rn(n[2], len);
   } else {
     fn[3 * t] = 0.0f;
     fn[3 * t + 1] = 0.0f;
     fn[3 * t + 2] = 1.0f;
   }
+}
+
+// The part of leaf_contribution (host builder, csrc/scene.cpp) that is the same
+// for every voxel of a triangle: 128 bytes, read by each of the triangle's
+// leaves (160 on average in the depth-11 icosphere) instead of computed there.
+struct __align__(16) TriRecord {
+  float p0[3], inv;   // vertex 0; 1 / det, 0 where the ray is parallel
+  float pv[3], e1[3], d[3];
+  float n0[3], n1[3], n2[3], c0[3], c1[3], c2[3];
+  float hits;         // 1: the ray meets the plane, 0: u = v = 0
+};
+static_assert(sizeof(TriRecord) == 128, "eight 16-byte loads");
+
+__global__ void tri_records_kernel(const float* __restrict__ V, const float* __restrict__ N,
+                                   const float* __restrict__ C, const uint32_t* __restrict__ T,
+                                   uint64_t nt, TriRecord* __restrict__ out) {
+  const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nt) return;
+  TriRecord r;
+  float p1[3], p2[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const uint64_t i0 = 3 * (uint64_t)T[3 * t] + k, i1 = 3 * (uint64_t)T[3 * t + 1] + k,
+                   i2 = 3 * (uint64_t)T[3 * t + 2] + k;
+    r.p0[k] = V[i0];
+    p1[k] = V[i1];
+    p2[k] = V[i2];
+    r.n0[k] = N[i0];
+    r.n1[k] = N[i1];
+    r.n2[k] = N[i2];
+    r.c0[k] = C[i0];
+    r.c1[k] = C[i1];
+    r.c2[k] = C[i2];
+    r.d[k] = __fdiv_rn(__fadd_rn(__fadd_rn(r.n0[k], r.n1[k]), r.n2[k]), 3.0f);
+  }
+  const float len = len3(r.d[0], r.d[1], r.d[2]);
+  if (len > 0.0f) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) r.d[k] = __fdiv_rn(r.d[k], len);
+  }
+  float e2[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    r.e1[k] = __fsub_rn(p1[k], r.p0[k]);
+    e2[k] = __fsub_rn(p2[k], r.p0[k]);
+  }
+  r.pv[0] = __fsub_rn(__fmul_rn(r.d[1], e2[2]), __fmul_rn(r.d[2], e2[1]));
+  r.pv[1] = __fsub_rn(__fmul_rn(r.d[2], e2[0]), __fmul_rn(r.d[0], e2[2]));
+  r.pv[2] = __fsub_rn(__fmul_rn(r.d[0], e2[1]), __fmul_rn(r.d[1], e2[0]));
+  const float det = dot3(r.e1[0], r.e1[1], r.e1[2], r.pv);
+  const bool hits = !(det > -1e-8f && det < 1e-8f);
+  r.hits = hits ? 1.0f : 0.0f;
+  r.inv = hits ? __fdiv_rn(1.0f, det) : 0.0f;
+  out[t] = r;
 }
 
 // ---- 2. voxelisation ---------------------------------------------------------
@@ -186,150 +254,343 @@ struct Chunk {
   uint32_t tri_bits;   // bits of the triangle index in a key
 };
 
-// Walks the host builder's candidate voxels of triangle t inside the chunk;
-// calls emit(code) for each overlapping voxel, in the host's order.
-template <class Emit>
-__device__ __forceinline__ void voxel_walk(const float* __restrict__ V,
-                                           const uint32_t* __restrict__ T, uint64_t t,
-                                           uint32_t depth, const Chunk& ch, Emit&& emit) {
+// A triangle as the voxeliser walks it: columns of voxels along axis w (the
+// dominant one of its normal), iu in [ulo, ulo + nu), iv in [vlo, vlo + nv).
+struct TriWalk {
+  float a[3], b[3], c[3], n[3], pd;
+  int w, u, v, ulo, vlo, wlo, whi;
+  uint32_t nu, nv;  // both 0: no candidate voxel in the chunk
+};
+
+__device__ __forceinline__ void tri_walk(const float* __restrict__ V,
+                                         const uint32_t* __restrict__ T, uint64_t t,
+                                         uint32_t depth, const Chunk& ch, TriWalk& s) {
   const uint32_t R = 1u << depth;
   const float Rf = (float)R;
-  const float inv = __fdiv_rn(1.0f, Rf);
-  const float h = __fmul_rn(0.5f, inv);
-  float a[3], b[3], c[3];
+  const uint64_t i0 = 3 * (uint64_t)T[3 * t], i1 = 3 * (uint64_t)T[3 * t + 1],
+                 i2 = 3 * (uint64_t)T[3 * t + 2];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    a[k] = V[3 * (uint64_t)T[3 * t] + k];
-    b[k] = V[3 * (uint64_t)T[3 * t + 1] + k];
-    c[k] = V[3 * (uint64_t)T[3 * t + 2] + k];
+    s.a[k] = V[i0 + k];
+    s.b[k] = V[i1 + k];
+    s.c[k] = V[i2 + k];
   }
-  const float n[3] = {__fsub_rn(__fmul_rn(__fsub_rn(b[1], a[1]), __fsub_rn(c[2], a[2])),
-                                __fmul_rn(__fsub_rn(b[2], a[2]), __fsub_rn(c[1], a[1]))),
-                      __fsub_rn(__fmul_rn(__fsub_rn(b[2], a[2]), __fsub_rn(c[0], a[0])),
-                                __fmul_rn(__fsub_rn(b[0], a[0]), __fsub_rn(c[2], a[2]))),
-                      __fsub_rn(__fmul_rn(__fsub_rn(b[0], a[0]), __fsub_rn(c[1], a[1])),
-                                __fmul_rn(__fsub_rn(b[1], a[1]), __fsub_rn(c[0], a[0])))};
+  face_normal(s.a, s.b, s.c, s.n);
   int lo[3], hi[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const float mn = smin(a[k], smin(b[k], c[k]));
-    const float mx = smax(a[k], smax(b[k], c[k]));
+    const float mn = smin(s.a[k], smin(s.b[k], s.c[k]));
+    const float mx = smax(s.a[k], smax(s.b[k], s.c[k]));
     lo[k] = max(0, cell_floor(__fmul_rn(__fadd_rn(mn, 0.5f), Rf), R));
     hi[k] = min((int)R - 1, cell_floor(__fmul_rn(__fadd_rn(mx, 0.5f), Rf), R));
-    if (lo[k] > hi[k]) lo[k] = hi[k] + 1;
   }
-  if (lo[0] > hi[0] || lo[1] > hi[1] || lo[2] > hi[2]) return;
-  int w = 0;
-  if (fabsf(n[1]) > fabsf(n[w])) w = 1;
-  if (fabsf(n[2]) > fabsf(n[w])) w = 2;
-  const int u = (w + 1) % 3, v = (w + 2) % 3;
-  const float pd = dot3(n[0], n[1], n[2], a);
+  s.w = 0;
+  if (fabsf(s.n[1]) > fabsf(s.n[0])) s.w = 1;
+  if (fabsf(s.n[2]) > fabsf(s.w == 1 ? s.n[1] : s.n[0])) s.w = 2;
+  s.u = s.w == 2 ? 0 : s.w + 1;
+  s.v = s.u == 2 ? 0 : s.u + 1;
+  s.pd = dot3(s.n[0], s.n[1], s.n[2], s.a);
+  const bool none = lo[0] > hi[0] || lo[1] > hi[1] || lo[2] > hi[2];
   // the chunk restricts the (u, v) range and each column's w range
-  const int ulo = max(lo[u], ch.lo[u]), uhi = min(hi[u], ch.hi[u]);
-  const int vlo = max(lo[v], ch.lo[v]), vhi = min(hi[v], ch.hi[v]);
-  for (int iu = ulo; iu <= uhi; ++iu)
-    for (int iv = vlo; iv <= vhi; ++iv) {
-      int wlo = lo[w], whi = hi[w];
-      if (n[w] != 0.0f) {
-        const float u0 = __fadd_rn(-0.5f, __fmul_rn((float)iu, inv)), u1 = __fadd_rn(u0, inv);
-        const float v0 = __fadd_rn(-0.5f, __fmul_rn((float)iv, inv)), v1 = __fadd_rn(v0, inv);
-        float wmin = 1e30f, wmax = -1e30f;
-        const float us[2] = {u0, u1}, vs[2] = {v0, v1};
+  auto pick = [](const int* x, int k) { return k == 0 ? x[0] : (k == 1 ? x[1] : x[2]); };
+  s.ulo = max(pick(lo, s.u), pick(ch.lo, s.u));
+  s.vlo = max(pick(lo, s.v), pick(ch.lo, s.v));
+  const int uhi = min(pick(hi, s.u), pick(ch.hi, s.u)), vhi = min(pick(hi, s.v), pick(ch.hi, s.v));
+  s.wlo = pick(lo, s.w);
+  s.whi = pick(hi, s.w);
+  const bool out = none || s.ulo > uhi || s.vlo > vhi || max(s.wlo, pick(ch.lo, s.w)) > min(s.whi, pick(ch.hi, s.w));
+  s.nu = out ? 0u : (uint32_t)(uhi - s.ulo + 1);
+  s.nv = out ? 0u : (uint32_t)(vhi - s.vlo + 1);
+}
+
+// The candidate voxels of column (iu, iv), w from *wlo to *whi.
+__device__ __forceinline__ void column_range(const TriWalk& s, uint32_t depth, const Chunk& ch,
+                                             int iu, int iv, int* wlo, int* whi) {
+  const uint32_t R = 1u << depth;
+  const float Rf = (float)R;
+  const float inv = __fdiv_rn(1.0f, Rf);
+  auto pick = [](const float* x, int k) { return k == 0 ? x[0] : (k == 1 ? x[1] : x[2]); };
+  const float nw = pick(s.n, s.w), nu = pick(s.n, s.u), nv = pick(s.n, s.v);
+  *wlo = s.wlo;
+  *whi = s.whi;
+  if (nw != 0.0f) {
+    const float u0 = __fadd_rn(-0.5f, __fmul_rn((float)iu, inv)), u1 = __fadd_rn(u0, inv);
+    const float v0 = __fadd_rn(-0.5f, __fmul_rn((float)iv, inv)), v1 = __fadd_rn(v0, inv);
+    float wmin = 1e30f, wmax = -1e30f;
+    const float us[2] = {u0, u1}, vs[2] = {v0, v1};
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            const float ww = __fdiv_rn(
-                __fsub_rn(__fsub_rn(pd, __fmul_rn(n[u], us[i])), __fmul_rn(n[v], vs[j])), n[w]);
-            wmin = smin(wmin, ww);
-            wmax = smax(wmax, ww);
-          }
-        wlo = max(wlo, cell_floor(__fmul_rn(__fadd_rn(wmin, 0.5f), Rf), R) - 1);
-        whi = min(whi, cell_floor(__fmul_rn(__fadd_rn(wmax, 0.5f), Rf), R) + 1);
+      for (int j = 0; j < 2; ++j) {
+        const float ww = __fdiv_rn(
+            __fsub_rn(__fsub_rn(s.pd, __fmul_rn(nu, us[i])), __fmul_rn(nv, vs[j])), nw);
+        wmin = smin(wmin, ww);
+        wmax = smax(wmax, ww);
       }
-      wlo = max(wlo, ch.lo[w]);
-      whi = min(whi, ch.hi[w]);
-      for (int iw = wlo; iw <= whi; ++iw) {
-        int ijk[3];
-        ijk[u] = iu;
-        ijk[v] = iv;
-        ijk[w] = iw;
-        const float bc[3] = {__fadd_rn(-0.5f, __fmul_rn(__fadd_rn((float)ijk[0], 0.5f), inv)),
-                             __fadd_rn(-0.5f, __fmul_rn(__fadd_rn((float)ijk[1], 0.5f), inv)),
-                             __fadd_rn(-0.5f, __fmul_rn(__fadd_rn((float)ijk[2], 0.5f), inv))};
-        if (tri_box_overlap(bc, h, a, b, c))
-          emit(morton3((uint32_t)ijk[0], (uint32_t)ijk[1], (uint32_t)ijk[2]));
+    *wlo = max(*wlo, cell_floor(__fmul_rn(__fadd_rn(wmin, 0.5f), Rf), R) - 1);
+    *whi = min(*whi, cell_floor(__fmul_rn(__fadd_rn(wmax, 0.5f), Rf), R) + 1);
+  }
+  const int clo = s.w == 0 ? ch.lo[0] : (s.w == 1 ? ch.lo[1] : ch.lo[2]);
+  const int chi = s.w == 0 ? ch.hi[0] : (s.w == 1 ? ch.hi[1] : ch.hi[2]);
+  *wlo = max(*wlo, clo);
+  *whi = min(*whi, chi);
+}
+
+__device__ __forceinline__ void voxel_of(const TriWalk& s, int iu, int iv, int iw, uint32_t ijk[3]) {
+  ijk[0] = (uint32_t)(s.w == 0 ? iw : (s.u == 0 ? iu : iv));
+  ijk[1] = (uint32_t)(s.w == 1 ? iw : (s.u == 1 ? iu : iv));
+  ijk[2] = (uint32_t)(s.w == 2 ? iw : (s.u == 2 ? iu : iv));
+}
+
+__device__ __forceinline__ bool voxel_hit(const TriWalk& s, uint32_t depth, const uint32_t ijk[3]) {
+  const float inv = __fdiv_rn(1.0f, (float)(1u << depth));
+  const float h = __fmul_rn(0.5f, inv);
+  const float bc[3] = {__fadd_rn(-0.5f, __fmul_rn(__fadd_rn((float)ijk[0], 0.5f), inv)),
+                       __fadd_rn(-0.5f, __fmul_rn(__fadd_rn((float)ijk[1], 0.5f), inv)),
+                       __fadd_rn(-0.5f, __fmul_rn(__fadd_rn((float)ijk[2], 0.5f), inv))};
+  return tri_box_overlap(bc, h, s.a, s.b, s.c);
+}
+
+// cols[t]: the columns of triangle t inside the chunk; cols[nt] = 0, so that an
+// exclusive sum over nt + 1 entries ends with the total.
+__global__ void column_count_kernel(const float* __restrict__ V, const uint32_t* __restrict__ T,
+                                    uint64_t nt, uint32_t depth, Chunk ch,
+                                    uint64_t* __restrict__ cols) {
+  const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t > nt) return;
+  if (t == nt) {
+    cols[t] = 0;
+    return;
+  }
+  TriWalk s;
+  tri_walk(V, T, t, depth, ch, s);
+  cols[t] = (uint64_t)s.nu * s.nv;
+}
+
+// The last index of off[lo..hi] whose value is <= x (off[lo] <= x).
+__device__ __forceinline__ uint64_t last_at_most(const uint64_t* __restrict__ off, uint64_t lo,
+                                                 uint64_t hi, uint64_t x) {
+  while (lo < hi) {
+    const uint64_t mid = (lo + hi + 1) / 2;
+    if (off[mid] <= x)
+      lo = mid;
+    else
+      hi = mid - 1;
+  }
+  return lo;
+}
+
+constexpr int kColThreads = 256;
+// A column's hits: bit i of the low byte for the voxel i above the first
+// candidate, whose w is in the bits above; columns of more than eight candidates
+// (a triangle without a dominant axis) are tested again where they are emitted.
+constexpr uint32_t kTestAgain = 0xFFFFFFFFu;
+
+// The triangle of column c: the block's first and last column are looked up in
+// all of `off`, the others between those two.
+__device__ __forceinline__ uint64_t column_triangle(const uint64_t* __restrict__ off, uint64_t nt,
+                                                    uint64_t columns, uint64_t c) {
+  __shared__ uint64_t ends[2];
+  const uint64_t base = (uint64_t)blockIdx.x * kColThreads;
+  if (threadIdx.x == 0) ends[0] = last_at_most(off, 0, nt - 1, base);
+  if (threadIdx.x == 32)
+    ends[1] = last_at_most(off, 0, nt - 1, min(base + kColThreads - 1, columns - 1));
+  __syncthreads();
+  return c < columns ? last_at_most(off, ends[0], ends[1], c) : 0;
+}
+
+__global__ void __launch_bounds__(kColThreads) column_test_kernel(
+    const float* __restrict__ V, const uint32_t* __restrict__ T, uint64_t nt, uint32_t depth,
+    Chunk ch, const uint64_t* __restrict__ off, uint64_t columns, uint32_t* __restrict__ rec,
+    uint64_t* __restrict__ block_hits) {
+  const uint64_t c = (uint64_t)blockIdx.x * kColThreads + threadIdx.x;
+  const uint64_t t = column_triangle(off, nt, columns, c);
+  uint32_t hits = 0;
+  if (c < columns) {
+    TriWalk s;
+    tri_walk(V, T, t, depth, ch, s);
+    const uint64_t k = c - off[t];
+    const int iu = s.ulo + (int)(k / s.nv), iv = s.vlo + (int)(k % s.nv);
+    int wlo, whi;
+    column_range(s, depth, ch, iu, iv, &wlo, &whi);
+    uint32_t mask = 0;
+    for (int iw = wlo; iw <= whi; ++iw) {
+      uint32_t ijk[3];
+      voxel_of(s, iu, iv, iw, ijk);
+      if (voxel_hit(s, depth, ijk)) {
+        ++hits;
+        mask |= 1u << ((iw - wlo) & 31);
       }
     }
-}
-
-__global__ void voxel_count_kernel(const float* __restrict__ V, const uint32_t* __restrict__ T,
-                                   uint64_t nt, uint32_t depth, Chunk ch,
-                                   uint64_t* __restrict__ counts) {
-  const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nt) return;
-  uint64_t n = 0;
-  voxel_walk(V, T, t, depth, ch, [&](uint64_t) { ++n; });
-  counts[t] = n;
-}
-
-__global__ void voxel_emit_kernel(const float* __restrict__ V, const uint32_t* __restrict__ T,
-                                  uint64_t nt, uint32_t depth, Chunk ch,
-                                  const uint64_t* __restrict__ offsets,
-                                  uint64_t* __restrict__ keys) {
-  const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nt) return;
-  uint64_t pos = offsets[t];
-  const uint64_t low = ch.shift >= 64 ? ~0ull : ((1ull << ch.shift) - 1ull);
-  voxel_walk(V, T, t, depth, ch,
-             [&](uint64_t code) { keys[pos++] = ((code & low) << ch.tri_bits) | t; });
-}
-
-// ---- 3. leaves -----------------------------------------------------------------
-
-__global__ void run_heads_kernel(const uint64_t* __restrict__ keys, uint64_t n, uint32_t tri_bits,
-                                 uint32_t* __restrict__ heads) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  heads[i] = (i == 0 || (keys[i] >> tri_bits) != (keys[i - 1] >> tri_bits)) ? 1u : 0u;
-}
-
-// One thread per run of equal codes: the normalised sum of the face normals
-// in triangle order (host: build_mesh_leaves' final loop).
-__global__ void leaf_reduce_kernel(const uint64_t* __restrict__ keys, uint64_t n,
-                                   uint32_t tri_bits, uint64_t chunk_base,
-                                   const uint32_t* __restrict__ heads,
-                                   const uint32_t* __restrict__ run_of,
-                                   const float* __restrict__ fn, uint64_t* __restrict__ codes,
-                                   svo_attrib* __restrict__ attribs) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || !heads[i]) return;
-  const uint64_t code = keys[i] >> tri_bits;
-  const uint64_t tmask = (1ull << tri_bits) - 1ull;
-  float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f;
-  uint64_t j = i;
-  do {
-    const uint64_t t = keys[j] & tmask;
-    s0 = __fadd_rn(s0, fn[3 * t]);
-    s1 = __fadd_rn(s1, fn[3 * t + 1]);
-    s2 = __fadd_rn(s2, fn[3 * t + 2]);
-    ++j;
-  } while (j < n && (keys[j] >> tri_bits) == code);
-  const float len = len3(s0, s1, s2);
-  if (len > 0.0f) {
-    s0 = __fdiv_rn(s0, len);
-    s1 = __fdiv_rn(s1, len);
-    s2 = __fdiv_rn(s2, len);
-  } else {
-    s0 = 0.0f;
-    s1 = 0.0f;
-    s2 = 1.0f;
+    rec[c] = hits == 0 ? 0u : (whi - wlo >= 8 ? kTestAgain : ((uint32_t)wlo << 8) | mask);
   }
-  const uint32_t r = run_of[i];
-  codes[r] = chunk_base | code;
-  const uint32_t packed = pack_normal(s0, s1, s2);
-  attribs[r] = svo_attrib{packed, packed};  // colour = normal * 0.5 + 0.5 = the packed normal
+  __shared__ uint32_t warp_hits[kColThreads / 32];
+  const uint32_t sum = __reduce_add_sync(0xFFFFFFFFu, hits);
+  if (threadIdx.x % 32 == 0) warp_hits[threadIdx.x / 32] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint64_t n = 0;
+    for (int i = 0; i < kColThreads / 32; ++i) n += warp_hits[i];
+    block_hits[blockIdx.x] = n;
+    if (blockIdx.x == gridDim.x - 1) block_hits[gridDim.x] = 0;  // the sum's total lands here
+  }
 }
+
+__global__ void __launch_bounds__(kColThreads) column_emit_kernel(
+    const float* __restrict__ V, const uint32_t* __restrict__ T, uint64_t nt, uint32_t depth,
+    Chunk ch, const uint64_t* __restrict__ off, uint64_t columns, const uint32_t* __restrict__ rec,
+    const uint64_t* __restrict__ block_off, uint64_t* __restrict__ keys) {
+  const uint64_t c = (uint64_t)blockIdx.x * kColThreads + threadIdx.x;
+  const uint64_t t = column_triangle(off, nt, columns, c);
+  const uint32_t r = c < columns ? rec[c] : 0u;
+  TriWalk s;
+  int iu = 0, iv = 0, wlo = 0, whi = -1;
+  uint32_t n = 0;
+  if (r != 0u) {
+    tri_walk(V, T, t, depth, ch, s);
+    const uint64_t k = c - off[t];
+    iu = s.ulo + (int)(k / s.nv);
+    iv = s.vlo + (int)(k % s.nv);
+    if (r == kTestAgain) {
+      column_range(s, depth, ch, iu, iv, &wlo, &whi);
+      for (int iw = wlo; iw <= whi; ++iw) {
+        uint32_t ijk[3];
+        voxel_of(s, iu, iv, iw, ijk);
+        n += voxel_hit(s, depth, ijk) ? 1u : 0u;
+      }
+    } else {
+      wlo = (int)(r >> 8);
+      n = (uint32_t)__popc(r & 0xFFu);
+    }
+  }
+  // exclusive position inside the block
+  __shared__ uint32_t warp_sum[kColThreads / 32];
+  const uint32_t lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+  uint32_t x = n;
+  for (uint32_t d = 1; d < 32; d <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
+    if (lane >= d) x += y;
+  }
+  if (lane == 31) warp_sum[warp] = x;
+  __syncthreads();
+  uint64_t pos = block_off[blockIdx.x] + (x - n);
+  for (uint32_t i = 0; i < warp; ++i) pos += warp_sum[i];
+  if (r == 0u) return;
+  const uint64_t low = ch.shift >= 64 ? ~0ull : ((1ull << ch.shift) - 1ull);
+  auto put = [&](int iw) {
+    uint32_t ijk[3];
+    voxel_of(s, iu, iv, iw, ijk);
+    keys[pos++] = ((morton3(ijk[0], ijk[1], ijk[2]) & low) << ch.tri_bits) | t;
+  };
+  if (r == kTestAgain) {
+    for (int iw = wlo; iw <= whi; ++iw) {
+      uint32_t ijk[3];
+      voxel_of(s, iu, iv, iw, ijk);
+      if (voxel_hit(s, depth, ijk)) put(iw);
+    }
+  } else {
+    for (uint32_t m = r & 0xFFu; m != 0u; m &= m - 1u) put(wlo + __ffs((int)m) - 1);
+  }
+}
+
+// ---- 3. levels from the sorted keys ------------------------------------------------
+
+constexpr int kMaxLevels = 22;
+
+// The coarsest level that begins a node at key i: a node of level d holds the
+// keys with the same leading d octal digits of their codes.  depth + 1 where
+// the code is the one before (another triangle of the same voxel).
+struct KeyLevels {
+  const uint64_t* keys;
+  uint64_t n;
+  uint32_t tri_bits, depth;
+  uint32_t first_level;  // at the chunk's first key
+  __device__ __forceinline__ uint32_t operator()(uint64_t i) const {
+    if (i >= n) return depth + 1u;
+    if (i == 0) return first_level;
+    const uint64_t diff = (keys[i] ^ keys[i - 1]) >> tri_bits;
+    return diff == 0 ? depth + 1u : depth - (uint32_t)(63 - __clzll((long long)diff)) / 3u;
+  }
+};
+
+constexpr int kKeyThreads = 256;
+constexpr int kKeyRows = 4;  // a block takes 4 rows of 256 keys
+constexpr int kKeyBlock = kKeyThreads * kKeyRows;
+
+// counts[d * nblocks + block]: the nodes of level d that begin in the block.
+__global__ void __launch_bounds__(kKeyThreads) level_count_kernel(KeyLevels kl, uint64_t nblocks,
+                                                                  uint32_t* __restrict__ counts) {
+  __shared__ uint32_t sums[kMaxLevels];
+  if (threadIdx.x < kMaxLevels) sums[threadIdx.x] = 0;
+  __syncthreads();
+  uint32_t k[kKeyRows];
+#pragma unroll
+  for (int r = 0; r < kKeyRows; ++r)
+    k[r] = kl((uint64_t)blockIdx.x * kKeyBlock + r * kKeyThreads + threadIdx.x);
+  for (uint32_t d = 0; d <= kl.depth; ++d) {
+    uint32_t n = 0;
+#pragma unroll
+    for (int r = 0; r < kKeyRows; ++r) n += (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, k[r] <= d));
+    if (threadIdx.x % 32 == 0 && n) atomicAdd(&sums[d], n);
+  }
+  __syncthreads();
+  if (threadIdx.x <= kl.depth) counts[threadIdx.x * nblocks + blockIdx.x] = sums[threadIdx.x];
+}
+
+// One block per level: counts become the level's node index at each key block,
+// on from totals[level], which is advanced by the chunk's nodes.
+__global__ void __launch_bounds__(1024) level_scan_kernel(uint32_t* __restrict__ counts,
+                                                          uint64_t nblocks,
+                                                          uint64_t* __restrict__ totals) {
+  uint32_t* c = counts + (uint64_t)blockIdx.x * nblocks;
+  __shared__ uint32_t warp_sum[32];
+  __shared__ uint64_t carry;
+  const uint32_t lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+  if (threadIdx.x == 0) carry = totals[blockIdx.x];
+  constexpr uint32_t kItems = 4;
+  for (uint64_t base = 0; base < nblocks; base += 1024 * kItems) {
+    uint32_t v[kItems], sum = 0;
+    for (uint32_t k = 0; k < kItems; ++k) {
+      const uint64_t i = base + threadIdx.x * kItems + k;
+      v[k] = i < nblocks ? c[i] : 0u;
+      sum += v[k];
+    }
+    uint32_t x = sum;
+    for (uint32_t d = 1; d < 32; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
+      if (lane >= d) x += y;
+    }
+    if (lane == 31) warp_sum[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+      uint32_t y = warp_sum[lane];
+      for (uint32_t d = 1; d < 32; d <<= 1) {
+        const uint32_t z = __shfl_up_sync(0xFFFFFFFFu, y, d);
+        if (lane >= d) y += z;
+      }
+      warp_sum[lane] = y;
+    }
+    __syncthreads();
+    uint64_t at = carry + (warp ? warp_sum[warp - 1] : 0u) + (x - sum);
+    for (uint32_t k = 0; k < kItems; ++k) {
+      const uint64_t i = base + threadIdx.x * kItems + k;
+      if (i < nblocks) c[i] = (uint32_t)at;  // below 2^32: the totals are looked at before use
+      at += v[k];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) carry += warp_sum[31];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) totals[blockIdx.x] = carry;
+}
+
+// A chunk's part of the levels, indexed by a level's node index less base[level].
+struct LevelOut {
+  uint32_t* first[kMaxLevels];  // a node's first child; levels above the leaves
+  uint8_t* octant[kMaxLevels];  // a node's place in its parent
+  svo_attrib* leaf_attribs;
+  uint32_t base[kMaxLevels];
+};
 
 __device__ __forceinline__ uint32_t compact3(uint64_t x) {
   x &= 0x1249249249249249ull;
@@ -341,99 +602,84 @@ __device__ __forceinline__ uint32_t compact3(uint64_t x) {
   return (uint32_t)x;
 }
 
-// leaf_contribution of the host builder (csrc/scene.cpp), operation for
-// operation: the reference's interpolated vertex normal and colour of one
-// triangle at the voxel centre c.
-__device__ void leaf_contribution(const float* __restrict__ V, const float* __restrict__ N,
-                                  const float* __restrict__ C, const uint32_t* tri,
-                                  const float c[3], float n_out[3], float c_out[3]) {
-  const float* p0 = V + 3 * (uint64_t)tri[0];
-  const float* p1 = V + 3 * (uint64_t)tri[1];
-  const float* p2 = V + 3 * (uint64_t)tri[2];
-  const float* n0 = N + 3 * (uint64_t)tri[0];
-  const float* n1 = N + 3 * (uint64_t)tri[1];
-  const float* n2 = N + 3 * (uint64_t)tri[2];
-  const float* c0 = C + 3 * (uint64_t)tri[0];
-  const float* c1 = C + 3 * (uint64_t)tri[1];
-  const float* c2 = C + 3 * (uint64_t)tri[2];
-  float d[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) d[k] = __fdiv_rn(__fadd_rn(__fadd_rn(n0[k], n1[k]), n2[k]), 3.0f);
-  float len = len3(d[0], d[1], d[2]);
-  if (len > 0.0f) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) d[k] = __fdiv_rn(d[k], len);
-  }
-  const float e1[3] = {__fsub_rn(p1[0], p0[0]), __fsub_rn(p1[1], p0[1]), __fsub_rn(p1[2], p0[2])};
-  const float e2[3] = {__fsub_rn(p2[0], p0[0]), __fsub_rn(p2[1], p0[1]), __fsub_rn(p2[2], p0[2])};
-  const float pv[3] = {__fsub_rn(__fmul_rn(d[1], e2[2]), __fmul_rn(d[2], e2[1])),
-                       __fsub_rn(__fmul_rn(d[2], e2[0]), __fmul_rn(d[0], e2[2])),
-                       __fsub_rn(__fmul_rn(d[0], e2[1]), __fmul_rn(d[1], e2[0]))};
-  const float det = dot3(e1[0], e1[1], e1[2], pv);
+// What the leaves' attributes are made of: face normals, or the triangles'
+// records where the mesh has vertex normals and colours (records != nullptr).
+struct LeafInput {
+  const float* face_normals;
+  const TriRecord* records;
+  uint64_t chunk_base;  // the code bits above the key's
+};
+
+// The reference's interpolated vertex normal and colour of one triangle at the
+// voxel centre c (leaf_contribution of the host builder, operation for
+// operation; the voxel-independent part is in the record).
+__device__ __forceinline__ void leaf_contribution(const TriRecord& r, const float c[3],
+                                                  float n_out[3], float c_out[3]) {
   float u = 0.0f, v = 0.0f;
-  if (!(det > -1e-8f && det < 1e-8f)) {
-    const float inv = __fdiv_rn(1.0f, det);
-    const float tv[3] = {__fsub_rn(c[0], p0[0]), __fsub_rn(c[1], p0[1]), __fsub_rn(c[2], p0[2])};
-    u = __fmul_rn(dot3(tv[0], tv[1], tv[2], pv), inv);
-    const float qv[3] = {__fsub_rn(__fmul_rn(tv[1], e1[2]), __fmul_rn(tv[2], e1[1])),
-                         __fsub_rn(__fmul_rn(tv[2], e1[0]), __fmul_rn(tv[0], e1[2])),
-                         __fsub_rn(__fmul_rn(tv[0], e1[1]), __fmul_rn(tv[1], e1[0]))};
-    v = __fmul_rn(dot3(d[0], d[1], d[2], qv), inv);
+  if (r.hits != 0.0f) {
+    const float tv[3] = {__fsub_rn(c[0], r.p0[0]), __fsub_rn(c[1], r.p0[1]),
+                         __fsub_rn(c[2], r.p0[2])};
+    u = __fmul_rn(dot3(tv[0], tv[1], tv[2], r.pv), r.inv);
+    const float qv[3] = {__fsub_rn(__fmul_rn(tv[1], r.e1[2]), __fmul_rn(tv[2], r.e1[1])),
+                         __fsub_rn(__fmul_rn(tv[2], r.e1[0]), __fmul_rn(tv[0], r.e1[2])),
+                         __fsub_rn(__fmul_rn(tv[0], r.e1[1]), __fmul_rn(tv[1], r.e1[0]))};
+    v = __fmul_rn(dot3(r.d[0], r.d[1], r.d[2], qv), r.inv);
   }
   u = u < 0.0f ? 0.0f : (u > 1.0f ? 1.0f : u);
   v = v < 0.0f ? 0.0f : (v > 1.0f ? 1.0f : v);
   const float w = __fsub_rn(__fsub_rn(1.0f, u), v);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    n_out[k] = __fadd_rn(__fadd_rn(__fmul_rn(n0[k], w), __fmul_rn(n1[k], u)), __fmul_rn(n2[k], v));
-    c_out[k] = __fadd_rn(__fadd_rn(__fmul_rn(c0[k], w), __fmul_rn(c1[k], u)), __fmul_rn(c2[k], v));
+    n_out[k] = __fadd_rn(__fadd_rn(__fmul_rn(r.n0[k], w), __fmul_rn(r.n1[k], u)), __fmul_rn(r.n2[k], v));
+    c_out[k] = __fadd_rn(__fadd_rn(__fmul_rn(r.c0[k], w), __fmul_rn(r.c1[k], u)), __fmul_rn(r.c2[k], v));
   }
-  len = len3(n_out[0], n_out[1], n_out[2]);
+  const float len = len3(n_out[0], n_out[1], n_out[2]);
   if (len > 0.0f) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) n_out[k] = __fdiv_rn(n_out[k], len);
   }
 }
 
-// One thread per run of equal codes, with per-vertex attributes: the mean of
-// the triangles' interpolated normals (normalised) and colours.
-__global__ void leaf_reduce_attr_kernel(const uint64_t* __restrict__ keys, uint64_t n,
-                                        uint32_t tri_bits, uint64_t chunk_base, uint32_t depth,
-                                        const uint32_t* __restrict__ heads,
-                                        const uint32_t* __restrict__ run_of,
-                                        const float* __restrict__ V, const float* __restrict__ N,
-                                        const float* __restrict__ C,
-                                        const uint32_t* __restrict__ T,
-                                        uint64_t* __restrict__ codes,
-                                        svo_attrib* __restrict__ attribs) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || !heads[i]) return;
-  const uint64_t code = keys[i] >> tri_bits;
-  const uint64_t full = chunk_base | code;
-  const uint64_t tmask = (1ull << tri_bits) - 1ull;
-  const float inv_r = __fdiv_rn(1.0f, (float)(1u << depth));
+// The attributes of the leaf whose first key is i: over its triangles in order,
+// the mean of the interpolated normals (normalised) and colours, or the
+// normalised sum of the face normals.
+__device__ __forceinline__ svo_attrib leaf_attrib(const KeyLevels& kl, const LeafInput& in,
+                                                  uint64_t i) {
+  const uint64_t code = kl.keys[i] >> kl.tri_bits;
+  const uint64_t tmask = (1ull << kl.tri_bits) - 1ull;
+  const uint64_t full = in.chunk_base | code;
+  const float inv_r = __fdiv_rn(1.0f, (float)(1u << kl.depth));
   const uint32_t x = compact3(full >> 2), y = compact3(full >> 1), z = compact3(full);
   const float c[3] = {__fadd_rn(-0.5f, __fmul_rn(__fadd_rn((float)x, 0.5f), inv_r)),
                       __fadd_rn(-0.5f, __fmul_rn(__fadd_rn((float)y, 0.5f), inv_r)),
                       __fadd_rn(-0.5f, __fmul_rn(__fadd_rn((float)z, 0.5f), inv_r))};
   float sn[3] = {0.0f, 0.0f, 0.0f}, sc[3] = {0.0f, 0.0f, 0.0f};
-  uint64_t j = i;
+  uint64_t j = i, key = kl.keys[i];
   do {
-    const uint64_t t = keys[j] & tmask;
-    float nn[3], cc[3];
-    leaf_contribution(V, N, C, T + 3 * t, c, nn, cc);
+    const uint64_t t = key & tmask;
+    float nn[3], cc[3] = {0.0f, 0.0f, 0.0f};
+    if (in.records != nullptr) {
+      const TriRecord r = in.records[t];
+      leaf_contribution(r, c, nn, cc);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) nn[k] = in.face_normals[3 * t + k];
+    }
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       sn[k] = __fadd_rn(sn[k], nn[k]);
       sc[k] = __fadd_rn(sc[k], cc[k]);
     }
     ++j;
-  } while (j < n && (keys[j] >> tri_bits) == code);
-  const float cnt = (float)(j - i);
+    if (j < kl.n) key = kl.keys[j];
+  } while (j < kl.n && (key >> kl.tri_bits) == code);
+  if (in.records != nullptr) {
+    const float cnt = (float)(j - i);
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    sn[k] = __fdiv_rn(sn[k], cnt);
-    sc[k] = __fdiv_rn(sc[k], cnt);
+    for (int k = 0; k < 3; ++k) {
+      sn[k] = __fdiv_rn(sn[k], cnt);
+      sc[k] = __fdiv_rn(sc[k], cnt);
+    }
   }
   const float len = len3(sn[0], sn[1], sn[2]);
   if (len > 0.0f) {
@@ -444,47 +690,94 @@ __global__ void leaf_reduce_attr_kernel(const uint64_t* __restrict__ keys, uint6
     sn[1] = 0.0f;
     sn[2] = 1.0f;
   }
-  const uint32_t r = run_of[i];
-  codes[r] = full;
-  attribs[r] = svo_attrib{pack_normal(sn[0], sn[1], sn[2]), pack_color(sc[0], sc[1], sc[2])};
+  const uint32_t normal = pack_normal(sn[0], sn[1], sn[2]);
+  // without vertex colours, colour = normal * 0.5 + 0.5 = the packed normal
+  return svo_attrib{normal, in.records != nullptr ? pack_color(sc[0], sc[1], sc[2]) : normal};
 }
 
-// ---- 4. levels -------------------------------------------------------------------
-
-__global__ void parent_heads_kernel(const uint64_t* __restrict__ codes, uint64_t n,
-                                    uint32_t* __restrict__ heads) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  heads[i] = (i == 0 || (codes[i] >> 3) != (codes[i - 1] >> 3)) ? 1u : 0u;
+// Every level's nodes that begin in the block, and the leaves' attributes.
+__global__ void __launch_bounds__(kKeyThreads) level_write_kernel(
+    KeyLevels kl, LeafInput in, uint64_t nblocks, const uint32_t* __restrict__ counts, LevelOut out) {
+  // before[d][g]: the nodes of level d that begin in the block ahead of group g
+  // (a row's warp)
+  constexpr int kGroups = kKeyRows * kKeyThreads / 32;
+  static_assert(kGroups == 32, "one warp scans the groups of a level");
+  __shared__ uint32_t before[kMaxLevels][kGroups];
+  const uint32_t lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+  uint32_t k[kKeyRows];
+#pragma unroll
+  for (int r = 0; r < kKeyRows; ++r)
+    k[r] = kl((uint64_t)blockIdx.x * kKeyBlock + r * kKeyThreads + threadIdx.x);
+  for (uint32_t d = 0; d <= kl.depth; ++d) {
+#pragma unroll
+    for (int r = 0; r < kKeyRows; ++r) {
+      const uint32_t b = __ballot_sync(0xFFFFFFFFu, k[r] <= d);
+      if (lane == 0) before[d][r * (kKeyThreads / 32) + warp] = (uint32_t)__popc(b);
+    }
+  }
+  __syncthreads();
+  for (uint32_t d = warp; d <= kl.depth; d += kKeyThreads / 32) {
+    const uint32_t n = before[d][lane];
+    uint32_t x = n;
+    for (uint32_t s = 1; s < 32; s <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, s);
+      if (lane >= s) x += y;
+    }
+    before[d][lane] = counts[d * nblocks + blockIdx.x] - out.base[d] + x - n;
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int r = 0; r < kKeyRows; ++r) {
+    const uint64_t i = (uint64_t)blockIdx.x * kKeyBlock + r * kKeyThreads + threadIdx.x;
+    const uint32_t kr = k[0];
+    k[0] = k[1];
+    k[1] = k[2];
+    k[2] = k[3];
+    const uint64_t code = kr <= kl.depth ? in.chunk_base | (kl.keys[i] >> kl.tri_bits) : 0;
+    uint32_t up = 0;  // the node's index one level up
+    for (uint32_t d = 0; d <= kl.depth; ++d) {
+      const uint32_t b = __ballot_sync(0xFFFFFFFFu, kr <= d);
+      if (kr > d) continue;
+      const uint32_t at = before[d][r * (kKeyThreads / 32) + warp] + __popc(b & ((1u << lane) - 1u));
+      if (kr < d) out.first[d - 1][up] = at + out.base[d];
+      out.octant[d][at] = (uint8_t)((code >> (3 * (kl.depth - d))) & 7u);
+      up = at;
+    }
+    if (kr <= kl.depth) out.leaf_attribs[up] = leaf_attrib(kl, in, i);
+  }
 }
 
-// One thread per parent (host: octree_from_leaves' inner loop).
-__global__ void parent_reduce_kernel(const uint64_t* __restrict__ cc,
-                                     const svo_attrib* __restrict__ ca, uint64_t n,
-                                     const uint32_t* __restrict__ heads,
-                                     const uint32_t* __restrict__ run_of,
-                                     uint64_t* __restrict__ pc, uint8_t* __restrict__ pm,
-                                     uint32_t* __restrict__ pf, svo_attrib* __restrict__ pa) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || !heads[i]) return;
-  const uint64_t parent = cc[i] >> 3;
+// ---- 4. inner attributes ---------------------------------------------------------
+
+// One thread per parent (host: octree_from_leaves' inner loop): the valid mask
+// and the mean of the children's attributes, in order.  An attribute byte is one
+// of 256 values, so its unpacked forms (a division by 255 each on the host) are
+// read from two tables.
+constexpr int kParentThreads = 256;
+__global__ void __launch_bounds__(kParentThreads) parent_kernel(
+    const uint32_t* __restrict__ first, uint32_t n, uint32_t children,
+    const uint8_t* __restrict__ octant, const svo_attrib* __restrict__ ca,
+    uint8_t* __restrict__ masks, svo_attrib* __restrict__ pa) {
+  __shared__ float col[256], nrm[256];
+  col[threadIdx.x] = __fdiv_rn((float)threadIdx.x, 255.0f);
+  nrm[threadIdx.x] = __fmul_rn(__fsub_rn(col[threadIdx.x], 0.5f), 2.0f);
+  __syncthreads();
+  const uint32_t p = blockIdx.x * kParentThreads + threadIdx.x;
+  if (p >= n) return;
+  const uint32_t f = first[p], end = p + 1 < n ? first[p + 1] : children;
   uint32_t mask = 0;
   float n0 = 0.0f, n1 = 0.0f, n2 = 0.0f, c0 = 0.0f, c1 = 0.0f, c2 = 0.0f;
-  uint64_t j = i;
-  do {
-    mask |= 1u << (uint32_t)(cc[j] & 7u);
-    float v[3];
-    unpack_color(ca[j].packed_normal, v);
-    n0 = __fadd_rn(n0, __fmul_rn(__fsub_rn(v[0], 0.5f), 2.0f));
-    n1 = __fadd_rn(n1, __fmul_rn(__fsub_rn(v[1], 0.5f), 2.0f));
-    n2 = __fadd_rn(n2, __fmul_rn(__fsub_rn(v[2], 0.5f), 2.0f));
-    unpack_color(ca[j].packed_color, v);
-    c0 = __fadd_rn(c0, v[0]);
-    c1 = __fadd_rn(c1, v[1]);
-    c2 = __fadd_rn(c2, v[2]);
-    ++j;
-  } while (j < n && (cc[j] >> 3) == parent);
-  const float cnt = (float)(j - i);
+  for (uint32_t j = f; j < end; ++j) {
+    mask |= 1u << octant[j];
+    const svo_attrib a = ca[j];
+    n0 = __fadd_rn(n0, nrm[a.packed_normal >> 24]);
+    n1 = __fadd_rn(n1, nrm[(a.packed_normal >> 16) & 255u]);
+    n2 = __fadd_rn(n2, nrm[(a.packed_normal >> 8) & 255u]);
+    c0 = __fadd_rn(c0, col[a.packed_color >> 24]);
+    c1 = __fadd_rn(c1, col[(a.packed_color >> 16) & 255u]);
+    c2 = __fadd_rn(c2, col[(a.packed_color >> 8) & 255u]);
+  }
+  const float cnt = (float)(end - f);
   n0 = __fdiv_rn(n0, cnt);
   n1 = __fdiv_rn(n1, cnt);
   n2 = __fdiv_rn(n2, cnt);
@@ -501,16 +794,11 @@ __global__ void parent_reduce_kernel(const uint64_t* __restrict__ cc,
     n1 = 0.0f;
     n2 = 1.0f;
   }
-  const uint32_t r = run_of[i];
-  pc[r] = parent;
-  pm[r] = (uint8_t)mask;
-  pf[r] = (uint32_t)i;
-  pa[r] = svo_attrib{pack_normal(n0, n1, n2), pack_color(c0, c1, c2)};
+  masks[p] = (uint8_t)mask;
+  pa[p] = svo_attrib{pack_normal(n0, n1, n2), pack_color(c0, c1, c2)};
 }
 
 // ---- 5. treelet cut ------------------------------------------------------------
-
-constexpr int kMaxLevels = 22;
 
 struct LevelPtrs {
   const uint8_t* masks[kMaxLevels];
@@ -567,7 +855,7 @@ __global__ void treelet_sizes_kernel(LevelPtrs L, CutParams cp, uint32_t num_tre
 // One block per treelet: its slot (slot = gid, as insert_all fills an empty
 // pool) with every sub-treelet root copied into this treelet's leaf and
 // re-pointed (insert_treelet's patch), leaf flags of resident sub-treelets
-// cleared, tail left zero.
+// cleared, tail zero.
 __global__ void __launch_bounds__(256) cut_kernel(LevelPtrs L, CutParams cp,
                                                   uint32_t num_treelets,
                                                   uint2* __restrict__ nodes,
@@ -618,55 +906,173 @@ __global__ void __launch_bounds__(256) cut_kernel(LevelPtrs L, CutParams cp,
       nodes[base + p] = rec;
     }
   }
+  // the rest of the slot: the pool is written once, without clearing it first
+  const uint64_t used = off[s - r] + (hi[s - r] - lo[s - r]);
+  for (uint64_t p = used + threadIdx.x; p < cp.N; p += blockDim.x) {
+    nodes[base + p] = make_uint2(0u, 0u);
+    attribs[base + p] = svo_attrib{0u, 0u};
+  }
 }
 
 // ---- host side -----------------------------------------------------------------------
 
+// Columns of one chunk: 2 GB of records, about 5 GB of keys.
+constexpr uint64_t kMaxColumns = 1ull << 29;
+constexpr int kMaxDevices = 64;
+
+// What builds keep between them, per device.  Scratch: a stream-ordered memory
+// pool that holds on to at most kScratchKeep (allocating and freeing device
+// memory took 50 of the 70 ms of a depth-11 build).  Pools of destroyed scenes:
+// at most kPoolKeep, plain cudaMalloc memory like every scene's pool, for the
+// next scene of about that size.  Both go back to the device when the last
+// scene is destroyed.
+constexpr uint64_t kScratchKeep = 1ull << 30;
+constexpr uint64_t kPoolKeep = 1ull << 30;
+struct KeptPool {
+  void* p;
+  uint64_t bytes;
+};
+struct Kept {
+  std::mutex mu;
+  cudaMemPool_t scratch = nullptr;
+  std::vector<KeptPool> pools;
+  uint64_t pool_bytes = 0;
+  uint64_t users = 0;  // scenes alive and builds running
+};
+Kept g_kept[kMaxDevices];
+
+cudaError_t scratch_pool(int dev, cudaMemPool_t* out) {
+  Kept& k = g_kept[dev];
+  std::lock_guard<std::mutex> lock(k.mu);
+  if (!k.scratch) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    cudaError_t e = cudaMemPoolCreate(&pool, &props);
+    if (e != cudaSuccess) return e;
+    uint64_t keep = kScratchKeep;
+    e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+      cudaMemPoolDestroy(pool);
+      return e;
+    }
+    k.scratch = pool;
+  }
+  *out = k.scratch;
+  return cudaSuccess;
+}
+
+void free_kept_pools(Kept& k) {  // k.mu is held
+  for (const KeptPool& p : k.pools) cudaFree(p.p);
+  k.pools.clear();
+  k.pool_bytes = 0;
+}
+
+// Scene pool memory: a kept block of at most a quarter more than asked for, else
+// new memory (after what is kept has been given up, if need be).
+cudaError_t pool_alloc(int dev, uint64_t bytes, void** out, uint64_t* got) {
+  Kept& k = g_kept[dev];
+  std::lock_guard<std::mutex> lock(k.mu);
+  size_t best = k.pools.size();
+  for (size_t i = 0; i < k.pools.size(); ++i)
+    if (k.pools[i].bytes >= bytes && k.pools[i].bytes - bytes <= bytes / 4 &&
+        (best == k.pools.size() || k.pools[i].bytes < k.pools[best].bytes))
+      best = i;
+  if (best < k.pools.size()) {
+    *out = k.pools[best].p;
+    *got = k.pools[best].bytes;
+    k.pool_bytes -= *got;
+    k.pools.erase(k.pools.begin() + (ptrdiff_t)best);
+    return cudaSuccess;
+  }
+  *got = bytes;
+  cudaError_t e = cudaMalloc(out, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    free_kept_pools(k);
+    if (k.scratch) cudaMemPoolTrimTo(k.scratch, 0);
+    e = cudaMalloc(out, bytes);
+  }
+  return e;
+}
+
+// The scene's pool memory, once nothing reads it any more (cudaFree waits for
+// the device; a block that is kept must wait as well).
+void pool_free(int dev, void* p, uint64_t bytes) {
+  if (!p) return;
+  Kept& k = g_kept[dev];
+  std::lock_guard<std::mutex> lock(k.mu);
+  if (k.users > 1 && k.pool_bytes + bytes <= kPoolKeep && cudaDeviceSynchronize() == cudaSuccess) {
+    try {
+      k.pools.push_back({p, bytes});
+      k.pool_bytes += bytes;
+      return;
+    } catch (...) {
+    }
+  }
+  cudaFree(p);
+}
+
+void user_begins(int dev) {
+  std::lock_guard<std::mutex> lock(g_kept[dev].mu);
+  ++g_kept[dev].users;
+}
+
+void user_ends(int dev) {
+  Kept& k = g_kept[dev];
+  std::lock_guard<std::mutex> lock(k.mu);
+  if (--k.users) return;
+  cudaDeviceSynchronize();  // scratch still in use by a failed build
+  free_kept_pools(k);
+  if (k.scratch) cudaMemPoolTrimTo(k.scratch, 0);
+}
+
+// Scratch of one build, ordered on its stream.
+struct Scratch {
+  cudaMemPool_t pool = nullptr;
+  cudaStream_t st = nullptr;
+};
+
 template <class T>
 struct DevBuf {
   T* p = nullptr;
-  size_t n = 0;
+  cudaStream_t st = nullptr;
   DevBuf() = default;
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
-  DevBuf(DevBuf&& o) noexcept : p(o.p), n(o.n) {
-    o.p = nullptr;
-    o.n = 0;
-  }
+  DevBuf(DevBuf&& o) noexcept : p(o.p), st(o.st) { o.p = nullptr; }
   DevBuf& operator=(DevBuf&& o) noexcept {
     if (this != &o) {
       reset();
       p = o.p;
-      n = o.n;
+      st = o.st;
       o.p = nullptr;
-      o.n = 0;
     }
     return *this;
   }
   ~DevBuf() { reset(); }
   void reset() {
-    if (p) cudaFree(p);
+    if (p) cudaFreeAsync(p, st);
     p = nullptr;
-    n = 0;
   }
-  cudaError_t alloc(size_t count) {
+  cudaError_t alloc(const Scratch& s, size_t count) {
     reset();
-    if (count == 0) count = 1;
-    const cudaError_t e = cudaMalloc(&p, count * sizeof(T));
-    if (e != cudaSuccess) {
-      p = nullptr;
-      return e;
-    }
-    n = count;
-    return cudaSuccess;
+    st = s.st;
+    const cudaError_t e =
+        cudaMallocFromPoolAsync((void**)&p, (count ? count : 1) * sizeof(T), s.pool, s.st);
+    if (e != cudaSuccess) p = nullptr;
+    return e;
   }
 };
 
-struct Level {
-  uint64_t size = 0;
-  DevBuf<uint8_t> masks;
-  DevBuf<uint32_t> first;
-  DevBuf<svo_attrib> attribs;
+// The levels of a chunk, or of the whole octree.
+struct Levels {
+  uint64_t size[kMaxLevels] = {};
+  DevBuf<uint32_t> first[kMaxLevels];
+  DevBuf<uint8_t> octant[kMaxLevels];
+  DevBuf<svo_attrib> leaf_attribs;
 };
 
 uint32_t bits_for(uint64_t v) {
@@ -694,20 +1100,35 @@ unsigned grid_of(uint64_t n, unsigned threads) {
   return (unsigned)((n + threads - 1) / threads);
 }
 
-// exclusive sum of u32 flags into u32 positions; returns the total
-int scan_flags(const uint32_t* flags, uint32_t* pos, uint64_t n, uint64_t* total,
-               cudaStream_t st) {
+// In-place exclusive sum of n + 1 counts, the last of them 0; returns the total.
+int sum_counts(const Scratch& sc, uint64_t* counts, uint64_t n, uint64_t* total) {
   size_t bytes = 0;
-  GB_TRY(cub::DeviceScan::ExclusiveSum(nullptr, bytes, flags, pos, n, st));
+  GB_TRY(cub::DeviceScan::ExclusiveSum(nullptr, bytes, counts, counts, n + 1, sc.st));
   DevBuf<uint8_t> tmp;
-  GB_TRY(tmp.alloc(bytes));
-  GB_TRY(cub::DeviceScan::ExclusiveSum(tmp.p, bytes, flags, pos, n, st));
-  uint32_t last_pos = 0, last_flag = 0;
-  GB_TRY(cudaMemcpyAsync(&last_pos, pos + n - 1, 4, cudaMemcpyDeviceToHost, st));
-  GB_TRY(cudaMemcpyAsync(&last_flag, flags + n - 1, 4, cudaMemcpyDeviceToHost, st));
-  GB_TRY(cudaStreamSynchronize(st));
-  *total = (uint64_t)last_pos + last_flag;
+  GB_TRY(tmp.alloc(sc, bytes));
+  GB_TRY(cub::DeviceScan::ExclusiveSum(tmp.p, bytes, counts, counts, n + 1, sc.st));
+  GB_TRY(cudaMemcpyAsync(total, counts + n, 8, cudaMemcpyDeviceToHost, sc.st));
+  GB_TRY(cudaStreamSynchronize(sc.st));
   return SVO_OK;
+}
+
+Chunk chunk_of(uint32_t ci, uint32_t chunk_levels, uint32_t depth, uint32_t tri_bits) {
+  // chunk ci in Morton order: its code prefix is ci
+  uint32_t cxyz[3] = {0, 0, 0};
+  for (uint32_t b = 0; b < chunk_levels; ++b) {
+    cxyz[0] |= ((ci >> (3 * b + 2)) & 1u) << b;
+    cxyz[1] |= ((ci >> (3 * b + 1)) & 1u) << b;
+    cxyz[2] |= ((ci >> (3 * b)) & 1u) << b;
+  }
+  const uint32_t cs = (1u << depth) >> chunk_levels;  // voxels per chunk per axis
+  Chunk ch;
+  for (int k = 0; k < 3; ++k) {
+    ch.lo[k] = (int)(cxyz[k] * cs);
+    ch.hi[k] = (int)((cxyz[k] + 1) * cs) - 1;
+  }
+  ch.shift = 3 * (depth - chunk_levels);
+  ch.tri_bits = tri_bits;
+  return ch;
 }
 
 }  // namespace
@@ -719,175 +1140,213 @@ int DeviceScene::build_mesh(const float* h_vertices, const float* h_normals,
   if (depth_ < 1 || depth_ > 21) return SVO_ERR_RANGE;
   if (nt == 0 || nv == 0) return SVO_ERR_INVALID;
   if ((h_normals == nullptr) != (h_colors == nullptr)) return SVO_ERR_INVALID;
-  for (uint64_t i = 0; i < 3 * nt; ++i)
-    if (h_triangles[i] >= nv) return SVO_ERR_INVALID;
+  uint32_t largest = 0;
+  for (uint64_t i = 0; i < 3 * nt; ++i) largest = std::max(largest, h_triangles[i]);
+  if (largest >= nv) return SVO_ERR_INVALID;
   depth = depth_;
   const uint32_t tri_bits = bits_for(nt);
   // chunk levels: enough that a key (code inside the chunk, triangle) fits 64 bits
-  uint32_t chunk_levels = 1;
+  uint32_t chunk_levels = 0;
   while (chunk_levels < depth && 3 * (depth - chunk_levels) + tri_bits > 64) ++chunk_levels;
   if (chunk_levels > 3 || 3 * (depth - chunk_levels) + tri_bits > 64) return SVO_ERR_RANGE;
-  chunk_levels = std::min(chunk_levels, depth);
+  int dev = 0;
+  GB_TRY(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= kMaxDevices) return SVO_ERR_RANGE;
+  device = dev;
+  user_begins(dev);  // until this scene is destroyed
+  Scratch sc;
+  sc.st = st;
+  GB_TRY(scratch_pool(dev, &sc.pool));
 
   DevBuf<float> dV, dFn, dN, dC;
   DevBuf<uint32_t> dT;
-  GB_TRY(dV.alloc(3 * nv));
-  GB_TRY(dT.alloc(3 * nt));
-  GB_TRY(dFn.alloc(3 * nt));
+  DevBuf<TriRecord> dRec;
+  GB_TRY(dV.alloc(sc, 3 * nv));
+  GB_TRY(dT.alloc(sc, 3 * nt));
   GB_TRY(cudaMemcpyAsync(dV.p, h_vertices, 3 * nv * sizeof(float), cudaMemcpyHostToDevice, st));
-  const bool attributed = h_normals != nullptr;
-  if (attributed) {
-    GB_TRY(dN.alloc(3 * nv));
-    GB_TRY(dC.alloc(3 * nv));
+  GB_TRY(cudaMemcpyAsync(dT.p, h_triangles, 3 * nt * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+  LeafInput leaf_in = {nullptr, nullptr, 0};
+  if (h_normals != nullptr) {
+    GB_TRY(dN.alloc(sc, 3 * nv));
+    GB_TRY(dC.alloc(sc, 3 * nv));
+    GB_TRY(dRec.alloc(sc, nt));
     GB_TRY(cudaMemcpyAsync(dN.p, h_normals, 3 * nv * sizeof(float), cudaMemcpyHostToDevice, st));
     GB_TRY(cudaMemcpyAsync(dC.p, h_colors, 3 * nv * sizeof(float), cudaMemcpyHostToDevice, st));
+    tri_records_kernel<<<grid_of(nt, 128), 128, 0, st>>>(dV.p, dN.p, dC.p, dT.p, nt, dRec.p);
+    leaf_in.records = dRec.p;
+  } else {
+    GB_TRY(dFn.alloc(sc, 3 * nt));
+    face_normals_kernel<<<grid_of(nt, 256), 256, 0, st>>>(dV.p, dT.p, nt, dFn.p);
+    leaf_in.face_normals = dFn.p;
   }
-  GB_TRY(cudaMemcpyAsync(dT.p, h_triangles, 3 * nt * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-  face_normals_kernel<<<grid_of(nt, 256), 256, 0, st>>>(dV.p, dT.p, nt, dFn.p);
   GB_TRY(cudaGetLastError());
-
-  // -- voxelise chunk by chunk; each chunk's leaves are sorted and unique
-  const uint32_t R = 1u << depth;
-  const uint32_t C = 1u << chunk_levels;  // chunks per axis
-  const uint32_t cs = R / C;              // voxels per chunk per axis
-  DevBuf<uint64_t> counts, offsets;
-  GB_TRY(counts.alloc(nt));
-  GB_TRY(offsets.alloc(nt));
-  std::vector<DevBuf<uint64_t>> chunk_codes;
-  std::vector<DevBuf<svo_attrib>> chunk_attr;
-  std::vector<uint64_t> chunk_leaves;
-  const uint32_t num_chunks = C * C * C;
-  for (uint32_t ci = 0; ci < num_chunks; ++ci) {
-    // chunk ci in Morton order: its code prefix is ci
-    uint32_t cxyz[3] = {0, 0, 0};
-    for (uint32_t b = 0; b < chunk_levels; ++b) {
-      cxyz[0] |= ((ci >> (3 * b + 2)) & 1u) << b;
-      cxyz[1] |= ((ci >> (3 * b + 1)) & 1u) << b;
-      cxyz[2] |= ((ci >> (3 * b)) & 1u) << b;
-    }
-    Chunk ch;
-    for (int k = 0; k < 3; ++k) {
-      ch.lo[k] = (int)(cxyz[k] * cs);
-      ch.hi[k] = (int)((cxyz[k] + 1) * cs) - 1;
-    }
-    ch.shift = 3 * (depth - chunk_levels);
-    ch.tri_bits = tri_bits;
-    voxel_count_kernel<<<grid_of(nt, 128), 128, 0, st>>>(dV.p, dT.p, nt, depth, ch, counts.p);
-    GB_TRY(cudaGetLastError());
-    size_t bytes = 0;
-    GB_TRY(cub::DeviceScan::ExclusiveSum(nullptr, bytes, counts.p, offsets.p, nt, st));
-    {
-      DevBuf<uint8_t> tmp;
-      GB_TRY(tmp.alloc(bytes));
-      GB_TRY(cub::DeviceScan::ExclusiveSum(tmp.p, bytes, counts.p, offsets.p, nt, st));
-    }
-    uint64_t last_off = 0, last_cnt = 0;
-    GB_TRY(cudaMemcpyAsync(&last_off, offsets.p + nt - 1, 8, cudaMemcpyDeviceToHost, st));
-    GB_TRY(cudaMemcpyAsync(&last_cnt, counts.p + nt - 1, 8, cudaMemcpyDeviceToHost, st));
-    GB_TRY(cudaStreamSynchronize(st));
-    const uint64_t P = last_off + last_cnt;
-    pairs += P;
-    chunk_codes.emplace_back();
-    chunk_attr.emplace_back();
-    chunk_leaves.push_back(0);
-    if (P == 0) continue;
-    DevBuf<uint64_t> keys, sorted;
-    GB_TRY(keys.alloc(P));
-    GB_TRY(sorted.alloc(P));
-    voxel_emit_kernel<<<grid_of(nt, 128), 128, 0, st>>>(dV.p, dT.p, nt, depth, ch, offsets.p,
-                                                       keys.p);
-    GB_TRY(cudaGetLastError());
-    bytes = 0;
-    const int end_bit = (int)(ch.shift + tri_bits);
-    GB_TRY(cub::DeviceRadixSort::SortKeys(nullptr, bytes, keys.p, sorted.p, P, 0, end_bit, st));
-    {
-      DevBuf<uint8_t> tmp;
-      GB_TRY(tmp.alloc(bytes));
-      GB_TRY(cub::DeviceRadixSort::SortKeys(tmp.p, bytes, keys.p, sorted.p, P, 0, end_bit, st));
-    }
-    keys.reset();
-    DevBuf<uint32_t> heads, run_of;
-    GB_TRY(heads.alloc(P));
-    GB_TRY(run_of.alloc(P));
-    run_heads_kernel<<<grid_of(P, 256), 256, 0, st>>>(sorted.p, P, tri_bits, heads.p);
-    GB_TRY(cudaGetLastError());
-    uint64_t M = 0;
-    int rc = scan_flags(heads.p, run_of.p, P, &M, st);
-    if (rc != SVO_OK) return rc;
-    GB_TRY(chunk_codes.back().alloc(M));
-    GB_TRY(chunk_attr.back().alloc(M));
-    if (attributed)
-      leaf_reduce_attr_kernel<<<grid_of(P, 256), 256, 0, st>>>(
-          sorted.p, P, tri_bits, (uint64_t)ci << ch.shift, depth, heads.p, run_of.p, dV.p, dN.p,
-          dC.p, dT.p, chunk_codes.back().p, chunk_attr.back().p);
-    else
-      leaf_reduce_kernel<<<grid_of(P, 256), 256, 0, st>>>(
-          sorted.p, P, tri_bits, (uint64_t)ci << ch.shift, heads.p, run_of.p, dFn.p,
-          chunk_codes.back().p, chunk_attr.back().p);
-    GB_TRY(cudaGetLastError());
-    chunk_leaves.back() = M;
-  }
-  counts.reset();
-  offsets.reset();
-  dV.reset();
-  dT.reset();
-  dFn.reset();
   dN.reset();
   dC.reset();
 
-  // -- concatenate the chunks' leaves
-  leaf_voxels = 0;
-  for (uint64_t m : chunk_leaves) leaf_voxels += m;
-  if (leaf_voxels == 0) return SVO_ERR_INVALID;
-  if (leaf_voxels > 0xFFFFFFFFull) return SVO_ERR_RANGE;
-  std::vector<Level> levels(depth + 1);
-  DevBuf<uint64_t> codes;
-  GB_TRY(codes.alloc(leaf_voxels));
-  GB_TRY(levels[depth].attribs.alloc(leaf_voxels));
-  {
-    uint64_t at = 0;
-    for (uint32_t ci = 0; ci < num_chunks; ++ci) {
-      const uint64_t m = chunk_leaves[ci];
-      if (m == 0) continue;
-      GB_TRY(cudaMemcpyAsync(codes.p + at, chunk_codes[ci].p, m * 8, cudaMemcpyDeviceToDevice, st));
-      GB_TRY(cudaMemcpyAsync(levels[depth].attribs.p + at, chunk_attr[ci].p, m * 8,
-                             cudaMemcpyDeviceToDevice, st));
-      at += m;
-    }
-    GB_TRY(cudaStreamSynchronize(st));
-    chunk_codes.clear();
-    chunk_attr.clear();
-  }
-  levels[depth].size = leaf_voxels;
-
-  // -- levels bottom-up
-  for (int d = (int)depth - 1; d >= 0; --d) {
-    const uint64_t n = levels[d + 1].size;
-    DevBuf<uint32_t> heads, run_of;
-    GB_TRY(heads.alloc(n));
-    GB_TRY(run_of.alloc(n));
-    parent_heads_kernel<<<grid_of(n, 256), 256, 0, st>>>(codes.p, n, heads.p);
+  // -- voxels and levels, chunk by chunk; a chunk's leaves are sorted and unique
+  DevBuf<uint64_t> cols, d_totals;
+  GB_TRY(cols.alloc(sc, nt + 1));
+  GB_TRY(d_totals.alloc(sc, kMaxLevels));
+  GB_TRY(cudaMemsetAsync(d_totals.p, 0, kMaxLevels * sizeof(uint64_t), st));
+  std::vector<Levels> parts;
+  uint64_t totals[kMaxLevels] = {};
+  auto count_columns = [&](const Chunk& ch, uint64_t* n) -> int {
+    column_count_kernel<<<grid_of(nt + 1, 128), 128, 0, st>>>(dV.p, dT.p, nt, depth, ch, cols.p);
     GB_TRY(cudaGetLastError());
-    uint64_t np = 0;
-    int rc = scan_flags(heads.p, run_of.p, n, &np, st);
+    return sum_counts(sc, cols.p, nt, n);
+  };
+  uint64_t columns = 0;
+  Chunk ch = chunk_of(0, chunk_levels, depth, tri_bits);
+  int rc = count_columns(ch, &columns);
+  if (rc != SVO_OK) return rc;
+  if (chunk_levels == 0 && columns > kMaxColumns && depth > 1) {
+    // the columns spread over 8^levels cells, about half of them empty
+    while (chunk_levels < std::min(depth - 1, 3u) && (columns >> (2 * chunk_levels)) > kMaxColumns)
+      ++chunk_levels;
+    ch = chunk_of(0, chunk_levels, depth, tri_bits);
+    rc = count_columns(ch, &columns);
     if (rc != SVO_OK) return rc;
-    DevBuf<uint64_t> pcodes;
-    Level& lv = levels[d];
-    GB_TRY(pcodes.alloc(np));
-    GB_TRY(lv.masks.alloc(np));
-    GB_TRY(lv.first.alloc(np));
-    GB_TRY(lv.attribs.alloc(np));
-    parent_reduce_kernel<<<grid_of(n, 256), 256, 0, st>>>(codes.p, levels[d + 1].attribs.p, n,
-                                                          heads.p, run_of.p, pcodes.p, lv.masks.p,
-                                                          lv.first.p, lv.attribs.p);
-    GB_TRY(cudaGetLastError());
-    lv.size = np;
-    codes = std::move(pcodes);
   }
-  if (levels[0].size != 1) return SVO_ERR_INVALID;
-  codes.reset();
-  octree_nodes = 0;
-  for (const Level& lv : levels) octree_nodes += lv.size;
+  const uint32_t num_chunks = 1u << (3 * chunk_levels);
+  uint32_t last_chunk = 0;  // the last chunk with leaves
+  for (uint32_t ci = 0; ci < num_chunks; ++ci) {
+    if (ci > 0) {
+      ch = chunk_of(ci, chunk_levels, depth, tri_bits);
+      rc = count_columns(ch, &columns);
+      if (rc != SVO_OK) return rc;
+    }
+    if (columns == 0) continue;
+    const uint64_t col_blocks = (columns + kColThreads - 1) / kColThreads;
+    if (col_blocks > 0x7FFFFFFFull) return SVO_ERR_RANGE;
+    DevBuf<uint64_t> keys, keys2;
+    uint64_t P = 0;
+    {
+      DevBuf<uint32_t> rec;
+      DevBuf<uint64_t> block_hits;
+      GB_TRY(rec.alloc(sc, columns));
+      GB_TRY(block_hits.alloc(sc, col_blocks + 1));
+      column_test_kernel<<<(unsigned)col_blocks, kColThreads, 0, st>>>(
+          dV.p, dT.p, nt, depth, ch, cols.p, columns, rec.p, block_hits.p);
+      GB_TRY(cudaGetLastError());
+      rc = sum_counts(sc, block_hits.p, col_blocks, &P);
+      if (rc != SVO_OK) return rc;
+      pairs += P;
+      if (P == 0) continue;
+      GB_TRY(keys.alloc(sc, P));
+      column_emit_kernel<<<(unsigned)col_blocks, kColThreads, 0, st>>>(
+          dV.p, dT.p, nt, depth, ch, cols.p, columns, rec.p, block_hits.p, keys.p);
+      GB_TRY(cudaGetLastError());
+    }
+    // stable, by code alone: the triangles of a code are ascending already
+    GB_TRY(keys2.alloc(sc, P));
+    cub::DoubleBuffer<uint64_t> kb(keys.p, keys2.p);
+    const int lo_bit = (int)tri_bits, hi_bit = (int)(ch.shift + tri_bits);
+    size_t bytes = 0;
+    GB_TRY(cub::DeviceRadixSort::SortKeys(nullptr, bytes, kb, P, lo_bit, hi_bit, st));
+    {
+      DevBuf<uint8_t> tmp;
+      GB_TRY(tmp.alloc(sc, bytes));
+      GB_TRY(cub::DeviceRadixSort::SortKeys(tmp.p, bytes, kb, P, lo_bit, hi_bit, st));
+    }
+    if (kb.Current() == keys.p)
+      keys2.reset();
+    else
+      keys = std::move(keys2);
+    KeyLevels kl;
+    kl.keys = keys.p;
+    kl.n = P;
+    kl.tri_bits = tri_bits;
+    kl.depth = depth;
+    kl.first_level = 0;
+    if (!parts.empty()) {  // the chunk's prefix against the last one's
+      uint32_t digit = 0;
+      while ((last_chunk ^ ci) >> (3 * (digit + 1))) ++digit;
+      kl.first_level = chunk_levels - digit;
+    }
+    last_chunk = ci;
+    const uint64_t key_blocks = (P + kKeyBlock - 1) / kKeyBlock;
+    if (key_blocks > 0x7FFFFFFFull) return SVO_ERR_RANGE;
+    DevBuf<uint32_t> counts;
+    GB_TRY(counts.alloc(sc, (depth + 1) * key_blocks));
+    level_count_kernel<<<(unsigned)key_blocks, kKeyThreads, 0, st>>>(kl, key_blocks, counts.p);
+    GB_TRY(cudaGetLastError());
+    level_scan_kernel<<<depth + 1, 1024, 0, st>>>(counts.p, key_blocks, d_totals.p);
+    GB_TRY(cudaGetLastError());
+    uint64_t now[kMaxLevels];
+    GB_TRY(cudaMemcpyAsync(now, d_totals.p, sizeof(now), cudaMemcpyDeviceToHost, st));
+    GB_TRY(cudaStreamSynchronize(st));
+    if (now[depth] > 0xFFFFFFFFull) return SVO_ERR_RANGE;
+    parts.emplace_back();
+    Levels& lv = parts.back();
+    LevelOut out = {};
+    for (uint32_t d = 0; d <= depth; ++d) {
+      lv.size[d] = now[d] - totals[d];
+      out.base[d] = (uint32_t)totals[d];
+      totals[d] = now[d];
+      GB_TRY(lv.octant[d].alloc(sc, lv.size[d]));
+      out.octant[d] = lv.octant[d].p;
+      if (d == depth) continue;
+      GB_TRY(lv.first[d].alloc(sc, lv.size[d]));
+      out.first[d] = lv.first[d].p;
+    }
+    GB_TRY(lv.leaf_attribs.alloc(sc, lv.size[depth]));
+    out.leaf_attribs = lv.leaf_attribs.p;
+    leaf_in.chunk_base = (uint64_t)ci << ch.shift;
+    level_write_kernel<<<(unsigned)key_blocks, kKeyThreads, 0, st>>>(kl, leaf_in, key_blocks, counts.p,
+                                                                    out);
+    GB_TRY(cudaGetLastError());
+  }
+  cols.reset();
+  dV.reset();
+  dT.reset();
+  dFn.reset();
+  dRec.reset();
+  if (parts.empty()) return SVO_ERR_INVALID;
+  leaf_voxels = totals[depth];
+  if (totals[0] != 1) return SVO_ERR_INVALID;
+
+  // -- the chunks' levels one after another
+  if (parts.size() > 1) {
+    Levels all;
+    auto join = [&](auto get, uint32_t d, auto& to) -> int {
+      GB_TRY(to.alloc(sc, totals[d]));
+      uint64_t at = 0;
+      for (Levels& lv : parts) {
+        auto& from = get(lv);
+        GB_TRY(cudaMemcpyAsync(to.p + at, from.p, lv.size[d] * sizeof(*to.p), cudaMemcpyDeviceToDevice, st));
+        at += lv.size[d];
+        from.reset();
+      }
+      return SVO_OK;
+    };
+    for (uint32_t d = 0; d <= depth && rc == SVO_OK; ++d) {
+      rc = join([d](Levels& lv) -> auto& { return lv.octant[d]; }, d, all.octant[d]);
+      if (rc == SVO_OK && d < depth)
+        rc = join([d](Levels& lv) -> auto& { return lv.first[d]; }, d, all.first[d]);
+    }
+    if (rc == SVO_OK) rc = join([](Levels& lv) -> auto& { return lv.leaf_attribs; }, depth, all.leaf_attribs);
+    if (rc != SVO_OK) return rc;
+    parts.clear();
+    parts.push_back(std::move(all));
+  }
+  Levels& lv = parts[0];
+
+  // -- attributes and masks, bottom-up
+  DevBuf<uint8_t> masks[kMaxLevels];
+  DevBuf<svo_attrib> attribs[kMaxLevels];
+  attribs[depth] = std::move(lv.leaf_attribs);
+  octree_nodes = totals[depth];
+  for (int d = (int)depth - 1; d >= 0; --d) {
+    const uint32_t n = (uint32_t)totals[d];
+    octree_nodes += n;
+    GB_TRY(masks[d].alloc(sc, n));
+    GB_TRY(attribs[d].alloc(sc, n));
+    parent_kernel<<<grid_of(n, kParentThreads), kParentThreads, 0, st>>>(
+        lv.first[d].p, n, (uint32_t)totals[d + 1], lv.octant[d + 1].p, attribs[d + 1].p, masks[d].p,
+        attribs[d].p);
+    GB_TRY(cudaGetLastError());
+    lv.octant[d + 1].reset();
+  }
 
   // -- partitions (treelet boundary levels) and gids
   CutParams cp{};
@@ -900,23 +1359,23 @@ int DeviceScene::build_mesh(const float* h_vertices, const float* h_normals,
     P.root_level = r;
     P.stop_level = stop_level_of(depth, treelet_levels, r);
     P.gid_base = (uint32_t)gid_next;
-    P.count = (uint32_t)levels[r].size;
-    gid_next += levels[r].size;
+    P.count = (uint32_t)totals[r];
+    gid_next += totals[r];
     if (gid_next > 0x7FFFFFFFull) return SVO_ERR_RANGE;
   }
   cp.num_parts = np;
   num_treelets = (uint32_t)gid_next;
   LevelPtrs L{};
   for (uint32_t d = 0; d <= depth; ++d) {
-    L.masks[d] = levels[d].masks.p;
-    L.first[d] = levels[d].first.p;
-    L.attribs[d] = levels[d].attribs.p;
+    L.masks[d] = masks[d].p;
+    L.first[d] = lv.first[d].p;
+    L.attribs[d] = attribs[d].p;
   }
 
   // -- slot size: the largest treelet + 8 (cut_treelets' automatic size)
   {
     DevBuf<unsigned long long> stats;  // {largest treelet, sum of treelet sizes}
-    GB_TRY(stats.alloc(2));
+    GB_TRY(stats.alloc(sc, 2));
     GB_TRY(cudaMemsetAsync(stats.p, 0, 16, st));
     treelet_sizes_kernel<<<grid_of(num_treelets, 128), 128, 0, st>>>(L, cp, num_treelets, stats.p);
     GB_TRY(cudaGetLastError());
@@ -931,11 +1390,12 @@ int DeviceScene::build_mesh(const float* h_vertices, const float* h_normals,
   cp.N = nodes_per_slot;
   pool_nodes = (uint64_t)num_treelets * nodes_per_slot;
 
-  // -- the pool
-  GB_TRY(cudaMalloc(&d_nodes, pool_nodes * sizeof(svo_node)));
-  GB_TRY(cudaMalloc(&d_attribs, pool_nodes * sizeof(svo_attrib)));
-  GB_TRY(cudaMemsetAsync(d_nodes, 0, pool_nodes * sizeof(svo_node), st));
-  GB_TRY(cudaMemsetAsync(d_attribs, 0, pool_nodes * sizeof(svo_attrib), st));
+  // -- the pool: nodes, then attributes, in one allocation
+  const uint64_t half = (pool_nodes * sizeof(svo_node) + 255u) & ~255ull;
+  void* mem = nullptr;
+  GB_TRY(pool_alloc(dev, 2 * half, &mem, &pool_bytes_));
+  d_nodes = (svo_node*)mem;
+  d_attribs = (svo_attrib*)((char*)mem + half);
   cut_kernel<<<num_treelets, 256, 0, st>>>(L, cp, num_treelets, reinterpret_cast<uint2*>(d_nodes),
                                            d_attribs);
   GB_TRY(cudaGetLastError());
@@ -944,8 +1404,13 @@ int DeviceScene::build_mesh(const float* h_vertices, const float* h_normals,
 }
 
 DeviceScene::~DeviceScene() {
-  if (d_nodes) cudaFree(d_nodes);
-  if (d_attribs) cudaFree(d_attribs);
+  if (device < 0) return;
+  int now = device;
+  const bool other = cudaGetDevice(&now) == cudaSuccess && now != device;
+  if (other) cudaSetDevice(device);
+  pool_free(device, d_nodes, pool_bytes_);
+  user_ends(device);
+  if (other) cudaSetDevice(now);
 }
 
 }  // namespace svo

@@ -21,7 +21,8 @@ struct DeviceScene {
   uint64_t leaf_voxels = 0;
   uint64_t pairs = 0;           // voxel/triangle overlaps found by the voxeliser
   svo_node* d_nodes = nullptr;
-  svo_attrib* d_attribs = nullptr;
+  svo_attrib* d_attribs = nullptr;  // in the nodes' allocation, behind them
+  int device = -1;                  // set once the build has begun
 
   DeviceScene() = default;
   DeviceScene(const DeviceScene&) = delete;
@@ -33,6 +34,9 @@ struct DeviceScene {
   int build_mesh(const float* h_vertices, const float* h_normals, const float* h_colors,
                  uint64_t num_vertices, const uint32_t* h_triangles, uint64_t num_triangles,
                  uint32_t depth, uint32_t treelet_levels, cudaStream_t stream);
+
+ private:
+  uint64_t pool_bytes_ = 0;
 };
 
 }  // namespace svo
