@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include "feedback.h"
+#include "render.h"
 #include "shade.cuh"
 #include "traverse.cuh"
 
@@ -19,22 +20,20 @@ namespace svo {
 
 namespace {
 
-// One warp (8x4 pixels) per block: analysis buffers are small (128x128 for
-// a 1024x1024 frame at the reference's divisor 8), and one-warp blocks
-// spread their few rays over all SMs.
+// One warp per block, 8x4 pixels or fewer (rays_per_warp): analysis buffers are
+// small (128x128 for a 1024x1024 frame at the reference's divisor 8), and
+// one-warp blocks spread their few rays over all SMs.
 constexpr int kBlockW = 8;
-constexpr int kBlockH = 4;
-constexpr int kThreads = kBlockW * kBlockH;
+constexpr int kThreads = 32;
 
 __global__ void __launch_bounds__(kThreads) feedback_kernel(
     const uint2* __restrict__ nodes, uint64_t num_nodes, const svo_frame_params p, int S,
-    svo_feedback* __restrict__ out, uint32_t* __restrict__ rgba, uint32_t y0) {
+    svo_feedback* __restrict__ out, uint32_t* __restrict__ rgba, uint32_t y0, uint32_t rays) {
   extern __shared__ uint2 stack_smem[];
   const int t = threadIdx.x;
-  const int warp = t >> 5, lane = t & 31;
-  const uint32_t x = blockIdx.x * kBlockW + (warp % (kBlockW / 8)) * 8 + (lane & 7);
-  const uint32_t y = y0 + blockIdx.y * kBlockH + (warp / (kBlockW / 8)) * 4 + (lane >> 3);
-  if (x >= p.width || y >= p.height) return;
+  const uint32_t x = blockIdx.x * kBlockW + (t & 7);
+  const uint32_t y = y0 + blockIdx.y * (rays / kBlockW) + (t >> 3);
+  if (t >= (int)rays || x >= p.width || y >= p.height) return;
   float o[3], dx, dy, dz;
   pixel_ray(p, x, y, o, dx, dy, dz);
   const RayHit h = cast_ray<false>(GlobalFetch{nodes}, num_nodes, o, dx, dy, dz, p.t_scale_ratio,
@@ -67,12 +66,13 @@ int launch_feedback(const svo_node* nodes, uint64_t num_nodes, const svo_frame_p
   if (p.width == 0 || p.height == 0) return SVO_OK;
   if (p.height > 0xFFFFFFF0u) return SVO_ERR_RANGE;  // row indices stay below 2^32
   const size_t smem = (size_t)S * kThreads * sizeof(uint2);
-  constexpr uint32_t kRowsPerLaunch = 65535u * kBlockH;  // grid rows are at most 65535
-  for (uint32_t y0 = 0; y0 < p.height; y0 += kRowsPerLaunch) {
-    const uint32_t rows = p.height - y0 < kRowsPerLaunch ? p.height - y0 : kRowsPerLaunch;
-    const dim3 grid((p.width + kBlockW - 1) / kBlockW, (rows + kBlockH - 1) / kBlockH);
+  const uint32_t rays = rays_per_warp((uint64_t)p.width * p.height), block_h = rays / kBlockW;
+  const uint32_t per_launch = 65535u * block_h;  // grid rows are at most 65535
+  for (uint32_t y0 = 0; y0 < p.height; y0 += per_launch) {
+    const uint32_t rows = p.height - y0 < per_launch ? p.height - y0 : per_launch;
+    const dim3 grid((p.width + kBlockW - 1) / kBlockW, (rows + block_h - 1) / block_h);
     feedback_kernel<<<grid, kThreads, smem, stream>>>(reinterpret_cast<const uint2*>(nodes),
-                                                       num_nodes, p, S, out, rgba, y0);
+                                                       num_nodes, p, S, out, rgba, y0, rays);
     if (cudaGetLastError() != cudaSuccess) return SVO_ERR_CUDA;
   }
   return SVO_OK;

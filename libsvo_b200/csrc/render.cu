@@ -9,6 +9,7 @@
 // The RGBA8 epilogue is fused.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "render.h"
@@ -110,6 +111,18 @@ __device__ __forceinline__ uint32_t ordered_block(const BlockOrder& o, uint32_t 
   return __ldg(o.list + (uint64_t)bucket * o.nblocks + (r - before));
 }
 
+// The thread's pixel; false outside the frame.  Warp w of a block covers 8
+// columns and rays / 8 rows of it, two warps side by side (16x8 pixels at 32
+// rays a warp); rows start at y0 (frames taller than one grid's rows take
+// several launches).
+__device__ __forceinline__ bool block_pixel(const svo_frame_params& p, uint32_t bx, uint32_t by,
+                                            uint32_t y0, uint32_t rays, uint32_t* x, uint32_t* y) {
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, rows = rays / 8;
+  *x = bx * kBlockW + (warp % (kBlockW / 8)) * 8 + (lane & 7);
+  *y = y0 + by * (kBlockH / 4 * rows) + (warp / (kBlockW / 8)) * rows + (lane >> 3);
+  return lane < rays && *x < p.width && *y < p.height;
+}
+
 // kExt: view modes 2, 6 and 7 (shade_ext); the other modes compile without
 // the extra exit state.  With `order` (1-D grid) block r casts the r-th block
 // in estimated-cost order of a frame gx blocks wide; without it the grid is
@@ -118,7 +131,7 @@ template <bool kFlat, bool kExt>
 __global__ void __launch_bounds__(kThreads) render_frame_kernel(
     const uint2* __restrict__ nodes, const uint2* __restrict__ attribs, uint64_t num_nodes,
     const svo_frame_params p, int S, uint32_t* __restrict__ rgba, svo_hit* __restrict__ hits,
-    svo_stats* __restrict__ stats, uint32_t y0, const BlockOrder order, uint32_t gx) {
+    svo_stats* __restrict__ stats, uint32_t y0, const BlockOrder order, uint32_t gx, uint32_t rays) {
   extern __shared__ uint2 stack_smem[];
   const int t = threadIdx.x;
   const int warp = t >> 5, lane = t & 31;
@@ -136,11 +149,8 @@ __global__ void __launch_bounds__(kThreads) render_frame_kernel(
     bx = block % gx;
     by = block / gx;
   }
-  // warp w covers pixels [8*(w&1), +8) x [4*(w>>1), +4) of the 16x8 block;
-  // rows start at y0 (frames taller than one grid's rows take several launches)
-  const uint32_t x = bx * kBlockW + (warp % (kBlockW / 8)) * 8 + (lane & 7);
-  const uint32_t y = y0 + by * kBlockH + (warp / (kBlockW / 8)) * 4 + (lane >> 3);
-  if (x >= p.width || y >= p.height) return;
+  uint32_t x, y;
+  if (!block_pixel(p, bx, by, y0, rays, &x, &y)) return;
   float o[3], dx, dy, dz;
   pixel_ray(p, x, y, o, dx, dy, dz);
   const RayHit h = cast_ray<kFlat>(GlobalFetch{nodes}, num_nodes, o, dx, dy, dz, p.t_scale_ratio,
@@ -216,13 +226,11 @@ __global__ void __launch_bounds__(kThreads) render_shadow_kernel(
     const uint2* __restrict__ nodes, const uint2* __restrict__ attribs, uint64_t num_nodes,
     const svo_frame_params p, const svo_shadow_cfg sc, int S, uint32_t* __restrict__ rgba,
     svo_hit* __restrict__ hits, svo_hit* __restrict__ shadow_hits,
-    svo_stats* __restrict__ stats, uint32_t y0) {
+    svo_stats* __restrict__ stats, uint32_t y0, uint32_t rays) {
   extern __shared__ uint2 stack_smem[];
   const int t = threadIdx.x;
-  const int warp = t >> 5, lane = t & 31;
-  const uint32_t x = blockIdx.x * kBlockW + (warp % (kBlockW / 8)) * 8 + (lane & 7);
-  const uint32_t y = y0 + blockIdx.y * kBlockH + (warp / (kBlockW / 8)) * 4 + (lane >> 3);
-  if (x >= p.width || y >= p.height) return;
+  uint32_t x, y;
+  if (!block_pixel(p, blockIdx.x, blockIdx.y, y0, rays, &x, &y)) return;
   float o[3], dx, dy, dz;
   pixel_ray(p, x, y, o, dx, dy, dz);
   const RayHit h = cast_ray<false>(GlobalFetch{nodes}, num_nodes, o, dx, dy, dz, p.t_scale_ratio,
@@ -280,8 +288,8 @@ __global__ void __launch_bounds__(kThreads) trace_rays_kernel(
 
 size_t render_smem_bytes(int S) { return (size_t)S * kThreads * sizeof(uint2); }
 
-// Rows of one launch: a grid has at most 65535 blocks along y.
-constexpr uint32_t kRowsPerLaunch = 65535u * kBlockH;
+// Blocks along y of one launch.
+constexpr uint32_t kGridRows = 65535u;
 
 namespace {
 
@@ -387,17 +395,18 @@ int launch_render(const svo_node* nodes, const svo_attrib* attribs, uint64_t num
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = attr;
     lc.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&lc, fn, n2, a2, num_nodes, p, S, rgba, hits, stats, 0u, order, gx);
+    cudaError_t e = cudaLaunchKernelEx(&lc, fn, n2, a2, num_nodes, p, S, rgba, hits, stats, 0u, order, gx, 32u);
     const cudaError_t last = cudaGetLastError();  // clears a launch error
     if (e == cudaSuccess) e = last;
     cudaFreeAsync(const_cast<uint32_t*>(order.count), stream);
     return e == cudaSuccess ? SVO_OK : SVO_ERR_CUDA;
   }
-  for (uint32_t y0 = 0; y0 < p.height; y0 += kRowsPerLaunch) {
-    const uint32_t rows = p.height - y0 < kRowsPerLaunch ? p.height - y0 : kRowsPerLaunch;
-    const dim3 grid(gx, (rows + kBlockH - 1) / kBlockH);
+  const uint32_t rays = rays_per_warp((uint64_t)p.width * p.height), block_h = kBlockH / 4 * rays / 8;
+  for (uint32_t y0 = 0; y0 < p.height; y0 += kGridRows * block_h) {
+    const uint32_t rows = std::min(p.height - y0, kGridRows * block_h);
+    const dim3 grid(gx, (rows + block_h - 1) / block_h);
     fn<<<grid, kThreads, smem, stream>>>(n2, a2, num_nodes, p, S, rgba, hits, stats, y0,
-                                         BlockOrder{nullptr, nullptr, 0u}, gx);
+                                         BlockOrder{nullptr, nullptr, 0u}, gx, rays);
     if (cudaGetLastError() != cudaSuccess) return SVO_ERR_CUDA;
   }
   return SVO_OK;
@@ -421,11 +430,12 @@ int launch_render_shadow(const svo_node* nodes, const svo_attrib* attribs, uint6
   // shadow ray cast right after its primary ray finds the nodes of its
   // descent in L1; cast in a later pass it reads them from L2 again.
   const uint32_t gx = (p.width + kBlockW - 1) / kBlockW;
-  for (uint32_t y0 = 0; y0 < p.height; y0 += kRowsPerLaunch) {
-    const uint32_t rows = p.height - y0 < kRowsPerLaunch ? p.height - y0 : kRowsPerLaunch;
-    const dim3 grid(gx, (rows + kBlockH - 1) / kBlockH);
+  const uint32_t rays = rays_per_warp((uint64_t)p.width * p.height), block_h = kBlockH / 4 * rays / 8;
+  for (uint32_t y0 = 0; y0 < p.height; y0 += kGridRows * block_h) {
+    const uint32_t rows = std::min(p.height - y0, kGridRows * block_h);
+    const dim3 grid(gx, (rows + block_h - 1) / block_h);
     render_shadow_kernel<<<grid, kThreads, render_smem_bytes(S), stream>>>(
-        n2, a2, num_nodes, p, sc, S, rgba, hits, shadow_hits, stats, y0);
+        n2, a2, num_nodes, p, sc, S, rgba, hits, shadow_hits, stats, y0, rays);
     if (cudaGetLastError() != cudaSuccess) return SVO_ERR_CUDA;
   }
   return SVO_OK;
