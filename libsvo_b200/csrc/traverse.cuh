@@ -53,6 +53,26 @@ struct RayHit {
   float t_enter, t_exit;  // the root box (both 0 when the ray misses it)
 };
 
+__device__ __forceinline__ RayHit no_hit() {
+  RayHit h;
+  h.node = 0u;
+  h.t = 0.0f;
+  h.depth = 0u;
+  h.hit = 0u;
+  h.flags = 0u;
+  h.loops = 0u;
+  h.fetches = 0u;
+  h.tc_min = 0.0f;
+  h.sx2 = 0.0f;
+  h.leaf = 0u;
+  h.cx = 0.0f;
+  h.cy = 0.0f;
+  h.cz = 0.0f;
+  h.t_enter = 0.0f;
+  h.t_exit = 0.0f;
+  return h;
+}
+
 __device__ __forceinline__ float cl_max(float a, float b) { return (a < b) ? b : a; }
 __device__ __forceinline__ float cl_min(float a, float b) { return (b < a) ? b : a; }
 
@@ -485,11 +505,46 @@ __device__ __forceinline__ void descend_general(const Fetch& fetch, uint64_t num
 // only for a valid child, the one case that reads tcMin.  There is no NaN and
 // no -0 among the distances (see cast_ray), so the hardware min/max give the
 // reference's order bit for bit.
+//
+// With kYield the ray goes on from `w` and the loop also ends (kYields, with the
+// ray in `w` again) once no more than `keep` lanes of the warp are still in it.
 constexpr uint32_t kProgressPasses = 32;
-template <bool kFlat, class Fetch>
-__device__ __forceinline__ bool descend(const Fetch& fetch, uint64_t num_nodes, const Ray& r,
-                                        int S, uint2* stack, int stride, uint32_t limit,
-                                        RayState& st, RayHit& h) {
+enum Outcome { kEnded, kLeaves, kYields };
+
+// A ray between two passes of the loop.
+struct Descent {
+  uint32_t node;
+  float tmin, tmax, cx, cy, cz, sx2;
+  uint2 nd;
+  uint32_t passes, pops, check_at;
+  float seen;
+  uint32_t open;
+  uint2* sp;
+};
+
+template <class Fetch>
+__device__ __forceinline__ Descent descent_start(const Fetch& fetch, uint64_t num_nodes,
+                                                 const Ray& r, float t_min, uint32_t limit,
+                                                 uint2* stack) {
+  Descent w;
+  w.node = 0u;
+  w.tmin = t_min;
+  w.tmax = r.t_max;
+  w.cx = w.cy = w.cz = 0.0f;
+  w.sx2 = 0.5f;
+  w.nd = num_nodes ? fetch(0u) : make_uint2(0u, 0xFFFFu);
+  w.passes = w.pops = 0u;
+  w.check_at = kProgressPasses < limit ? kProgressPasses : limit;
+  w.seen = t_min;
+  w.open = 0x3f800000u;
+  w.sp = stack;
+  return w;
+}
+
+template <bool kFlat, bool kYield, class Fetch>
+__device__ __forceinline__ Outcome descend(const Fetch& fetch, uint64_t num_nodes, const Ray& r,
+                                           int S, uint2* stack, int stride, uint32_t limit,
+                                           int keep, Descent& w, RayState& st, RayHit& h) {
   const float eps = 0.00001f;
   const float sx2_last = last_size<kFlat>(S);
   // Pools hold at most 2^32 nodes, so the in-pool test of a 32-bit index is one
@@ -497,19 +552,20 @@ __device__ __forceinline__ bool descend(const Fetch& fetch, uint64_t num_nodes, 
   // leaves only: its test then ends the ray, where the index is looked at again.
   const uint32_t last_node = num_nodes ? (uint32_t)(num_nodes - 1u) : 0u;
   constexpr uint32_t kOne = 0x3f800000u;
-  uint32_t node = 0u;
-  float tmin = st.tmin, tmax = r.t_max;
-  float cx = 0.0f, cy = 0.0f, cz = 0.0f;
-  float sx2 = 0.5f;
-  uint2 nd = num_nodes ? fetch(0u) : make_uint2(0u, 0xFFFFu);
-  uint32_t passes = 0u, pops = 0u;  // tests (the reference's fetches) and popped levels
-  uint32_t check_at = kProgressPasses < limit ? kProgressPasses : limit;
-  float seen = tmin;  // tMin when it was last looked at
-  uint32_t open = kOne;
-  uint2* sp = stack;  // the next free stack word
-  if (interval_done<kFlat>(tmin, tmax)) {
+  if (!kYield) w = descent_start(fetch, num_nodes, r, st.tmin, limit, stack);
+  uint32_t node = w.node;
+  float tmin = w.tmin, tmax = w.tmax;
+  float cx = w.cx, cy = w.cy, cz = w.cz;
+  float sx2 = w.sx2;
+  uint2 nd = w.nd;
+  uint32_t passes = w.passes, pops = w.pops;  // tests (the reference's fetches), popped levels
+  uint32_t check_at = w.check_at;
+  float seen = w.seen;  // tMin when it was last looked at
+  uint32_t open = w.open;
+  uint2* sp = w.sp;  // the next free stack word
+  if (passes == 0u && interval_done<kFlat>(tmin, tmax)) {
     ray_missed(kFlat, r, 1u, 0u, h);
-    return true;
+    return kEnded;
   }
   for (;;) {
     if (passes == check_at) {
@@ -517,6 +573,12 @@ __device__ __forceinline__ bool descend(const Fetch& fetch, uint64_t num_nodes, 
       seen = tmin;
       check_at = check_at + kProgressPasses < limit ? check_at + kProgressPasses : limit;
     }
+#if defined(__CUDACC__)
+    if (kYield && __popc(__activemask()) <= keep) {
+      w = Descent{node, tmin, tmax, cx, cy, cz, sx2, nd, passes, pops, check_at, seen, open, sp};
+      return kYields;
+    }
+#endif
     ++passes;
     // childEntryPoint = (o + (tMin + eps) d) - centre and its sign test
     const float te = __fadd_rn(tmin, eps);
@@ -547,11 +609,11 @@ __device__ __forceinline__ bool descend(const Fetch& fetch, uint64_t num_nodes, 
         if (node > last_node || num_nodes == 0u) {  // the frame's node is outside the pool
           h.flags = SVO_HITFLAG_BOUNDS;
           h.fetches = passes - 1u;
-          return true;
+          return kEnded;
         }
         if (kFlat && !leaf && !lod) {  // non-leaf below the octree's depth: corrupt pool
           h.flags = SVO_HITFLAG_BOUNDS;
-          return true;
+          return kEnded;
         }
         h.hit = 1u;
         h.node = child;
@@ -563,7 +625,7 @@ __device__ __forceinline__ bool descend(const Fetch& fetch, uint64_t num_nodes, 
         h.cx = __fadd_rn(with_side(bx, half), cx);
         h.cy = __fadd_rn(with_side(by, half), cy);
         h.cz = __fadd_rn(with_side(bz, half), cz);
-        return true;
+        return kEnded;
       }
       // push: the current frame's tMin becomes tc_max (recovered on pop)
       if (tc_max != tmax) {
@@ -588,7 +650,7 @@ __device__ __forceinline__ bool descend(const Fetch& fetch, uint64_t num_nodes, 
       do {
         if (open == kOne) {  // above the root: the ray leaves the octree
           ray_missed(kFlat, r, passes + pops + level_of(sx2), passes, h);
-          return true;
+          return kEnded;
         }
         sp -= stride;
         const uint2 e = *sp;
@@ -611,41 +673,22 @@ __device__ __forceinline__ bool descend(const Fetch& fetch, uint64_t num_nodes, 
     }
   }
   st = RayState{node, tmin, tmax, cx, cy, cz, sx2, passes + pops, passes};
-  return false;
+  return kLeaves;
 }
 
-// One ray: root box test, direction clamp, then the descent.  pass_cap > 0
-// stops the ray after that many child tests instead of the watchdog's
-// (S+1)^2*5 iterations (used only to estimate costs; results under a cap are
-// not the reference's: h.tc_min is how far the ray has come).
-template <bool kFlat, class Fetch>
-__device__ __forceinline__ RayHit cast_ray(const Fetch& fetch, uint64_t num_nodes,
-                                           const float o[3], float dx, float dy, float dz,
-                                           float tsr, int S, uint2* stack, int stride,
-                                           uint32_t pass_cap = 0u) {
-  RayHit h;
-  h.node = 0u;
-  h.t = 0.0f;
-  h.depth = 0u;
-  h.hit = 0u;
-  h.flags = 0u;
-  h.loops = 0u;
-  h.fetches = 0u;
-  h.tc_min = 0.0f;
-  h.sx2 = 0.0f;
-  h.leaf = 0u;
-  h.cx = 0.0f;
-  h.cy = 0.0f;
-  h.cz = 0.0f;
-  h.t_enter = 0.0f;
-  h.t_exit = 0.0f;
-
-  float t_min, t_max;
+// The ray set up against the root box: kMissesBox, kFast where `descend` can
+// take it, else kGeneral.
+enum RayKind { kMissesBox, kFast, kGeneral };
+template <bool kFlat>
+__device__ __forceinline__ RayKind setup_ray(const float o[3], float dx, float dy, float dz,
+                                             float tsr, Ray& r, float& t_min, RayHit& h) {
+  h = no_hit();
+  float t_max;
   {
     const float d0[3] = {dx, dy, dz};
     if (!root_slab(o, d0, t_min, t_max)) {
       h.flags = SVO_HITFLAG_BOXMISS;
-      return h;
+      return kMissesBox;
     }
   }
   h.t_enter = t_min;
@@ -663,7 +706,6 @@ __device__ __forceinline__ RayHit cast_ray(const Fetch& fetch, uint64_t num_node
     if (fabsf(dy) < mn) dy = __fmul_rn(mn, cl_sign(dy));
     if (fabsf(dz) < mn) dz = __fmul_rn(mn, cl_sign(dz));
   }
-  Ray r;
   r.ox = o[0];
   r.oy = o[1];
   r.oz = o[2];
@@ -686,20 +728,42 @@ __device__ __forceinline__ RayHit cast_ray(const Fetch& fetch, uint64_t num_node
   const bool neg_zero = __float_as_uint(o[0]) == 0x80000000u ||
                         __float_as_uint(o[1]) == 0x80000000u ||
                         __float_as_uint(o[2]) == 0x80000000u;
-  RayState st = {0u, t_min, t_max, 0.0f, 0.0f, 0.0f, 0.5f, 0u, 0u};
-  if (isfinite(r.px) && isfinite(r.py) && isfinite(r.pz) && !neg_zero) {
-    // n passes are n tests, at most as many pushes, and so at most n plus the
-    // root's pops: below this many passes no ray comes to the watchdog
-    const uint32_t limit = ((uint32_t)((S + 1) * (S + 1) * 5) - 2u) / 2u;
+  return isfinite(r.px) && isfinite(r.py) && isfinite(r.pz) && !neg_zero ? kFast : kGeneral;
+}
+
+// Passes of the fast loop: n passes are n tests, at most as many pushes, and so
+// at most n pops plus the root's, so below this many no ray comes to the watchdog.
+__device__ __forceinline__ uint32_t pass_limit(int S) {
+  return ((uint32_t)((S + 1) * (S + 1) * 5) - 2u) / 2u;
+}
+
+// One ray: root box test, direction clamp, then the descent.  pass_cap > 0
+// stops the ray after that many child tests instead of the watchdog's
+// (S+1)^2*5 iterations (used only to estimate costs; results under a cap are
+// not the reference's: h.tc_min is how far the ray has come).
+template <bool kFlat, class Fetch>
+__device__ __forceinline__ RayHit cast_ray(const Fetch& fetch, uint64_t num_nodes,
+                                           const float o[3], float dx, float dy, float dz,
+                                           float tsr, int S, uint2* stack, int stride,
+                                           uint32_t pass_cap = 0u) {
+  RayHit h;
+  Ray r;
+  float t_min = 0.0f;
+  const RayKind kind = setup_ray<kFlat>(o, dx, dy, dz, tsr, r, t_min, h);
+  if (kind == kMissesBox) return h;
+  RayState st = {0u, t_min, r.t_max, 0.0f, 0.0f, 0.0f, 0.5f, 0u, 0u};
+  Descent w;
+  if (kind == kFast) {
     if (pass_cap) {
-      if (!descend<kFlat>(fetch, num_nodes, r, S, stack, stride, pass_cap, st, h)) {
+      if (descend<kFlat, false>(fetch, num_nodes, r, S, stack, stride, pass_cap, 0, w, st, h) != kEnded) {
         h.flags = SVO_HITFLAG_CAPPED;
         h.loops = st.loops;
         h.tc_min = st.tmin;
       }
       return h;
     }
-    if (descend<kFlat>(fetch, num_nodes, r, S, stack, stride, limit, st, h)) return h;
+    if (descend<kFlat, false>(fetch, num_nodes, r, S, stack, stride, pass_limit(S), 0, w, st, h) == kEnded)
+      return h;
   }
   descend_general<kFlat>(fetch, num_nodes, r, S, stack, stride, st, h, pass_cap);
   return h;
