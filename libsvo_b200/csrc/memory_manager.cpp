@@ -33,6 +33,7 @@ int TreeletMemoryManager::init(svo_scene&& scene, uint64_t incore_bytes) {
   incore_ = (svo_node*)std::calloc(slots * N_, sizeof(svo_node));
   incore_attr_ = (svo_attrib*)std::calloc(slots * N_, sizeof(svo_attrib));
   if (!incore_ || !incore_attr_) return SVO_ERR_NOMEM;
+  used_.assign(slots, 0u);
   return reset_incore_buffer();
 }
 
@@ -40,6 +41,8 @@ int TreeletMemoryManager::reset_incore_buffer() {
   before_host_write();
   free_.clear();
   upload_.clear();
+  patches_.clear();
+  body_dirty_.assign(slots_.size(), 0);
   children_.assign(scene_.treelets.size(), std::set<int32_t>());
   slot_of_.assign(scene_.treelets.size(), -1);
   for (auto& s : slots_) s = SlotInfo();
@@ -92,7 +95,7 @@ int TreeletMemoryManager::insert_treelet(const SlotInfo& tve) {
   w.bit = 1u << (uint32_t)t.parent_leaf_idx;
   w.set = false;
   write_leaf(pslot, w);
-  mark_upload(pslot);
+  mark_patch(pslot, w.leaf, w.leaf_parent);
   children_[t.parent_gid].insert(gid);
   return SVO_OK;
 }
@@ -116,7 +119,7 @@ int TreeletMemoryManager::remove_treelet(int32_t gid) {
   w.bit = 1u << (uint32_t)t.parent_leaf_idx;
   w.set = true;
   write_leaf((uint32_t)pslot, w);
-  mark_upload((uint32_t)pslot);
+  mark_patch((uint32_t)pslot, w.leaf, w.leaf_parent);
   slots_[slot] = SlotInfo();
   free_.push_back(slot);
   slot_of_[gid] = -1;
@@ -128,9 +131,13 @@ void TreeletMemoryManager::copy_body(uint32_t slot, int32_t gid) {
   const TreeletData& t = scene_.treelets[gid];
   const uint64_t pos = (uint64_t)slot * N_;
   std::memcpy(incore_ + pos, t.nodes.data(), (size_t)t.num_nodes * sizeof(svo_node));
-  std::memset(incore_ + pos + t.num_nodes, 0, (size_t)(N_ - t.num_nodes) * sizeof(svo_node));
   std::memcpy(incore_attr_ + pos, t.attribs.data(), (size_t)t.num_nodes * sizeof(svo_attrib));
-  std::memset(incore_attr_ + pos + t.num_nodes, 0, (size_t)(N_ - t.num_nodes) * sizeof(svo_attrib));
+  if (used_[slot] > t.num_nodes) {  // what the slot held before reached further
+    const size_t more = used_[slot] - t.num_nodes;
+    std::memset(incore_ + pos + t.num_nodes, 0, more * sizeof(svo_node));
+    std::memset(incore_attr_ + pos + t.num_nodes, 0, more * sizeof(svo_attrib));
+  }
+  used_[slot] = t.num_nodes;
 }
 
 void TreeletMemoryManager::write_leaf(uint32_t pslot, const LeafWrite& w) {
@@ -138,6 +145,8 @@ void TreeletMemoryManager::write_leaf(uint32_t pslot, const LeafWrite& w) {
     pending_ops_[pslot].push_back(w);
     return;
   }
+  const uint64_t end = std::max(w.leaf, w.leaf_parent) + 1u - (uint64_t)pslot * N_;
+  used_[pslot] = std::max(used_[pslot], (uint32_t)end);
   incore_[w.leaf] = w.value;
   if (w.set)
     incore_[w.leaf_parent].masks |= w.bit;
@@ -167,12 +176,16 @@ void TreeletMemoryManager::end_deferred() {
     if (pending_gid_[s] >= 0) todo.push_back(s);  // a slot placed twice is listed twice
   std::sort(todo.begin(), todo.end());
   todo.erase(std::unique(todo.begin(), todo.end()), todo.end());
-  // bodies first, on up to 8 threads for more than 16 slots ...
+  // bodies first, on up to 8 threads, one for each 2 MB (a thread costs about
+  // as much as copying a quarter of that) ...
   auto bodies = [&](size_t lo, size_t hi) {
     for (size_t i = lo; i < hi; ++i) copy_body(todo[i], pending_gid_[todo[i]]);
   };
   static const size_t hw = std::max(1u, std::thread::hardware_concurrency());
-  const size_t parts = todo.size() > 16 ? std::min<size_t>(std::min<size_t>(8, hw), todo.size() / 8) : 1;
+  size_t bytes = 0;
+  for (uint32_t s : todo)
+    bytes += (size_t)scene_.treelets[pending_gid_[s]].num_nodes * (sizeof(svo_node) + sizeof(svo_attrib));
+  const size_t parts = std::max<size_t>(1, std::min({(size_t)8, hw, todo.size(), bytes >> 21}));
   std::vector<std::thread> workers;
   size_t started = 1;  // part 0 runs on this thread
   try {
@@ -180,7 +193,7 @@ void TreeletMemoryManager::end_deferred() {
       workers.emplace_back(bodies, todo.size() * started / parts, todo.size() * (started + 1) / parts);
   } catch (...) {  // no more threads: the rest runs here
   }
-  bodies(0, parts ? todo.size() / parts : todo.size());
+  bodies(0, todo.size() / parts);
   if (started < parts) bodies(todo.size() * started / parts, todo.size());
   for (std::thread& w : workers) w.join();
   // ... then, per slot in order, the writes aimed at it
@@ -344,7 +357,7 @@ TreeletMemoryManagerCuda::~TreeletMemoryManagerCuda() {
     cudaHostUnregister(incore_);
     cudaHostUnregister(incore_attr_);
   }
-  if (h_slot_ids_) cudaFreeHost(h_slot_ids_);
+  if (h_jobs_) cudaFreeHost(h_jobs_);
   if (d2h_stream_) cudaStreamSynchronize(d2h_stream_);
   for (int i = 0; i < 2; ++i) {
     cudaFree(d_img_[i]);
@@ -395,6 +408,7 @@ int TreeletMemoryManagerCuda::init_transfer() {
 int TreeletMemoryManagerCuda::upload_all() {
   const uint64_t n = incore_nodes();
   if (mirror_pinned_) {
+    mirror_read_ = true;
     // page-locked mirror: two DMA copies straight from it, no staging
     SVO_CUDA_TRY(cudaMemcpyAsync(d_nodes_, incore_, n * sizeof(svo_node), cudaMemcpyHostToDevice,
                                  copy_stream_));
@@ -407,7 +421,7 @@ int TreeletMemoryManagerCuda::upload_all() {
   }
   SVO_CUDA_TRY(cudaEventRecord(upload_done_, copy_stream_));
   upload_pending_ = true;
-  upload_.clear();
+  uploads_done();
   return SVO_OK;
 }
 
@@ -531,18 +545,19 @@ int TreeletMemoryManagerCuda::set_upload_policy(int policy) {
     void* dn = nullptr;
     void* da = nullptr;
     void* di = nullptr;
-    if (e == cudaSuccess && !h_slot_ids_)
-      e = cudaHostAlloc(&h_slot_ids_, (size_t)num_slots() * sizeof(uint32_t), cudaHostAllocMapped);
+    if (e == cudaSuccess && !h_jobs_)
+      e = cudaHostAlloc(&h_jobs_, (patches_at() + 4 * kMaxPatches) * sizeof(uint32_t),
+                        cudaHostAllocMapped);
     if (e == cudaSuccess) e = cudaHostGetDevicePointer(&dn, incore_, 0);
     if (e == cudaSuccess) e = cudaHostGetDevicePointer(&da, incore_attr_, 0);
-    if (e == cudaSuccess) e = cudaHostGetDevicePointer(&di, h_slot_ids_, 0);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer(&di, h_jobs_, 0);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return cuda_status(e);
     }
     mapped_nodes_ = (const svo_node*)dn;
     mapped_attribs_ = (const svo_attrib*)da;
-    mapped_slot_ids_ = (const uint32_t*)di;
+    mapped_jobs_ = (const uint32_t*)di;
     mirror_pinned_ = true;
   }
   upload_policy_ = policy;
@@ -550,9 +565,11 @@ int TreeletMemoryManagerCuda::set_upload_policy(int policy) {
 }
 
 // With the mirror page-locked, the gather kernel and whole-pool uploads read
-// it directly: a host-side change waits for the copies still in flight.
+// it directly: the first host-side change after one waits for it.
 void TreeletMemoryManagerCuda::before_host_write() {
-  if (mirror_pinned_ && upload_pending_ && copy_stream_) cudaStreamSynchronize(copy_stream_);
+  if (!mirror_read_ || !copy_stream_) return;
+  cudaStreamSynchronize(copy_stream_);
+  mirror_read_ = false;
 }
 
 // Dirty slots packed back to back into a ring half ({nodes, attributes} per
@@ -610,21 +627,36 @@ int TreeletMemoryManagerCuda::update_device_memory(uint32_t* copy_calls) {
     if (rc != SVO_OK) return rc;
     SVO_CUDA_TRY(cudaEventRecord(upload_done_, copy_stream_));
     upload_pending_ = true;
-    upload_.clear();
+    uploads_done();
     return SVO_OK;
   }
   if (upload_policy_ == SVO_UPLOAD_PINNED) {
-    // the slot-id list is read by the previous gather until it finishes
-    if (upload_pending_) SVO_CUDA_TRY(cudaStreamSynchronize(copy_stream_));
+    before_host_write();  // the previous gather reads the job list until it finishes
+    uint32_t* jobs = h_jobs_;
     uint32_t k = 0;
-    for (uint32_t s : upload_) h_slot_ids_[k++] = s;
-    const int rc = launch_slot_gather(mapped_nodes_, mapped_attribs_, mapped_slot_ids_, k, N_,
-                                      d_nodes_, d_attribs_, copy_stream_);
+    for (uint32_t s : upload_) {
+      if (!body_dirty_[s]) continue;
+      jobs[2 * k] = s;
+      jobs[2 * k + 1] = used_[s];
+      ++k;
+    }
+    uint32_t* patch = h_jobs_ + patches_at();
+    for (size_t i = 0; i < patches_.size(); ++i) {
+      const svo_node& n = incore_[patches_[i]];
+      patch[4 * i] = patches_[i];
+      patch[4 * i + 1] = 0u;
+      patch[4 * i + 2] = n.first_child;
+      patch[4 * i + 3] = n.masks;
+    }
+    mirror_read_ = true;
+    const int rc = launch_slot_gather(mapped_nodes_, mapped_attribs_, mapped_jobs_, k, N_,
+                                      mapped_jobs_ + patches_at(),
+                                      (uint32_t)patches_.size(), d_nodes_, d_attribs_, copy_stream_);
     if (rc != SVO_OK) return rc;
     SVO_CUDA_TRY(cudaEventRecord(upload_done_, copy_stream_));
     upload_pending_ = true;
     if (copy_calls) *copy_calls = 1;
-    upload_.clear();
+    uploads_done();
     return SVO_OK;
   }
   const auto ranges = upload_ranges();
@@ -641,7 +673,7 @@ int TreeletMemoryManagerCuda::update_device_memory(uint32_t* copy_calls) {
   SVO_CUDA_TRY(cudaEventRecord(upload_done_, copy_stream_));
   upload_pending_ = true;
   if (copy_calls) *copy_calls = (uint32_t)ranges.size();
-  upload_.clear();
+  uploads_done();
   return SVO_OK;
 }
 

@@ -127,7 +127,30 @@ class TreeletMemoryManager {
   // Called before the host mirror changes, so uploads still reading it
   // (none with the staging ring) can finish first.
   virtual void before_host_write() {}
-  void mark_upload(uint32_t slot) { upload_.insert(slot); }
+  // A slot whose records changed as a whole ...
+  void mark_upload(uint32_t slot) {
+    upload_.insert(slot);
+    body_dirty_[slot] = 1;
+  }
+  // ... and one in which a leaf and its parent's mask were written: the records
+  // are listed, as long as there are not too many.
+  void mark_patch(uint32_t slot, uint64_t leaf, uint64_t leaf_parent) {
+    upload_.insert(slot);
+    if (body_dirty_[slot]) return;
+    if (patches_.size() + 2 > kMaxPatches) {
+      body_dirty_[slot] = 1;
+      return;
+    }
+    patches_.push_back((uint32_t)leaf);
+    patches_.push_back((uint32_t)leaf_parent);
+  }
+  // Every change so far is on the device.
+  void uploads_done() {
+    for (uint32_t s : upload_) body_dirty_[s] = 0;
+    upload_.clear();
+    patches_.clear();
+  }
+  static constexpr size_t kMaxPatches = 8192;
 
   svo_scene scene_;
   uint32_t N_ = 0;
@@ -138,6 +161,9 @@ class TreeletMemoryManager {
   std::vector<std::set<int32_t>> children_;
   std::vector<uint32_t> free_;  // top = back()
   std::set<uint32_t> upload_;
+  std::vector<uint8_t> body_dirty_;  // per slot in upload_: all of it, not only patches_
+  std::vector<uint32_t> patches_;    // changed records of the other slots in upload_
+  std::vector<uint32_t> used_;       // per slot: the mirror is zero from here on
   uint32_t search_pos_ = 1;
   float upload_ratio_ = 0.6f;
   bool evict_any_invisible_ = false;
@@ -187,7 +213,8 @@ class TreeletMemoryManagerCuda : public TreeletMemoryManager {
   // packed back to back into the pinned ring, one host-to-device copy per
   // 4 MB chunk, and a scatter kernel that moves each slot to its place.
   // SVO_UPLOAD_PINNED: the mirror itself is page-locked and mapped; one
-  // kernel reads the dirty slots from it over PCIe and writes them in place,
+  // kernel reads the dirty slots from it over PCIe and writes them in place
+  // (as far as they hold records, and single records where only leaves changed),
   // and whole-pool uploads (init_device_buffer, attach_device_buffers) are
   // two DMA copies straight from it.
   int set_upload_policy(int policy);
@@ -297,8 +324,12 @@ class TreeletMemoryManagerCuda : public TreeletMemoryManager {
   bool mirror_pinned_ = false;  // incore_ / incore_attr_ registered with CUDA
   const svo_node* mapped_nodes_ = nullptr;     // their device-side addresses
   const svo_attrib* mapped_attribs_ = nullptr;
-  uint32_t* h_slot_ids_ = nullptr;             // page-locked, mapped
-  const uint32_t* mapped_slot_ids_ = nullptr;
+  // page-locked, mapped: {slot, records} per slot, then {index, 0, record} per patch
+  uint32_t* h_jobs_ = nullptr;
+  const uint32_t* mapped_jobs_ = nullptr;
+  // the first patch's word: a patch is read in 16 bytes
+  size_t patches_at() const { return (2 * (size_t)num_slots() + 3) & ~(size_t)3; }
+  bool mirror_read_ = false;  // a copy out of the page-locked mirror may be in flight
   int stage_next_ = 0;
   uint32_t* d_rgba_ = nullptr;
   uint64_t d_rgba_pixels_ = 0;

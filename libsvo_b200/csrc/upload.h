@@ -13,11 +13,15 @@ namespace svo {
 int launch_slot_scatter(const void* stage, const uint32_t* ids, uint32_t count, uint64_t N,
                         svo_node* nodes, svo_attrib* attribs, cudaStream_t stream);
 
-// Reads `count` slots ids[i] straight from the page-locked, mapped host
-// mirror (host_nodes / host_attribs are its device-side addresses) and
-// writes them to the same slots of the device pools.
+// Brings `count` slots of the page-locked, mapped host mirror (host_nodes /
+// host_attribs are its device-side addresses) to the same slots of the device
+// pools -- jobs[2i] is a slot, jobs[2i + 1] the records that it holds; the rest
+// of it is zero and does not cross PCIe -- and writes `num_patches` single node
+// records: patches[4i] an index into the pool, patches[4i + 2], [4i + 3] the
+// record.
 int launch_slot_gather(const svo_node* host_nodes, const svo_attrib* host_attribs,
-                       const uint32_t* ids, uint32_t count, uint64_t N, svo_node* nodes,
-                       svo_attrib* attribs, cudaStream_t stream);
+                       const uint32_t* jobs, uint32_t count, uint64_t N, const uint32_t* patches,
+                       uint32_t num_patches, svo_node* nodes, svo_attrib* attribs,
+                       cudaStream_t stream);
 
 }  // namespace svo
