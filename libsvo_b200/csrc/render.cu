@@ -127,7 +127,10 @@ __device__ __forceinline__ bool block_pixel(const svo_frame_params& p, uint32_t 
 // the extra exit state.  With `order` (1-D grid) block r casts the r-th block
 // in estimated-cost order of a frame gx blocks wide; without it the grid is
 // the frame's blocks in raster order.
-template <bool kFlat, bool kExt>
+// kHost: rgba is page-locked host memory, written as the blocks end instead of
+// being copied after the last one.  A block's colours go through shared memory
+// so that its rows cross PCIe in 64-byte pieces (a warp's own tile has 32).
+template <bool kFlat, bool kExt, bool kHost>
 __global__ void __launch_bounds__(kThreads) render_frame_kernel(
     const uint2* __restrict__ nodes, const uint2* __restrict__ attribs, uint64_t num_nodes,
     const svo_frame_params p, int S, uint32_t* __restrict__ rgba, svo_hit* __restrict__ hits,
@@ -150,16 +153,30 @@ __global__ void __launch_bounds__(kThreads) render_frame_kernel(
     by = block / gx;
   }
   uint32_t x, y;
-  if (!block_pixel(p, bx, by, y0, rays, &x, &y)) return;
-  float o[3], dx, dy, dz;
-  pixel_ray(p, x, y, o, dx, dy, dz);
-  const RayHit h = cast_ray<kFlat>(GlobalFetch{nodes}, num_nodes, o, dx, dy, dz, p.t_scale_ratio,
-                                   S, stack_smem + t, kThreads);
-  const uint64_t pix = (uint64_t)y * p.width + x;
-  rgba[pix] = kExt ? shade_ext(p.mode, h, attribs, num_nodes, S, p.t_scale_ratio, dx, dy, dz)
-                   : shade(p.mode, h, attribs, num_nodes, S);
-  if (hits != nullptr) store_hit(hits, pix, h);
-  count_stats(stats, h);
+  const bool inside = block_pixel(p, bx, by, y0, rays, &x, &y);
+  if (!kHost && !inside) return;
+  uint32_t colour = 0u;
+  if (inside) {
+    float o[3], dx, dy, dz;
+    pixel_ray(p, x, y, o, dx, dy, dz);
+    const RayHit h = cast_ray<kFlat>(GlobalFetch{nodes}, num_nodes, o, dx, dy, dz, p.t_scale_ratio,
+                                     S, stack_smem + t, kThreads);
+    const uint64_t pix = (uint64_t)y * p.width + x;
+    colour = kExt ? shade_ext(p.mode, h, attribs, num_nodes, S, p.t_scale_ratio, dx, dy, dz)
+                  : shade(p.mode, h, attribs, num_nodes, S);
+    if (!kHost) rgba[pix] = colour;
+    if (hits != nullptr) store_hit(hits, pix, h);
+    count_stats(stats, h);
+  }
+  if (kHost) {
+    __shared__ uint32_t tile[kThreads];
+    const uint32_t rows = kBlockH / 4 * (rays / 8);  // of the block
+    const uint32_t bx0 = bx * kBlockW, by0 = y0 + by * rows;
+    if (lane < (int)rays) tile[(y - by0) * kBlockW + (x - bx0)] = colour;
+    __syncthreads();
+    const uint32_t px = bx0 + t % kBlockW, py = by0 + t / kBlockW;
+    if (t < (int)(rows * kBlockW) && px < p.width && py < p.height) rgba[(uint64_t)py * p.width + px] = tile[t];
+  }
 }
 
 // The bucket of a sample ray: six to a doubling of its expected iterations.
@@ -438,7 +455,7 @@ bool order_blocks(const uint2* nodes, uint64_t num_nodes, const svo_frame_params
 
 int launch_render(const svo_node* nodes, const svo_attrib* attribs, uint64_t num_nodes,
                   const svo_frame_params& p, const svo_trace_cfg& cfg, uint32_t* rgba,
-                  svo_hit* hits, svo_stats* stats, cudaStream_t stream) {
+                  svo_hit* hits, svo_stats* stats, cudaStream_t stream, bool host_image) {
   if (p.width == 0 || p.height == 0) return SVO_OK;
   if (p.height > 0xFFFFFFF0u) return SVO_ERR_RANGE;  // row indices stay below 2^32
   const int S = cfg.stack_size;
@@ -447,8 +464,11 @@ int launch_render(const svo_node* nodes, const svo_attrib* attribs, uint64_t num
   const uint2* a2 = reinterpret_cast<const uint2*>(attribs);
   const bool ext = p.mode == 2 || p.mode == 6 || p.mode == 7;
   const bool flat = cfg.traversal == SVO_TRAVERSAL_FLAT;
-  auto* fn = flat ? (ext ? render_frame_kernel<true, true> : render_frame_kernel<true, false>)
-                  : (ext ? render_frame_kernel<false, true> : render_frame_kernel<false, false>);
+  auto* fn = host_image
+                 ? (flat ? (ext ? render_frame_kernel<true, true, true> : render_frame_kernel<true, false, true>)
+                         : (ext ? render_frame_kernel<false, true, true> : render_frame_kernel<false, false, true>))
+                 : (flat ? (ext ? render_frame_kernel<true, true, false> : render_frame_kernel<true, false, false>)
+                         : (ext ? render_frame_kernel<false, true, false> : render_frame_kernel<false, false, false>));
   const uint32_t gx = (p.width + kBlockW - 1) / kBlockW;
   const uint64_t nblocks64 = (uint64_t)gx * ((p.height + kBlockH - 1) / kBlockH);
   BlockOrder order{nullptr, nullptr, 0u};

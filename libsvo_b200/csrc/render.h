@@ -20,9 +20,10 @@ inline uint32_t rays_per_warp(uint64_t rays) {
   return rays <= (1u << 14) ? 8u : (rays <= (3u << 14) ? 16u : 32u);
 }
 
+// host_image: rgba is the device-side address of page-locked host memory.
 int launch_render(const svo_node* nodes, const svo_attrib* attribs, uint64_t num_nodes,
                   const svo_frame_params& p, const svo_trace_cfg& cfg, uint32_t* rgba,
-                  svo_hit* hits, svo_stats* stats, cudaStream_t stream);
+                  svo_hit* hits, svo_stats* stats, cudaStream_t stream, bool host_image = false);
 
 int launch_render_shadow(const svo_node* nodes, const svo_attrib* attribs, uint64_t num_nodes,
                          const svo_frame_params& p, const svo_shadow_cfg& sc, int stack_size,
