@@ -41,8 +41,8 @@
 //
 // Scratch comes from a stream-ordered memory pool of the library's own; the host
 // waits four times a chunk for a size.  An 81,920-triangle icosphere at depth 11
-// (13 M leaves, 17.3 M nodes, a 628 MB pool) takes 4.1 ms (69.7 before), a 131,072-triangle
-// terrain at depth 9 0.96 ms (22.7), the 5.2 M-triangle depth-14 octree 0.67 s (1.61).
+// (13 M leaves, 17.3 M nodes, a 628 MB pool) takes 3.2 ms (69.7 before), a 131,072-triangle
+// terrain at depth 9 0.95 ms (22.7), the 5.2 M-triangle depth-14 octree 0.70 s (1.61).
 //
 // FP32 arithmetic uses explicit round-to-nearest intrinsics in the host
 // builder's operation order (the library is built with -fmad=false), so the
@@ -110,55 +110,6 @@ __device__ __forceinline__ int cell_floor(float x, uint32_t R) {
 
 __device__ __forceinline__ float dot3(float ax, float ay, float az, const float v[3]) {
   return __fadd_rn(__fadd_rn(__fmul_rn(ax, v[0]), __fmul_rn(ay, v[1])), __fmul_rn(az, v[2]));
-}
-
-__device__ __forceinline__ bool separated(float ax, float ay, float az, const float v0[3],
-                                          const float v1[3], const float v2[3], float h) {
-  const float p0 = dot3(ax, ay, az, v0), p1 = dot3(ax, ay, az, v1), p2 = dot3(ax, ay, az, v2);
-  const float mn = smin(p0, smin(p1, p2)), mx = smax(p0, smax(p1, p2));
-  const float r = __fmul_rn(h, __fadd_rn(__fadd_rn(fabsf(ax), fabsf(ay)), fabsf(az)));
-  return mn > r || mx < -r;
-}
-
-// tri_box_overlap of the host builder (Akenine-Moeller 2001, restated there).
-__device__ bool tri_box_overlap(const float bc[3], float h, const float a[3], const float b[3],
-                                const float c[3]) {
-  float v0[3], v1[3], v2[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    v0[i] = __fsub_rn(a[i], bc[i]);
-    v1[i] = __fsub_rn(b[i], bc[i]);
-    v2[i] = __fsub_rn(c[i], bc[i]);
-  }
-  const float e[3][3] = {{__fsub_rn(v1[0], v0[0]), __fsub_rn(v1[1], v0[1]), __fsub_rn(v1[2], v0[2])},
-                         {__fsub_rn(v2[0], v1[0]), __fsub_rn(v2[1], v1[1]), __fsub_rn(v2[2], v1[2])},
-                         {__fsub_rn(v0[0], v2[0]), __fsub_rn(v0[1], v2[1]), __fsub_rn(v0[2], v2[2])}};
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const float* ek = e[k];
-    if (separated(0.0f, ek[2], -ek[1], v0, v1, v2, h)) return false;
-    if (separated(-ek[2], 0.0f, ek[0], v0, v1, v2, h)) return false;
-    if (separated(ek[1], -ek[0], 0.0f, v0, v1, v2, h)) return false;
-  }
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const float mn = smin(v0[i], smin(v1[i], v2[i]));
-    const float mx = smax(v0[i], smax(v1[i], v2[i]));
-    if (mn > h || mx < -h) return false;
-  }
-  const float n[3] = {
-      __fsub_rn(__fmul_rn(e[0][1], e[1][2]), __fmul_rn(e[0][2], e[1][1])),
-      __fsub_rn(__fmul_rn(e[0][2], e[1][0]), __fmul_rn(e[0][0], e[1][2])),
-      __fsub_rn(__fmul_rn(e[0][0], e[1][1]), __fmul_rn(e[0][1], e[1][0]))};
-  const float d = -dot3(n[0], n[1], n[2], v0);
-  float vmin[3], vmax[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    vmin[i] = n[i] > 0.0f ? -h : h;
-    vmax[i] = n[i] > 0.0f ? h : -h;
-  }
-  if (__fadd_rn(dot3(n[0], n[1], n[2], vmin), d) > 0.0f) return false;
-  return __fadd_rn(dot3(n[0], n[1], n[2], vmax), d) >= 0.0f;
 }
 
 // ---- 1. triangle records -------------------------------------------------------
@@ -255,52 +206,67 @@ struct Chunk {
 };
 
 // A triangle as the voxeliser walks it: columns of voxels along axis w (the
-// dominant one of its normal), iu in [ulo, ulo + nu), iv in [vlo, vlo + nv).
-struct TriWalk {
-  float a[3], b[3], c[3], n[3], pd;
-  int w, u, v, ulo, vlo, wlo, whi;
-  uint32_t nu, nv;  // both 0: no candidate voxel in the chunk
+// dominant one of its normal), iu in [ulo, ulo + nu), iv in [vlo, vlo + nv).  Its
+// coordinates are kept in the order (u, v, w), a cyclic turn of (x, y, z).
+struct __align__(16) TriWalk {
+  float a[3], b[3], c[3], n[3], pd;  // pd: dot(n, a), in the order x, y, z
+  int w, ulo, vlo, wlo, whi;
+  uint32_t nv, pad;
 };
+static_assert(sizeof(TriWalk) == 80, "five 16-byte loads");
 
-__device__ __forceinline__ void tri_walk(const float* __restrict__ V,
-                                         const uint32_t* __restrict__ T, uint64_t t,
-                                         uint32_t depth, const Chunk& ch, TriWalk& s) {
+__device__ __forceinline__ float turned(const float* x, int w, int k) {  // k: 0 u, 1 v, 2 w
+  const int i = k == 2 ? w : (k == 0 ? (w == 2 ? 0 : w + 1) : (w == 0 ? 2 : w - 1));
+  return i == 0 ? x[0] : (i == 1 ? x[1] : x[2]);
+}
+__device__ __forceinline__ int turned(const int* x, int w, int k) {
+  const int i = k == 2 ? w : (k == 0 ? (w == 2 ? 0 : w + 1) : (w == 0 ? 2 : w - 1));
+  return i == 0 ? x[0] : (i == 1 ? x[1] : x[2]);
+}
+
+// Returns the number of columns with candidate voxels in the chunk.
+__device__ __forceinline__ uint64_t tri_walk(const float* __restrict__ V,
+                                             const uint32_t* __restrict__ T, uint64_t t,
+                                             uint32_t depth, const Chunk& ch, TriWalk& s) {
   const uint32_t R = 1u << depth;
   const float Rf = (float)R;
   const uint64_t i0 = 3 * (uint64_t)T[3 * t], i1 = 3 * (uint64_t)T[3 * t + 1],
                  i2 = 3 * (uint64_t)T[3 * t + 2];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    s.a[k] = V[i0 + k];
-    s.b[k] = V[i1 + k];
-    s.c[k] = V[i2 + k];
-  }
-  face_normal(s.a, s.b, s.c, s.n);
+  const float a[3] = {V[i0], V[i0 + 1], V[i0 + 2]}, b[3] = {V[i1], V[i1 + 1], V[i1 + 2]},
+              c[3] = {V[i2], V[i2 + 1], V[i2 + 2]};
+  float n[3];
+  face_normal(a, b, c, n);
   int lo[3], hi[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const float mn = smin(s.a[k], smin(s.b[k], s.c[k]));
-    const float mx = smax(s.a[k], smax(s.b[k], s.c[k]));
+    const float mn = smin(a[k], smin(b[k], c[k]));
+    const float mx = smax(a[k], smax(b[k], c[k]));
     lo[k] = max(0, cell_floor(__fmul_rn(__fadd_rn(mn, 0.5f), Rf), R));
     hi[k] = min((int)R - 1, cell_floor(__fmul_rn(__fadd_rn(mx, 0.5f), Rf), R));
   }
-  s.w = 0;
-  if (fabsf(s.n[1]) > fabsf(s.n[0])) s.w = 1;
-  if (fabsf(s.n[2]) > fabsf(s.w == 1 ? s.n[1] : s.n[0])) s.w = 2;
-  s.u = s.w == 2 ? 0 : s.w + 1;
-  s.v = s.u == 2 ? 0 : s.u + 1;
-  s.pd = dot3(s.n[0], s.n[1], s.n[2], s.a);
-  const bool none = lo[0] > hi[0] || lo[1] > hi[1] || lo[2] > hi[2];
+  int w = 0;
+  if (fabsf(n[1]) > fabsf(n[0])) w = 1;
+  if (fabsf(n[2]) > fabsf(w == 1 ? n[1] : n[0])) w = 2;
+  s.w = w;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    s.a[k] = turned(a, w, k);
+    s.b[k] = turned(b, w, k);
+    s.c[k] = turned(c, w, k);
+    s.n[k] = turned(n, w, k);
+  }
+  s.pd = dot3(n[0], n[1], n[2], a);
   // the chunk restricts the (u, v) range and each column's w range
-  auto pick = [](const int* x, int k) { return k == 0 ? x[0] : (k == 1 ? x[1] : x[2]); };
-  s.ulo = max(pick(lo, s.u), pick(ch.lo, s.u));
-  s.vlo = max(pick(lo, s.v), pick(ch.lo, s.v));
-  const int uhi = min(pick(hi, s.u), pick(ch.hi, s.u)), vhi = min(pick(hi, s.v), pick(ch.hi, s.v));
-  s.wlo = pick(lo, s.w);
-  s.whi = pick(hi, s.w);
-  const bool out = none || s.ulo > uhi || s.vlo > vhi || max(s.wlo, pick(ch.lo, s.w)) > min(s.whi, pick(ch.hi, s.w));
-  s.nu = out ? 0u : (uint32_t)(uhi - s.ulo + 1);
-  s.nv = out ? 0u : (uint32_t)(vhi - s.vlo + 1);
+  s.ulo = max(turned(lo, w, 0), turned(ch.lo, w, 0));
+  s.vlo = max(turned(lo, w, 1), turned(ch.lo, w, 1));
+  const int uhi = min(turned(hi, w, 0), turned(ch.hi, w, 0)), vhi = min(turned(hi, w, 1), turned(ch.hi, w, 1));
+  s.wlo = turned(lo, w, 2);
+  s.whi = turned(hi, w, 2);
+  s.pad = 0;
+  const bool none = lo[0] > hi[0] || lo[1] > hi[1] || lo[2] > hi[2] || s.ulo > uhi || s.vlo > vhi ||
+                    max(s.wlo, turned(ch.lo, w, 2)) > min(s.whi, turned(ch.hi, w, 2));
+  s.nv = none ? 0u : (uint32_t)(vhi - s.vlo + 1);
+  return none ? 0ull : (uint64_t)(uint32_t)(uhi - s.ulo + 1) * s.nv;
 }
 
 // The candidate voxels of column (iu, iv), w from *wlo to *whi.
@@ -309,11 +275,9 @@ __device__ __forceinline__ void column_range(const TriWalk& s, uint32_t depth, c
   const uint32_t R = 1u << depth;
   const float Rf = (float)R;
   const float inv = __fdiv_rn(1.0f, Rf);
-  auto pick = [](const float* x, int k) { return k == 0 ? x[0] : (k == 1 ? x[1] : x[2]); };
-  const float nw = pick(s.n, s.w), nu = pick(s.n, s.u), nv = pick(s.n, s.v);
   *wlo = s.wlo;
   *whi = s.whi;
-  if (nw != 0.0f) {
+  if (s.n[2] != 0.0f) {
     const float u0 = __fadd_rn(-0.5f, __fmul_rn((float)iu, inv)), u1 = __fadd_rn(u0, inv);
     const float v0 = __fadd_rn(-0.5f, __fmul_rn((float)iv, inv)), v1 = __fadd_rn(v0, inv);
     float wmin = 1e30f, wmax = -1e30f;
@@ -323,39 +287,113 @@ __device__ __forceinline__ void column_range(const TriWalk& s, uint32_t depth, c
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const float ww = __fdiv_rn(
-            __fsub_rn(__fsub_rn(s.pd, __fmul_rn(nu, us[i])), __fmul_rn(nv, vs[j])), nw);
+            __fsub_rn(__fsub_rn(s.pd, __fmul_rn(s.n[0], us[i])), __fmul_rn(s.n[1], vs[j])), s.n[2]);
         wmin = smin(wmin, ww);
         wmax = smax(wmax, ww);
       }
     *wlo = max(*wlo, cell_floor(__fmul_rn(__fadd_rn(wmin, 0.5f), Rf), R) - 1);
     *whi = min(*whi, cell_floor(__fmul_rn(__fadd_rn(wmax, 0.5f), Rf), R) + 1);
   }
-  const int clo = s.w == 0 ? ch.lo[0] : (s.w == 1 ? ch.lo[1] : ch.lo[2]);
-  const int chi = s.w == 0 ? ch.hi[0] : (s.w == 1 ? ch.hi[1] : ch.hi[2]);
-  *wlo = max(*wlo, clo);
-  *whi = min(*whi, chi);
+  *wlo = max(*wlo, turned(ch.lo, s.w, 2));
+  *whi = min(*whi, turned(ch.hi, s.w, 2));
 }
 
-__device__ __forceinline__ void voxel_of(const TriWalk& s, int iu, int iv, int iw, uint32_t ijk[3]) {
-  ijk[0] = (uint32_t)(s.w == 0 ? iw : (s.u == 0 ? iu : iv));
-  ijk[1] = (uint32_t)(s.w == 1 ? iw : (s.u == 1 ? iu : iv));
-  ijk[2] = (uint32_t)(s.w == 2 ? iw : (s.u == 2 ? iu : iv));
+// The host builder's tri_box_overlap (Akenine-Moeller 2001, restated there) in
+// two parts.  A voxel overlaps when no axis separates it from the triangle, in
+// whatever order the axes are tried, and the axes without a w component see the
+// same values in every voxel of a column, bit for bit: they are tried once a
+// column (half of the columns of a triangle's box end there), the others per
+// voxel.  An axis is the cross product of an edge and a coordinate axis, so it
+// has a zero and two components, whose products may be summed in any order; the
+// zero's product is kept for coordinates that are not finite.
+__device__ __forceinline__ bool separated(float s, float t, float p0s, float p0t, float p0z, float p1s,
+                                          float p1t, float p1z, float p2s, float p2t, float p2z, float h) {
+  const float p0 = __fadd_rn(__fadd_rn(__fmul_rn(s, p0s), __fmul_rn(t, p0t)), __fmul_rn(0.0f, p0z));
+  const float p1 = __fadd_rn(__fadd_rn(__fmul_rn(s, p1s), __fmul_rn(t, p1t)), __fmul_rn(0.0f, p1z));
+  const float p2 = __fadd_rn(__fadd_rn(__fmul_rn(s, p2s), __fmul_rn(t, p2t)), __fmul_rn(0.0f, p2z));
+  const float mn = smin(p0, smin(p1, p2)), mx = smax(p0, smax(p1, p2));
+  const float r = __fmul_rn(h, __fadd_rn(fabsf(s), fabsf(t)));
+  return mn > r || mx < -r;
 }
 
-__device__ __forceinline__ bool voxel_hit(const TriWalk& s, uint32_t depth, const uint32_t ijk[3]) {
+__device__ __forceinline__ float center_of(int i, float inv) {
+  return __fadd_rn(-0.5f, __fmul_rn(__fadd_rn((float)i, 0.5f), inv));
+}
+
+__device__ __forceinline__ bool column_may_overlap(const TriWalk& s, uint32_t depth, int iu, int iv) {
   const float inv = __fdiv_rn(1.0f, (float)(1u << depth));
   const float h = __fmul_rn(0.5f, inv);
-  const float bc[3] = {__fadd_rn(-0.5f, __fmul_rn(__fadd_rn((float)ijk[0], 0.5f), inv)),
-                       __fadd_rn(-0.5f, __fmul_rn(__fadd_rn((float)ijk[1], 0.5f), inv)),
-                       __fadd_rn(-0.5f, __fmul_rn(__fadd_rn((float)ijk[2], 0.5f), inv))};
-  return tri_box_overlap(bc, h, s.a, s.b, s.c);
+  const float bu = center_of(iu, inv), bv = center_of(iv, inv);
+  const float u[3] = {__fsub_rn(s.a[0], bu), __fsub_rn(s.b[0], bu), __fsub_rn(s.c[0], bu)};
+  const float v[3] = {__fsub_rn(s.a[1], bv), __fsub_rn(s.b[1], bv), __fsub_rn(s.c[1], bv)};
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float eu = __fsub_rn(u[(k + 1) % 3], u[k]), ev = __fsub_rn(v[(k + 1) % 3], v[k]);
+    if (separated(ev, -eu, u[0], v[0], s.a[2], u[1], v[1], s.b[2], u[2], v[2], s.c[2], h)) return false;
+  }
+  if (smin(u[0], smin(u[1], u[2])) > h || smax(u[0], smax(u[1], u[2])) < -h) return false;
+  return !(smin(v[0], smin(v[1], v[2])) > h || smax(v[0], smax(v[1], v[2])) < -h);
 }
 
-// cols[t]: the columns of triangle t inside the chunk; cols[nt] = 0, so that an
-// exclusive sum over nt + 1 entries ends with the total.
+// u, v and w products summed in the order x, y, z.
+__device__ __forceinline__ float sum_xyz(float u, float v, float w, int axis) {
+  const float x = axis == 0 ? w : (axis == 1 ? v : u), y = axis == 0 ? u : (axis == 1 ? w : v),
+              z = axis == 0 ? v : (axis == 1 ? u : w);
+  return __fadd_rn(__fadd_rn(x, y), z);
+}
+
+__device__ __forceinline__ bool voxel_overlaps(const TriWalk& s, uint32_t depth, int iu, int iv, int iw) {
+  const float inv = __fdiv_rn(1.0f, (float)(1u << depth));
+  const float h = __fmul_rn(0.5f, inv);
+  const float bc[3] = {center_of(iu, inv), center_of(iv, inv), center_of(iw, inv)};
+  float p[3][3];  // vertex, coordinate
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    p[0][k] = __fsub_rn(s.a[k], bc[k]);
+    p[1][k] = __fsub_rn(s.b[k], bc[k]);
+    p[2][k] = __fsub_rn(s.c[k], bc[k]);
+  }
+  if (smin(p[0][2], smin(p[1][2], p[2][2])) > h || smax(p[0][2], smax(p[1][2], p[2][2])) < -h) return false;
+  float e[3][3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) e[k][i] = __fsub_rn(p[(k + 1) % 3][i], p[k][i]);
+  float n[3], f[3], g[3], m[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const int j = (i + 1) % 3, k = (i + 2) % 3;
+    n[i] = __fsub_rn(__fmul_rn(e[0][j], e[1][k]), __fmul_rn(e[0][k], e[1][j]));
+    f[i] = __fmul_rn(n[i], p[0][i]);
+    g[i] = __fmul_rn(n[i], n[i] > 0.0f ? -h : h);
+    m[i] = __fmul_rn(n[i], n[i] > 0.0f ? h : -h);
+  }
+  const float d = -sum_xyz(f[0], f[1], f[2], s.w);
+  if (__fadd_rn(sum_xyz(g[0], g[1], g[2], s.w), d) > 0.0f) return false;
+  if (!(__fadd_rn(sum_xyz(m[0], m[1], m[2], s.w), d) >= 0.0f)) return false;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    if (separated(e[k][2], -e[k][1], p[0][1], p[0][2], p[0][0], p[1][1], p[1][2], p[1][0], p[2][1], p[2][2],
+                  p[2][0], h))
+      return false;
+    if (separated(e[k][0], -e[k][2], p[0][2], p[0][0], p[0][1], p[1][2], p[1][0], p[1][1], p[2][2], p[2][0],
+                  p[2][1], h))
+      return false;
+  }
+  return true;
+}
+
+__device__ __forceinline__ uint64_t voxel_code(int w, int iu, int iv, int iw) {
+  const uint32_t x = (uint32_t)(w == 0 ? iw : (w == 1 ? iv : iu)), y = (uint32_t)(w == 0 ? iu : (w == 1 ? iw : iv)),
+                 z = (uint32_t)(w == 0 ? iv : (w == 1 ? iu : iw));
+  return morton3(x, y, z);
+}
+
+// walks[t], and cols[t]: the columns of triangle t inside the chunk; cols[nt] =
+// 0, so that an exclusive sum over nt + 1 entries ends with the total.
 __global__ void column_count_kernel(const float* __restrict__ V, const uint32_t* __restrict__ T,
                                     uint64_t nt, uint32_t depth, Chunk ch,
-                                    uint64_t* __restrict__ cols) {
+                                    TriWalk* __restrict__ walks, uint64_t* __restrict__ cols) {
   const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t > nt) return;
   if (t == nt) {
@@ -363,8 +401,8 @@ __global__ void column_count_kernel(const float* __restrict__ V, const uint32_t*
     return;
   }
   TriWalk s;
-  tri_walk(V, T, t, depth, ch, s);
-  cols[t] = (uint64_t)s.nu * s.nv;
+  cols[t] = tri_walk(V, T, t, depth, ch, s);
+  walks[t] = s;
 }
 
 // The last index of off[lo..hi] whose value is <= x (off[lo] <= x).
@@ -386,41 +424,51 @@ constexpr int kColThreads = 256;
 // (a triangle without a dominant axis) are tested again where they are emitted.
 constexpr uint32_t kTestAgain = 0xFFFFFFFFu;
 
-// The triangle of column c: the block's first and last column are looked up in
-// all of `off`, the others between those two.
-__device__ __forceinline__ uint64_t column_triangle(const uint64_t* __restrict__ off, uint64_t nt,
-                                                    uint64_t columns, uint64_t c) {
-  __shared__ uint64_t ends[2];
-  const uint64_t base = (uint64_t)blockIdx.x * kColThreads;
-  if (threadIdx.x == 0) ends[0] = last_at_most(off, 0, nt - 1, base);
-  if (threadIdx.x == 32)
-    ends[1] = last_at_most(off, 0, nt - 1, min(base + kColThreads - 1, columns - 1));
-  __syncthreads();
-  return c < columns ? last_at_most(off, ends[0], ends[1], c) : 0;
+// block_tri[b]: the triangle of the first column of block b, and of the last
+// column behind the last block.  (Looked up by one thread of each block, the
+// search was a third of the test and half of the emission.)
+__global__ void block_triangles_kernel(const uint64_t* __restrict__ off, uint64_t nt, uint64_t columns,
+                                       uint64_t blocks, uint32_t* __restrict__ block_tri) {
+  const uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (b <= blocks)
+    block_tri[b] = (uint32_t)last_at_most(off, 0, nt - 1, min(b * kColThreads, columns - 1));
+}
+
+// The triangle of column c, and the column's place (iu, iv) in it.
+__device__ __forceinline__ uint64_t column_triangle(const uint64_t* __restrict__ off,
+                                                    const uint32_t* __restrict__ block_tri, uint64_t c) {
+  return last_at_most(off, block_tri[blockIdx.x], block_tri[blockIdx.x + 1], c);
+}
+__device__ __forceinline__ void column_place(const TriWalk& s, uint64_t k, int* iu, int* iv) {
+  uint64_t row;
+  if (k >> 32)  // a triangle of more than 2^32 columns
+    row = k / s.nv;
+  else
+    row = (uint32_t)k / s.nv;
+  *iu = s.ulo + (int)row;
+  *iv = s.vlo + (int)(uint32_t)(k - row * s.nv);
 }
 
 __global__ void __launch_bounds__(kColThreads) column_test_kernel(
-    const float* __restrict__ V, const uint32_t* __restrict__ T, uint64_t nt, uint32_t depth,
-    Chunk ch, const uint64_t* __restrict__ off, uint64_t columns, uint32_t* __restrict__ rec,
-    uint64_t* __restrict__ block_hits) {
+    const TriWalk* __restrict__ walks, uint32_t depth, Chunk ch,
+    const uint64_t* __restrict__ off, const uint32_t* __restrict__ block_tri, uint64_t columns,
+    uint32_t* __restrict__ rec, uint64_t* __restrict__ block_hits) {
   const uint64_t c = (uint64_t)blockIdx.x * kColThreads + threadIdx.x;
-  const uint64_t t = column_triangle(off, nt, columns, c);
   uint32_t hits = 0;
   if (c < columns) {
-    TriWalk s;
-    tri_walk(V, T, t, depth, ch, s);
-    const uint64_t k = c - off[t];
-    const int iu = s.ulo + (int)(k / s.nv), iv = s.vlo + (int)(k % s.nv);
-    int wlo, whi;
-    column_range(s, depth, ch, iu, iv, &wlo, &whi);
+    const uint64_t t = column_triangle(off, block_tri, c);
+    const TriWalk s = walks[t];
+    int iu, iv;
+    column_place(s, c - off[t], &iu, &iv);
+    int wlo = 0, whi = -1;
     uint32_t mask = 0;
-    for (int iw = wlo; iw <= whi; ++iw) {
-      uint32_t ijk[3];
-      voxel_of(s, iu, iv, iw, ijk);
-      if (voxel_hit(s, depth, ijk)) {
-        ++hits;
-        mask |= 1u << ((iw - wlo) & 31);
-      }
+    if (column_may_overlap(s, depth, iu, iv)) {
+      column_range(s, depth, ch, iu, iv, &wlo, &whi);
+      for (int iw = wlo; iw <= whi; ++iw)
+        if (voxel_overlaps(s, depth, iu, iv, iw)) {
+          ++hits;
+          mask |= 1u << ((iw - wlo) & 31);
+        }
     }
     rec[c] = hits == 0 ? 0u : (whi - wlo >= 8 ? kTestAgain : ((uint32_t)wlo << 8) | mask);
   }
@@ -437,27 +485,23 @@ __global__ void __launch_bounds__(kColThreads) column_test_kernel(
 }
 
 __global__ void __launch_bounds__(kColThreads) column_emit_kernel(
-    const float* __restrict__ V, const uint32_t* __restrict__ T, uint64_t nt, uint32_t depth,
-    Chunk ch, const uint64_t* __restrict__ off, uint64_t columns, const uint32_t* __restrict__ rec,
+    const TriWalk* __restrict__ walks, uint32_t depth, Chunk ch,
+    const uint64_t* __restrict__ off, const uint32_t* __restrict__ block_tri, uint64_t columns,
+    const uint32_t* __restrict__ rec,
     const uint64_t* __restrict__ block_off, uint64_t* __restrict__ keys) {
   const uint64_t c = (uint64_t)blockIdx.x * kColThreads + threadIdx.x;
-  const uint64_t t = column_triangle(off, nt, columns, c);
   const uint32_t r = c < columns ? rec[c] : 0u;
-  TriWalk s;
-  int iu = 0, iv = 0, wlo = 0, whi = -1;
+  uint64_t t = 0;
+  int w = 0, iu = 0, iv = 0, wlo = 0, whi = -1;
   uint32_t n = 0;
   if (r != 0u) {
-    tri_walk(V, T, t, depth, ch, s);
-    const uint64_t k = c - off[t];
-    iu = s.ulo + (int)(k / s.nv);
-    iv = s.vlo + (int)(k % s.nv);
+    t = column_triangle(off, block_tri, c);
+    const TriWalk& s = walks[t];
+    w = s.w;
+    column_place(s, c - off[t], &iu, &iv);
     if (r == kTestAgain) {
       column_range(s, depth, ch, iu, iv, &wlo, &whi);
-      for (int iw = wlo; iw <= whi; ++iw) {
-        uint32_t ijk[3];
-        voxel_of(s, iu, iv, iw, ijk);
-        n += voxel_hit(s, depth, ijk) ? 1u : 0u;
-      }
+      for (int iw = wlo; iw <= whi; ++iw) n += voxel_overlaps(s, depth, iu, iv, iw) ? 1u : 0u;
     } else {
       wlo = (int)(r >> 8);
       n = (uint32_t)__popc(r & 0xFFu);
@@ -477,17 +521,10 @@ __global__ void __launch_bounds__(kColThreads) column_emit_kernel(
   for (uint32_t i = 0; i < warp; ++i) pos += warp_sum[i];
   if (r == 0u) return;
   const uint64_t low = ch.shift >= 64 ? ~0ull : ((1ull << ch.shift) - 1ull);
-  auto put = [&](int iw) {
-    uint32_t ijk[3];
-    voxel_of(s, iu, iv, iw, ijk);
-    keys[pos++] = ((morton3(ijk[0], ijk[1], ijk[2]) & low) << ch.tri_bits) | t;
-  };
+  auto put = [&](int iw) { keys[pos++] = ((voxel_code(w, iu, iv, iw) & low) << ch.tri_bits) | t; };
   if (r == kTestAgain) {
-    for (int iw = wlo; iw <= whi; ++iw) {
-      uint32_t ijk[3];
-      voxel_of(s, iu, iv, iw, ijk);
-      if (voxel_hit(s, depth, ijk)) put(iw);
-    }
+    for (int iw = wlo; iw <= whi; ++iw)
+      if (voxel_overlaps(walks[t], depth, iu, iv, iw)) put(iw);
   } else {
     for (uint32_t m = r & 0xFFu; m != 0u; m &= m - 1u) put(wlo + __ffs((int)m) - 1);
   }
@@ -527,7 +564,8 @@ __global__ void __launch_bounds__(kKeyThreads) level_count_kernel(KeyLevels kl, 
 #pragma unroll
   for (int r = 0; r < kKeyRows; ++r)
     k[r] = kl((uint64_t)blockIdx.x * kKeyBlock + r * kKeyThreads + threadIdx.x);
-  for (uint32_t d = 0; d <= kl.depth; ++d) {
+  // few warps begin a node of the upper levels
+  for (uint32_t d = __reduce_min_sync(0xFFFFFFFFu, min(min(k[0], k[1]), min(k[2], k[3]))); d <= kl.depth; ++d) {
     uint32_t n = 0;
 #pragma unroll
     for (int r = 0; r < kKeyRows; ++r) n += (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, k[r] <= d));
@@ -640,40 +678,49 @@ __device__ __forceinline__ void leaf_contribution(const TriRecord& r, const floa
   }
 }
 
-// The attributes of the leaf whose first key is i: over its triangles in order,
-// the mean of the interpolated normals (normalised) and colours, or the
-// normalised sum of the face normals.
-__device__ __forceinline__ svo_attrib leaf_attrib(const KeyLevels& kl, const LeafInput& in,
-                                                  uint64_t i) {
-  const uint64_t code = kl.keys[i] >> kl.tri_bits;
-  const uint64_t tmask = (1ull << kl.tri_bits) - 1ull;
-  const uint64_t full = in.chunk_base | code;
-  const float inv_r = __fdiv_rn(1.0f, (float)(1u << kl.depth));
-  const uint32_t x = compact3(full >> 2), y = compact3(full >> 1), z = compact3(full);
-  const float c[3] = {__fadd_rn(-0.5f, __fmul_rn(__fadd_rn((float)x, 0.5f), inv_r)),
-                      __fadd_rn(-0.5f, __fmul_rn(__fadd_rn((float)y, 0.5f), inv_r)),
-                      __fadd_rn(-0.5f, __fmul_rn(__fadd_rn((float)z, 0.5f), inv_r))};
-  float sn[3] = {0.0f, 0.0f, 0.0f}, sc[3] = {0.0f, 0.0f, 0.0f};
-  uint64_t j = i, key = kl.keys[i];
-  do {
-    const uint64_t t = key & tmask;
-    float nn[3], cc[3] = {0.0f, 0.0f, 0.0f};
-    if (in.records != nullptr) {
-      const TriRecord r = in.records[t];
-      leaf_contribution(r, c, nn, cc);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) nn[k] = in.face_normals[3 * t + k];
-    }
+// One triangle's contribution to the leaf `code`.
+struct LeafPart {
+  float n[3], c[3];
+};
+__device__ __forceinline__ LeafPart leaf_part(const LeafInput& in, uint32_t depth, uint64_t code,
+                                              uint64_t t) {
+  LeafPart p;
+  if (in.records != nullptr) {
+    const float inv = __fdiv_rn(1.0f, (float)(1u << depth));
+    const float c[3] = {center_of((int)compact3(code >> 2), inv), center_of((int)compact3(code >> 1), inv),
+                        center_of((int)compact3(code), inv)};
+    leaf_contribution(in.records[t], c, p.n, p.c);
+  } else {
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      sn[k] = __fadd_rn(sn[k], nn[k]);
-      sc[k] = __fadd_rn(sc[k], cc[k]);
+      p.n[k] = in.face_normals[3 * t + k];
+      p.c[k] = 0.0f;
+    }
+  }
+  return p;
+}
+
+// The attributes of the leaf whose first key is i: over its triangles in order,
+// the mean of the interpolated normals (normalised) and colours, or the
+// normalised sum of the face normals.  The contributions of the keys up to `end`
+// are in `part`; a run that crosses it has the others made here.
+__device__ __forceinline__ svo_attrib leaf_attrib(const KeyLevels& kl, const LeafInput& in, uint64_t code,
+                                                  uint64_t i, uint64_t end,
+                                                  const LeafPart* __restrict__ part) {
+  const uint64_t own = kl.keys[i] >> kl.tri_bits;
+  float sn[3] = {0.0f, 0.0f, 0.0f}, sc[3] = {0.0f, 0.0f, 0.0f};
+  uint64_t j = i;
+  do {
+    const LeafPart p = j < end ? part[kKeyThreads - (end - j)]
+                               : leaf_part(in, kl.depth, code, kl.keys[j] & ((1ull << kl.tri_bits) - 1ull));
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      sn[k] = __fadd_rn(sn[k], p.n[k]);
+      sc[k] = __fadd_rn(sc[k], p.c[k]);
     }
     ++j;
-    if (j < kl.n) key = kl.keys[j];
-  } while (j < kl.n && (key >> kl.tri_bits) == code);
-  if (in.records != nullptr) {
+  } while (j < kl.n && (kl.keys[j] >> kl.tri_bits) == own);
+  if (in.records != nullptr && j - i > 1) {  // x / 1 is x
     const float cnt = (float)(j - i);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -703,14 +750,19 @@ __global__ void __launch_bounds__(kKeyThreads) level_write_kernel(
   constexpr int kGroups = kKeyRows * kKeyThreads / 32;
   static_assert(kGroups == 32, "one warp scans the groups of a level");
   __shared__ uint32_t before[kMaxLevels][kGroups];
+  __shared__ LeafPart part[kKeyThreads];
   const uint32_t lane = threadIdx.x % 32, warp = threadIdx.x / 32;
   uint32_t k[kKeyRows];
 #pragma unroll
   for (int r = 0; r < kKeyRows; ++r)
     k[r] = kl((uint64_t)blockIdx.x * kKeyBlock + r * kKeyThreads + threadIdx.x);
-  for (uint32_t d = 0; d <= kl.depth; ++d) {
+  for (uint32_t i = threadIdx.x; i < (kl.depth + 1) * kGroups; i += kKeyThreads) (&before[0][0])[i] = 0u;
+  __syncthreads();
+  uint32_t top[kKeyRows];  // the coarsest level that begins in the row's warp
 #pragma unroll
-    for (int r = 0; r < kKeyRows; ++r) {
+  for (int r = 0; r < kKeyRows; ++r) {
+    top[r] = __reduce_min_sync(0xFFFFFFFFu, k[r]);
+    for (uint32_t d = top[r]; d <= kl.depth; ++d) {
       const uint32_t b = __ballot_sync(0xFFFFFFFFu, k[r] <= d);
       if (lane == 0) before[d][r * (kKeyThreads / 32) + warp] = (uint32_t)__popc(b);
     }
@@ -728,14 +780,18 @@ __global__ void __launch_bounds__(kKeyThreads) level_write_kernel(
   __syncthreads();
 #pragma unroll 1
   for (int r = 0; r < kKeyRows; ++r) {
-    const uint64_t i = (uint64_t)blockIdx.x * kKeyBlock + r * kKeyThreads + threadIdx.x;
-    const uint32_t kr = k[0];
+    const uint64_t row = (uint64_t)blockIdx.x * kKeyBlock + r * kKeyThreads, i = row + threadIdx.x;
+    const uint32_t kr = k[0], from = top[0];
     k[0] = k[1];
     k[1] = k[2];
     k[2] = k[3];
-    const uint64_t code = kr <= kl.depth ? in.chunk_base | (kl.keys[i] >> kl.tri_bits) : 0;
+    top[0] = top[1];
+    top[1] = top[2];
+    top[2] = top[3];
+    const uint64_t key = i < kl.n ? kl.keys[i] : 0;
+    const uint64_t code = in.chunk_base | (key >> kl.tri_bits);
     uint32_t up = 0;  // the node's index one level up
-    for (uint32_t d = 0; d <= kl.depth; ++d) {
+    for (uint32_t d = from; d <= kl.depth; ++d) {
       const uint32_t b = __ballot_sync(0xFFFFFFFFu, kr <= d);
       if (kr > d) continue;
       const uint32_t at = before[d][r * (kKeyThreads / 32) + warp] + __popc(b & ((1u << lane) - 1u));
@@ -743,7 +799,11 @@ __global__ void __launch_bounds__(kKeyThreads) level_write_kernel(
       out.octant[d][at] = (uint8_t)((code >> (3 * (kl.depth - d))) & 7u);
       up = at;
     }
-    if (kr <= kl.depth) out.leaf_attribs[up] = leaf_attrib(kl, in, i);
+    // every key's contribution, then the leaves' sums over theirs
+    if (i < kl.n) part[threadIdx.x] = leaf_part(in, kl.depth, code, key & ((1ull << kl.tri_bits) - 1ull));
+    __syncthreads();
+    if (kr <= kl.depth) out.leaf_attribs[up] = leaf_attrib(kl, in, code, i, row + kKeyThreads, part);
+    __syncthreads();
   }
 }
 
@@ -1112,6 +1172,16 @@ int sum_counts(const Scratch& sc, uint64_t* counts, uint64_t n, uint64_t* total)
   return SVO_OK;
 }
 
+template <class Count>
+int sort_keys(const Scratch& sc, cub::DoubleBuffer<uint64_t>& kb, Count n, int lo_bit, int hi_bit) {
+  size_t bytes = 0;
+  GB_TRY(cub::DeviceRadixSort::SortKeys(nullptr, bytes, kb, n, lo_bit, hi_bit, sc.st));
+  DevBuf<uint8_t> tmp;
+  GB_TRY(tmp.alloc(sc, bytes));
+  GB_TRY(cub::DeviceRadixSort::SortKeys(tmp.p, bytes, kb, n, lo_bit, hi_bit, sc.st));
+  return SVO_OK;
+}
+
 Chunk chunk_of(uint32_t ci, uint32_t chunk_levels, uint32_t depth, uint32_t tri_bits) {
   // chunk ci in Morton order: its code prefix is ci
   uint32_t cxyz[3] = {0, 0, 0};
@@ -1185,13 +1255,15 @@ int DeviceScene::build_mesh(const float* h_vertices, const float* h_normals,
 
   // -- voxels and levels, chunk by chunk; a chunk's leaves are sorted and unique
   DevBuf<uint64_t> cols, d_totals;
+  DevBuf<TriWalk> walks;
+  GB_TRY(walks.alloc(sc, nt));
   GB_TRY(cols.alloc(sc, nt + 1));
   GB_TRY(d_totals.alloc(sc, kMaxLevels));
   GB_TRY(cudaMemsetAsync(d_totals.p, 0, kMaxLevels * sizeof(uint64_t), st));
   std::vector<Levels> parts;
   uint64_t totals[kMaxLevels] = {};
   auto count_columns = [&](const Chunk& ch, uint64_t* n) -> int {
-    column_count_kernel<<<grid_of(nt + 1, 128), 128, 0, st>>>(dV.p, dT.p, nt, depth, ch, cols.p);
+    column_count_kernel<<<grid_of(nt + 1, 128), 128, 0, st>>>(dV.p, dT.p, nt, depth, ch, walks.p, cols.p);
     GB_TRY(cudaGetLastError());
     return sum_counts(sc, cols.p, nt, n);
   };
@@ -1223,10 +1295,15 @@ int DeviceScene::build_mesh(const float* h_vertices, const float* h_normals,
     {
       DevBuf<uint32_t> rec;
       DevBuf<uint64_t> block_hits;
+      DevBuf<uint32_t> block_tri;
       GB_TRY(rec.alloc(sc, columns));
       GB_TRY(block_hits.alloc(sc, col_blocks + 1));
+      GB_TRY(block_tri.alloc(sc, col_blocks + 1));
+      block_triangles_kernel<<<grid_of(col_blocks + 1, 256), 256, 0, st>>>(cols.p, nt, columns, col_blocks,
+                                                                          block_tri.p);
+      GB_TRY(cudaGetLastError());
       column_test_kernel<<<(unsigned)col_blocks, kColThreads, 0, st>>>(
-          dV.p, dT.p, nt, depth, ch, cols.p, columns, rec.p, block_hits.p);
+          walks.p, depth, ch, cols.p, block_tri.p, columns, rec.p, block_hits.p);
       GB_TRY(cudaGetLastError());
       rc = sum_counts(sc, block_hits.p, col_blocks, &P);
       if (rc != SVO_OK) return rc;
@@ -1234,20 +1311,15 @@ int DeviceScene::build_mesh(const float* h_vertices, const float* h_normals,
       if (P == 0) continue;
       GB_TRY(keys.alloc(sc, P));
       column_emit_kernel<<<(unsigned)col_blocks, kColThreads, 0, st>>>(
-          dV.p, dT.p, nt, depth, ch, cols.p, columns, rec.p, block_hits.p, keys.p);
+          walks.p, depth, ch, cols.p, block_tri.p, columns, rec.p, block_hits.p, keys.p);
       GB_TRY(cudaGetLastError());
     }
     // stable, by code alone: the triangles of a code are ascending already
     GB_TRY(keys2.alloc(sc, P));
     cub::DoubleBuffer<uint64_t> kb(keys.p, keys2.p);
     const int lo_bit = (int)tri_bits, hi_bit = (int)(ch.shift + tri_bits);
-    size_t bytes = 0;
-    GB_TRY(cub::DeviceRadixSort::SortKeys(nullptr, bytes, kb, P, lo_bit, hi_bit, st));
-    {
-      DevBuf<uint8_t> tmp;
-      GB_TRY(tmp.alloc(sc, bytes));
-      GB_TRY(cub::DeviceRadixSort::SortKeys(tmp.p, bytes, kb, P, lo_bit, hi_bit, st));
-    }
+    rc = P <= 0x7FFFFFFFull ? sort_keys(sc, kb, (int)P, lo_bit, hi_bit) : sort_keys(sc, kb, P, lo_bit, hi_bit);
+    if (rc != SVO_OK) return rc;
     if (kb.Current() == keys.p)
       keys2.reset();
     else
@@ -1297,6 +1369,7 @@ int DeviceScene::build_mesh(const float* h_vertices, const float* h_normals,
     GB_TRY(cudaGetLastError());
   }
   cols.reset();
+  walks.reset();
   dV.reset();
   dT.reset();
   dFn.reset();
