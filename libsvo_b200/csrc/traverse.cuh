@@ -166,6 +166,17 @@ __device__ __forceinline__ uint32_t shift_in(uint32_t acc, uint32_t side) {
 #endif
 }
 
+// The valid bits of a node's children before child ci.
+__device__ __forceinline__ uint32_t valid_below(uint32_t ci) {
+#if defined(__CUDACC__)
+  uint32_t mask;
+  asm("bmsk.clamp.b32 %0, 8, %1;" : "=r"(mask) : "r"(ci));
+  return mask;
+#else
+  return (0x100u << ci) - 0x100u;
+#endif
+}
+
 // The centre coordinate of the ancestor at the level whose child size is sx2,
 // from a descendant's: as c + 1.5, in [1, 2), the coordinate's fraction is the
 // lattice coordinate in fixed point, so the ancestor's is its leading bits with
@@ -588,9 +599,12 @@ __device__ __forceinline__ Outcome descend(const Fetch& fetch, uint64_t num_node
     const float mx = __fadd_rn(__fmul_rn(r.rx, cx), r.px);
     const float my = __fadd_rn(__fmul_rn(r.ry, cy), r.py);
     const float mz = __fadd_rn(__fmul_rn(r.rz, cz), r.pz);
-    const float ox = __fadd_rn(__fmul_rn(r.rx, __fadd_rn(cx, with_side(bx, sx2))), r.px);
-    const float oy = __fadd_rn(__fmul_rn(r.ry, __fadd_rn(cy, with_side(by, sx2))), r.py);
-    const float oz = __fadd_rn(__fmul_rn(r.rz, __fadd_rn(cz, with_side(bz, sx2))), r.pz);
+    const float fx = __fadd_rn(cx, with_side(bx, sx2));  // the outer faces
+    const float fy = __fadd_rn(cy, with_side(by, sx2));
+    const float fz = __fadd_rn(cz, with_side(bz, sx2));
+    const float ox = __fadd_rn(__fmul_rn(r.rx, fx), r.px);
+    const float oy = __fadd_rn(__fmul_rn(r.ry, fy), r.py);
+    const float oz = __fadd_rn(__fmul_rn(r.rz, fz), r.pz);
     const float tc_max = fminf(fmaxf(mx, ox), fminf(fmaxf(my, oy), fmaxf(mz, oz)));
     const uint32_t ci = shift_in(shift_in(bx >> 31, by), bz);
     const uint32_t masks = nd.y;
@@ -598,7 +612,7 @@ __device__ __forceinline__ Outcome descend(const Fetch& fetch, uint64_t num_node
     if (sh & 0x100u) {
       const float tc_min = fmaxf(fminf(mx, ox), fmaxf(fminf(my, oy), fminf(mz, oz)));
       const float half = __fmul_rn(sx2, 0.5f);
-      const uint32_t below = __popc(masks & ((0x100u << ci) - 0x100u));
+      const uint32_t below = __popc(masks & valid_below(ci));
       const uint32_t child = (kFlat ? 0u : node) + nd.x + below;
       const bool leaf = sh & 1u;
       const bool lod = kFlat ? (__fmul_rn(r.tsr, tc_max) > sx2)
@@ -638,9 +652,12 @@ __device__ __forceinline__ Outcome descend(const Fetch& fetch, uint64_t num_node
       if (node <= last_node) nd = fetch(node);
       tmin = tc_min;
       tmax = tc_max;
-      cx = __fadd_rn(with_side(bx, half), cx);
-      cy = __fadd_rn(with_side(by, half), cy);
-      cz = __fadd_rn(with_side(bz, half), cz);
+      // the child's centre, between its faces (exact): an add and a multiply, not
+      // a select and an add, as the selects' pipe is the busier one (a 3840x2160
+      // frame 770 -> 726 us, 48 batched views 1010 -> 960 us with the mask below)
+      cx = __fmul_rn(__fadd_rn(cx, fx), 0.5f);
+      cy = __fmul_rn(__fadd_rn(cy, fy), 0.5f);
+      cz = __fmul_rn(__fadd_rn(cz, fz), 0.5f);
       sx2 = half;
     } else {
       tmin = tc_max;  // advance to the next sibling
