@@ -290,10 +290,11 @@ template <bool kFlat>
 __global__ void __launch_bounds__(kThreads) trace_rays_kernel(
     const uint2* __restrict__ nodes, uint64_t num_nodes, const float* __restrict__ origins,
     const float* __restrict__ dirs, uint64_t n, float tsr, int S, svo_hit* __restrict__ hits,
-    svo_stats* __restrict__ stats) {
+    svo_stats* __restrict__ stats, uint32_t rays) {
   extern __shared__ uint2 stack_smem[];
-  const uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-  if (i >= n) return;
+  const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const uint64_t i = ((uint64_t)blockIdx.x * (kThreads / 32) + warp) * rays + lane;
+  if (lane >= rays || i >= n) return;
   const float o[3] = {origins[3 * i], origins[3 * i + 1], origins[3 * i + 2]};
   const RayHit h = cast_ray<kFlat>(GlobalFetch{nodes}, num_nodes, o, dirs[3 * i], dirs[3 * i + 1],
                                    dirs[3 * i + 2], tsr, S, stack_smem + threadIdx.x, kThreads);
@@ -577,7 +578,10 @@ int launch_trace_rays(const svo_node* nodes, uint64_t num_nodes, const float* or
                       const float* dirs, uint64_t n, float tsr, const svo_trace_cfg& cfg,
                       svo_hit* hits, svo_stats* stats, cudaStream_t stream) {
   if (n == 0) return SVO_OK;
-  const uint64_t blocks = (n + kThreads - 1) / kThreads;
+  // (us, 32 / 16 / 8 lanes: 1,000 rays over a depth-10 icosphere 50.5 / 47.8 /
+  // 44.4, 8,000 62.0 / 60.1 / 56.7, 30,000 71.7 / 68.9 / 72.5, 50,000 78 / 85 / 94)
+  const uint32_t rays = n <= (1u << 15) ? rays_per_warp(n) : 32u;
+  const uint64_t per_block = kThreads / 32 * rays, blocks = (n + per_block - 1) / per_block;
   if (blocks > 0x7FFFFFFFull) return SVO_ERR_RANGE;
   const int S = cfg.stack_size;
   const size_t smem = render_smem_bytes(S);
@@ -589,10 +593,10 @@ int launch_trace_rays(const svo_node* nodes, uint64_t num_nodes, const float* or
   }
   if (cfg.traversal == SVO_TRAVERSAL_FLAT)
     trace_rays_kernel<true><<<(unsigned)blocks, kThreads, smem, stream>>>(
-        n2, num_nodes, origins, dirs, n, tsr, S, hits, stats);
+        n2, num_nodes, origins, dirs, n, tsr, S, hits, stats, rays);
   else
     trace_rays_kernel<false><<<(unsigned)blocks, kThreads, smem, stream>>>(
-        n2, num_nodes, origins, dirs, n, tsr, S, hits, stats);
+        n2, num_nodes, origins, dirs, n, tsr, S, hits, stats, rays);
   return cudaGetLastError() == cudaSuccess ? SVO_OK : SVO_ERR_CUDA;
 }
 

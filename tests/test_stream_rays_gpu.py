@@ -55,6 +55,18 @@ def test_rays_match_the_oracle(cuda, n, flat):
     assert int(stats[0]) == int((want["flags"] == L.HITFLAG_CAPPED).sum())
 
 
+@pytest.mark.parametrize("n", [1, 7, 9, 31, 33, (1 << 14) - 1, 1 << 14, (1 << 14) + 1, 1 << 15, (1 << 15) + 1])
+def test_few_rays_match_the_oracle(cuda, n):
+    """Counts cast with 8, 16 and 32 rays a warp."""
+    import torch
+
+    nodes, o, d = make(n % 5, n)
+    want, _ = oracle.cast_rays(nodes, o, d, 0.001)
+    hits, _ = launch(torch, nodes, o, d, 0.001, L.trace_cfg())
+    torch.cuda.synchronize()
+    assert same(hits, want)
+
+
 def test_every_ray_misses(cuda):
     import torch
 
