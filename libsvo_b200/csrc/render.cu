@@ -37,17 +37,19 @@ constexpr int kThreads = kBlockW * kBlockH;
 // The estimate is a chain of dependent node reads per ray, so its time grows
 // with the cap on its passes.  A ray at the cap counts for what its progress
 // says about the rest of its way through the root box, so that the long blocks
-// are told from one another: 1920x1080 icosphere frames took 226 us with 48
-// passes so extended, 255 us with the 48 counted as they are, 243 us with 32,
-// 233 us with 64 passes, 235 us with one sample a block, and 256 us in raster
-// order.  Sixteen of a warp's lanes cast samples: with all 32 the paths of more
-// cells diverge in each of a warp's passes (248 against 241 us).
+// are told from one another (with the capped counts as they are, the 1920x1080
+// icosphere took 255 us against 226 us, as long as in raster order).  The cap
+// (us, 32 / 40 / 48 / 56 passes): 1920x1080 icospheres 236 / 224 / 229 / 243 and
+// 207 / 201 / 211 / 223, 2560x1440 372 / 353 / 357 / 361, a 1920x1080 terrain 202 /
+// 205 / 207 / 209.  One sample a block: 235 us against 226.  Sixteen of a warp's
+// lanes cast samples: with all 32 the paths of more cells diverge in each of a
+// warp's passes (248 against 241 us, 2560x1440 362 against 357).
 //
 // The line: the tail that the order removes is a few long rays, so it does not
 // grow with the frame, while the estimate is a share of it.  At 1280x720 the two
-// are equal (107 us); at 3840x2160 an icosphere takes 761 us either way and a
-// terrain 857 us ordered, 801 us in raster order.
-constexpr uint32_t kCostCap = 48;  // passes of an estimate ray
+// orders are equal (102 us); at 3840x2160 an icosphere took 761 us either way and
+// a terrain 857 us ordered, 801 us in raster order.
+constexpr uint32_t kCostCap = 40;  // passes of an estimate ray
 constexpr uint32_t kCostBuckets = 49;
 constexpr uint32_t kCostTop = kCostBuckets - 1;
 constexpr uint32_t kCostSamples = kBlockW / 8;  // one ray per 8x8 cell of a block
