@@ -155,7 +155,9 @@ int svo_scene_build_mesh(const float* h_vertices, uint64_t num_vertices,
  * (src/TreeletBuilderFromFaces.cpp:189-365, src/TreeletBuildManager.cpp:
  * 150-258) and the insertion loop (src/TreeletMemoryManager.cpp:518-545).
  * The slot size is always the automatic one (largest treelet + 8 nodes).
- * Blocks until the pool is built; scratch memory is freed before returning. */
+ * Blocks until the pool is built.  Up to 1 GB of scratch, and up to 1 GB of
+ * destroyed scenes' pools, is kept on the device for the next build; all of it
+ * is given back when the last scene is destroyed. */
 typedef struct svo_device_scene svo_device_scene;
 int svo_device_scene_build_mesh(const float* h_vertices, uint64_t num_vertices,
                                 const uint32_t* h_triangles, uint64_t num_triangles,
@@ -393,9 +395,10 @@ int svo_trace_rays(const svo_node* d_nodes, uint64_t num_nodes, const float* d_o
  * Counters accumulate in the manager (read with svo_mm_sync). */
 int svo_mm_render(svo_mm* mm, const svo_frame_params* params, const svo_trace_cfg* cfg,
                   uint32_t* d_rgba, svo_hit* d_hits, void* stream);
-/* Blocking frame into host memory: launch, copy the W*H RGBA8 image to
+/* Blocking frame into host memory: launch, bring the W*H RGBA8 image to
  * h_rgba, wait.  This is the reference's blocking enqueueKernel plus the
- * image read back. */
+ * image read back.  A page-locked, mapped h_rgba is written by the cast
+ * itself, any other is copied to. */
 int svo_mm_render_host(svo_mm* mm, const svo_frame_params* params, const svo_trace_cfg* cfg,
                        uint32_t* h_rgba, void* stream);
 /* Shadow rays: one per primary hit, toward a directional light. */

@@ -1031,7 +1031,7 @@ void free_kept_pools(Kept& k) {  // k.mu is held
 }
 
 // Scene pool memory: a kept block of at most a quarter more than asked for, else
-// new memory (after what is kept has been given up, if need be).
+// new memory (after what is kept has been given back, if need be).
 cudaError_t pool_alloc(int dev, uint64_t bytes, void** out, uint64_t* got) {
   Kept& k = g_kept[dev];
   std::lock_guard<std::mutex> lock(k.mu);
@@ -1202,6 +1202,15 @@ Chunk chunk_of(uint32_t ci, uint32_t chunk_levels, uint32_t depth, uint32_t tri_
 }
 
 }  // namespace
+
+void give_back_kept_memory() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return;
+  Kept& k = g_kept[dev];
+  std::lock_guard<std::mutex> lock(k.mu);
+  free_kept_pools(k);
+  if (k.scratch) cudaMemPoolTrimTo(k.scratch, 0);
+}
 
 int DeviceScene::build_mesh(const float* h_vertices, const float* h_normals,
                             const float* h_colors, uint64_t nv, const uint32_t* h_triangles,

@@ -10,6 +10,7 @@
 #include "analysis.h"
 #include "errors.h"
 #include "feedback.h"
+#include "gpu_builder.h"
 #include "render.h"
 #include "upload.h"
 
@@ -430,8 +431,14 @@ int TreeletMemoryManagerCuda::init_device_buffer() {
   int rc = init_transfer();
   if (rc != SVO_OK) return rc;
   const uint64_t n = incore_nodes();
-  if (cudaMalloc(&d_nodes_, n * sizeof(svo_node)) != cudaSuccess ||
-      cudaMalloc(&d_attribs_, n * sizeof(svo_attrib)) != cudaSuccess) {
+  auto alloc = [&](void** p, uint64_t bytes) {
+    if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+    cudaGetLastError();
+    give_back_kept_memory();
+    return cudaMalloc(p, bytes) == cudaSuccess;
+  };
+  if (!alloc((void**)&d_nodes_, n * sizeof(svo_node)) ||
+      !alloc((void**)&d_attribs_, n * sizeof(svo_attrib))) {
     cudaGetLastError();
     cudaFree(d_nodes_);
     cudaFree(d_attribs_);

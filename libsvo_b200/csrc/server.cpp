@@ -46,6 +46,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "gpu_builder.h"
 #include "../../include/libsvo_b200.h"
 #include "errors.h"
 #include "memory_manager.h"
@@ -62,7 +63,11 @@ class DevicePool {
   int init(uint64_t bytes) {
     size_ = bytes & ~255ull;
     if (size_ == 0) return SVO_ERR_RANGE;
-    SVO_CUDA_TRY(cudaMalloc(&base_, size_));
+    if (cudaMalloc(&base_, size_) != cudaSuccess) {
+      cudaGetLastError();
+      svo::give_back_kept_memory();
+      SVO_CUDA_TRY(cudaMalloc(&base_, size_));
+    }
     free_.clear();
     free_[0] = size_;
     return SVO_OK;
