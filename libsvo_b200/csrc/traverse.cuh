@@ -228,6 +228,16 @@ __device__ __forceinline__ Pair pair_fma(Pair a, Pair b, Pair c) {
 __device__ __forceinline__ Pair pair_mul_add(Pair a, Pair b, Pair c) {
   return pair_fma(pair_mul(a, b), kPairOfOnes, c);
 }
+// ancestor_center of both halves
+__device__ __forceinline__ Pair ancestor_centers(Pair c, uint32_t one, uint32_t keep) {
+  Pair q;
+  asm("add.rz.f32x2 %0, %1, %2;" : "=l"(q) : "l"(c), "l"(0x3fc000003fc00000ull));
+  float a, b;
+  halves(q, a, b);
+  return pair_add(pair_of(__uint_as_float((__float_as_uint(a) & keep) | one),
+                          __uint_as_float((__float_as_uint(b) & keep) | one)),
+                  0xbfc00000bfc00000ull);
+}
 // c - a: a times -1 is exact
 __device__ __forceinline__ Pair pair_sub_from(Pair a, Pair c) {
   return pair_fma(a, 0xbf800000bf800000ull, c);
@@ -241,6 +251,9 @@ inline void halves(Pair v, float& a, float& b) { a = v.a, b = v.b; }
 inline Pair pair_mul(Pair x, Pair y) { return Pair{x.a * y.a, x.b * y.b}; }
 inline Pair pair_add(Pair x, Pair y) { return Pair{x.a + y.a, x.b + y.b}; }
 inline Pair pair_mul_add(Pair x, Pair y, Pair z) { return pair_add(pair_mul(x, y), z); }
+inline Pair ancestor_centers(Pair c, uint32_t one, uint32_t keep) {
+  return Pair{ancestor_center(c.a, one, keep), ancestor_center(c.b, one, keep)};
+}
 // (the host's `above` compares; 1 stands for a negative difference)
 inline Pair pair_sub_from(Pair x, Pair z) { return Pair{x.a > z.a ? -1.0f : 1.0f, x.b > z.b ? -1.0f : 1.0f}; }
 #endif
@@ -759,8 +772,12 @@ __device__ __forceinline__ Outcome descend(const Fetch& fetch, uint64_t num_node
       nd = fetch(node);
       const uint32_t one = kOne | bit;
       const uint32_t keep = 0u - 2u * bit;
-      cx = ancestor_center(cx, one, keep);
-      cy = ancestor_center(cy, one, keep);
+      if (kPairs) {
+        halves(ancestor_centers(pair_of(cx, cy), one, keep), cx, cy);
+      } else {
+        cx = ancestor_center(cx, one, keep);
+        cy = ancestor_center(cy, one, keep);
+      }
       cz = ancestor_center(cz, one, keep);
       const float size = __fadd_rn(__uint_as_float(one), -1.0f);
       pops += (__float_as_uint(size) - __float_as_uint(sx2)) >> 23;
