@@ -166,6 +166,17 @@ __device__ __forceinline__ uint32_t shift_in(uint32_t acc, uint32_t side) {
 #endif
 }
 
+// The lanes that run a piece of code together at this moment.  Only a hint: CUDA
+// does not promise when lanes that parted come together again, so nothing may
+// wait for this number to change.  (A host caller is one lane.)
+__device__ __forceinline__ int lanes_together() {
+#if defined(__CUDACC__)
+  return __popc(__activemask());
+#else
+  return 1;
+#endif
+}
+
 // The valid bits of a node's children before child ci.
 __device__ __forceinline__ uint32_t valid_below(uint32_t ci) {
 #if defined(__CUDACC__)
@@ -585,6 +596,11 @@ __device__ __forceinline__ void descend_general(const Fetch& fetch, uint64_t num
 //
 // With kYield the ray goes on from `w` and the loop also ends (kYields, with the
 // ray in `w` again) once no more than `keep` lanes of the warp are still in it.
+// It is asked behind a pass, never before the first one: every call moves its ray
+// on by a pass or ends it, however few lanes run together, so a caller that calls
+// again until its rays have ended comes to an end.  (A million rays without order
+// 320 us when asked ahead of each pass, the first one too; 315 us behind it; 331 us
+// ahead of each but the first.)
 constexpr uint32_t kProgressPasses = 32;
 enum Outcome { kEnded, kLeaves, kYields };
 
@@ -655,12 +671,6 @@ __device__ __forceinline__ Outcome descend(const Fetch& fetch, uint64_t num_node
       seen = tmin;
       check_at = check_at + kProgressPasses < limit ? check_at + kProgressPasses : limit;
     }
-#if defined(__CUDACC__)
-    if (kYield && __popc(__activemask()) <= keep) {
-      w = Descent{node, tmin, tmax, cx, cy, cz, sx2, nd, passes, pops, check_at, seen, open, sp};
-      return kYields;
-    }
-#endif
     ++passes;
     // childEntryPoint = (o + (tMin + eps) d) - centre and its sign test
     const float te = __fadd_rn(tmin, eps);
@@ -782,6 +792,10 @@ __device__ __forceinline__ Outcome descend(const Fetch& fetch, uint64_t num_node
       const float size = __fadd_rn(__uint_as_float(one), -1.0f);
       pops += (__float_as_uint(size) - __float_as_uint(sx2)) >> 23;
       sx2 = size;
+    }
+    if (kYield && lanes_together() <= keep) {
+      w = Descent{node, tmin, tmax, cx, cy, cz, sx2, nd, passes, pops, check_at, seen, open, sp};
+      return kYields;
     }
   }
   st = RayState{node, tmin, tmax, cx, cy, cz, sx2, passes + pops, passes};
