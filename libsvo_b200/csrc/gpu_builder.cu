@@ -54,13 +54,13 @@
 
 #include <algorithm>
 #include <cstdint>
-#include <mutex>
 #include <utility>
 #include <vector>
 
 #include "../../include/libsvo_b200.h"
 #include "errors.h"
 #include "gpu_builder.h"
+#include "kept_memory.h"
 
 namespace svo {
 
@@ -978,117 +978,6 @@ __global__ void __launch_bounds__(256) cut_kernel(LevelPtrs L, CutParams cp,
 
 // Columns of one chunk: 2 GB of records, about 5 GB of keys.
 constexpr uint64_t kMaxColumns = 1ull << 29;
-constexpr int kMaxDevices = 64;
-
-// What builds keep between them, per device.  Scratch: a stream-ordered memory
-// pool that holds on to at most kScratchKeep (allocating and freeing device
-// memory took 50 of the 70 ms of a depth-11 build).  Pools of destroyed scenes:
-// at most kPoolKeep, plain cudaMalloc memory like every scene's pool, for the
-// next scene of about that size.  Both go back to the device when the last
-// scene is destroyed.
-constexpr uint64_t kScratchKeep = 1ull << 30;
-constexpr uint64_t kPoolKeep = 1ull << 30;
-struct KeptPool {
-  void* p;
-  uint64_t bytes;
-};
-struct Kept {
-  std::mutex mu;
-  cudaMemPool_t scratch = nullptr;
-  std::vector<KeptPool> pools;
-  uint64_t pool_bytes = 0;
-  uint64_t users = 0;  // scenes alive and builds running
-};
-Kept g_kept[kMaxDevices];
-
-cudaError_t scratch_pool(int dev, cudaMemPool_t* out) {
-  Kept& k = g_kept[dev];
-  std::lock_guard<std::mutex> lock(k.mu);
-  if (!k.scratch) {
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    cudaMemPool_t pool = nullptr;
-    cudaError_t e = cudaMemPoolCreate(&pool, &props);
-    if (e != cudaSuccess) return e;
-    uint64_t keep = kScratchKeep;
-    e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    if (e != cudaSuccess) {
-      cudaMemPoolDestroy(pool);
-      return e;
-    }
-    k.scratch = pool;
-  }
-  *out = k.scratch;
-  return cudaSuccess;
-}
-
-void free_kept_pools(Kept& k) {  // k.mu is held
-  for (const KeptPool& p : k.pools) cudaFree(p.p);
-  k.pools.clear();
-  k.pool_bytes = 0;
-}
-
-// Scene pool memory: a kept block of at most a quarter more than asked for, else
-// new memory (after what is kept has been given back, if need be).
-cudaError_t pool_alloc(int dev, uint64_t bytes, void** out, uint64_t* got) {
-  Kept& k = g_kept[dev];
-  std::lock_guard<std::mutex> lock(k.mu);
-  size_t best = k.pools.size();
-  for (size_t i = 0; i < k.pools.size(); ++i)
-    if (k.pools[i].bytes >= bytes && k.pools[i].bytes - bytes <= bytes / 4 &&
-        (best == k.pools.size() || k.pools[i].bytes < k.pools[best].bytes))
-      best = i;
-  if (best < k.pools.size()) {
-    *out = k.pools[best].p;
-    *got = k.pools[best].bytes;
-    k.pool_bytes -= *got;
-    k.pools.erase(k.pools.begin() + (ptrdiff_t)best);
-    return cudaSuccess;
-  }
-  *got = bytes;
-  cudaError_t e = cudaMalloc(out, bytes);
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    free_kept_pools(k);
-    if (k.scratch) cudaMemPoolTrimTo(k.scratch, 0);
-    e = cudaMalloc(out, bytes);
-  }
-  return e;
-}
-
-// The scene's pool memory, once nothing reads it any more (cudaFree waits for
-// the device; a block that is kept must wait as well).
-void pool_free(int dev, void* p, uint64_t bytes) {
-  if (!p) return;
-  Kept& k = g_kept[dev];
-  std::lock_guard<std::mutex> lock(k.mu);
-  if (k.users > 1 && k.pool_bytes + bytes <= kPoolKeep && cudaDeviceSynchronize() == cudaSuccess) {
-    try {
-      k.pools.push_back({p, bytes});
-      k.pool_bytes += bytes;
-      return;
-    } catch (...) {
-    }
-  }
-  cudaFree(p);
-}
-
-void user_begins(int dev) {
-  std::lock_guard<std::mutex> lock(g_kept[dev].mu);
-  ++g_kept[dev].users;
-}
-
-void user_ends(int dev) {
-  Kept& k = g_kept[dev];
-  std::lock_guard<std::mutex> lock(k.mu);
-  if (--k.users) return;
-  cudaDeviceSynchronize();  // scratch still in use by a failed build
-  free_kept_pools(k);
-  if (k.scratch) cudaMemPoolTrimTo(k.scratch, 0);
-}
-
 // Scratch of one build, ordered on its stream.
 struct Scratch {
   cudaMemPool_t pool = nullptr;
@@ -1202,15 +1091,6 @@ Chunk chunk_of(uint32_t ci, uint32_t chunk_levels, uint32_t depth, uint32_t tri_
 }
 
 }  // namespace
-
-void give_back_kept_memory() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return;
-  Kept& k = g_kept[dev];
-  std::lock_guard<std::mutex> lock(k.mu);
-  free_kept_pools(k);
-  if (k.scratch) cudaMemPoolTrimTo(k.scratch, 0);
-}
 
 int DeviceScene::build_mesh(const float* h_vertices, const float* h_normals,
                             const float* h_colors, uint64_t nv, const uint32_t* h_triangles,

@@ -39,8 +39,4 @@ struct DeviceScene {
   uint64_t pool_bytes_ = 0;
 };
 
-// Gives the memory that builds keep on the current device back to it; called
-// where a large allocation of the library's fails, before it is tried again.
-void give_back_kept_memory();
-
 }  // namespace svo

@@ -10,7 +10,7 @@
 #include "analysis.h"
 #include "errors.h"
 #include "feedback.h"
-#include "gpu_builder.h"
+#include "kept_memory.h"
 #include "render.h"
 #include "upload.h"
 

@@ -46,9 +46,9 @@
 #include <unordered_map>
 #include <vector>
 
-#include "gpu_builder.h"
 #include "../../include/libsvo_b200.h"
 #include "errors.h"
+#include "kept_memory.h"
 #include "memory_manager.h"
 #include "render.h"
 #include "scene.h"

@@ -1,0 +1,77 @@
+"""The device memory that builds keep (libsvo_b200/csrc/kept_memory.cpp), over a
+device that the host pretends to be (tests/hostsim/kept_memory_host.cpp): who gets
+it back, when, and who waits for whom."""
+import ctypes
+import os
+import subprocess
+from pathlib import Path
+
+import pytest
+
+HERE = Path(__file__).resolve().parent / "hostsim"
+SOURCE = HERE.parent.parent / "libsvo_b200" / "csrc" / "kept_memory.cpp"
+CUDA_HOME = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
+GB = 1 << 30
+
+
+def load(path, tag):
+    """The pretended device with the given source, in a library of its own."""
+    lib = HERE / "_build" / f"libkept_memory_{tag}.so"
+    lib.parent.mkdir(parents=True, exist_ok=True)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-pthread", "-Wl,-Bsymbolic", f"-I{CUDA_HOME / 'include'}",
+                    f'-DKEPT_MEMORY_SOURCE="{path}"', "-o", str(lib), str(HERE / "kept_memory_host.cpp")], check=True)
+    lib = ctypes.CDLL(str(lib))
+    u64 = ctypes.c_uint64
+    lib.fake_device.argtypes = [u64]
+    lib.fake_used.restype = lib.fake_plain.restype = u64
+    lib.block_alloc.argtypes, lib.block_alloc.restype = [u64, ctypes.POINTER(u64)], u64
+    lib.block_free.argtypes = [u64, u64]
+    return lib
+
+
+@pytest.fixture
+def device(request):
+    lib = load(SOURCE, request.node.name.replace("[", "_").replace("]", ""))
+    lib.fake_device(8 * GB)
+    return lib
+
+
+def block(device, size):
+    got = ctypes.c_uint64()
+    return device.block_alloc(size, ctypes.byref(got)), got.value
+
+
+@pytest.mark.parametrize("end", [0, 1])
+@pytest.mark.parametrize("other", [0, 1])
+def test_a_build_goes_on_while_a_scene_ends(device, end, other):
+    """A scene's end waits for the device; other threads do not wait for it."""
+    assert device.runs_beside(end, other) == 1
+    assert device.fake_used() == 0
+
+
+def test_blocks_are_kept_and_given_back(device):
+    device.begin()
+    device.begin()
+    p, got = block(device, GB // 2)
+    device.block_free(p, got)
+    assert device.fake_plain() == GB // 2  # kept
+    assert block(device, GB // 2 - 100)[0] == p  # and used again, if it fits
+    q, got_q = block(device, GB // 4)
+    assert q != p and got_q == GB // 4
+    device.block_free(p, got)
+    device.block_free(q, got_q)
+    assert device.fake_plain() == GB // 2 + GB // 4
+    big, got_big = block(device, 8 * GB - GB // 4)  # all that is kept comes back for it
+    assert big and got_big == 8 * GB - GB // 4
+    device.block_free(big, got_big)  # too large to keep
+    device.end()
+    device.end()
+    assert device.fake_used() == 0
+
+
+def test_nothing_is_kept_for_a_lone_scene(device):
+    device.begin()
+    p, got = block(device, GB // 8)
+    device.block_free(p, got)
+    device.end()
+    assert device.fake_used() == 0
