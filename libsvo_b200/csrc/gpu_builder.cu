@@ -1009,10 +1009,7 @@ struct DevBuf {
   cudaError_t alloc(const Scratch& s, size_t count) {
     reset();
     st = s.st;
-    const cudaError_t e =
-        cudaMallocFromPoolAsync((void**)&p, (count ? count : 1) * sizeof(T), s.pool, s.st);
-    if (e != cudaSuccess) p = nullptr;
-    return e;
+    return scratch_alloc(s.pool, (count ? count : 1) * sizeof(T), s.st, (void**)&p);
   }
 };
 

@@ -91,6 +91,24 @@ cudaError_t scratch_pool(int dev, cudaMemPool_t* out) {
   return cudaSuccess;
 }
 
+cudaError_t scratch_alloc(cudaMemPool_t pool, uint64_t bytes, cudaStream_t stream, void** out) {
+  cudaError_t e = cudaMallocFromPoolAsync(out, bytes, pool, stream);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    // what the stream has still to free goes back only once it has come to it
+    e = cudaStreamSynchronize(stream);
+    if (e == cudaSuccess) {
+      give_back_kept_memory();
+      e = cudaMallocFromPoolAsync(out, bytes, pool, stream);
+    }
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // the caller has it; the next launch's check must not
+    *out = nullptr;
+  }
+  return e;
+}
+
 cudaError_t pool_alloc(int dev, uint64_t bytes, void** out, uint64_t* got) {
   Kept& k = g_kept[dev];
   {
@@ -115,6 +133,7 @@ cudaError_t pool_alloc(int dev, uint64_t bytes, void** out, uint64_t* got) {
     give_back(k);
     e = cudaMalloc(out, bytes);
   }
+  if (e != cudaSuccess) cudaGetLastError();
   return e;
 }
 

@@ -26,6 +26,10 @@ void user_ends(int dev);
 // The device's pool of scratch memory.
 cudaError_t scratch_pool(int dev, cudaMemPool_t* out);
 
+// Scratch memory from it, in the stream's order; on the current device.  Where it
+// does not fit, what is kept is given back and it is tried once more.
+cudaError_t scratch_alloc(cudaMemPool_t pool, uint64_t bytes, cudaStream_t stream, void** out);
+
 // Scene pool memory: a kept block of at most a quarter more than asked for, else
 // new memory.  *got is the block's size.
 cudaError_t pool_alloc(int dev, uint64_t bytes, void** out, uint64_t* got);

@@ -173,6 +173,13 @@ uint64_t block_alloc(uint64_t bytes, uint64_t* got) {
   return svo::pool_alloc(0, bytes, &p, got) == cudaSuccess ? (uint64_t)p : 0u;
 }
 void block_free(uint64_t p, uint64_t bytes) { svo::pool_free(0, (void*)p, bytes); }
+uint64_t scratch(uint64_t bytes) {
+  cudaMemPool_t pool;
+  void* p = nullptr;
+  if (svo::scratch_pool(0, &pool) != cudaSuccess) return 0;
+  return svo::scratch_alloc(pool, bytes, nullptr, &p) == cudaSuccess ? (uint64_t)p : 0u;
+}
+void scratch_free(uint64_t p) { cudaFreeAsync((void*)p, nullptr); }
 void begin() { svo::user_begins(0); }
 void end() { svo::user_ends(0); }
 

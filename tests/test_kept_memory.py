@@ -26,6 +26,8 @@ def load(path, tag):
     lib.fake_used.restype = lib.fake_plain.restype = u64
     lib.block_alloc.argtypes, lib.block_alloc.restype = [u64, ctypes.POINTER(u64)], u64
     lib.block_free.argtypes = [u64, u64]
+    lib.scratch.argtypes, lib.scratch.restype = [u64], u64
+    lib.scratch_free.argtypes = [u64]
     return lib
 
 
@@ -73,5 +75,26 @@ def test_nothing_is_kept_for_a_lone_scene(device):
     device.begin()
     p, got = block(device, GB // 8)
     device.block_free(p, got)
+    device.end()
+    assert device.fake_used() == 0
+
+
+def test_scratch_takes_what_is_kept(device):
+    """A build whose keys fit only without a destroyed scene's pool, or without the
+    scratch that it has itself freed, gets them."""
+    device.begin()
+    device.begin()
+    p, got = block(device, GB)
+    device.block_free(p, got)
+    assert device.fake_used() == GB
+    a = device.scratch(7 * GB + GB // 2)
+    assert a and device.fake_used() == 7 * GB + GB // 2
+    device.scratch_free(a)  # the stream has not come to it
+    b = device.scratch(7 * GB + 3 * (GB // 4))
+    assert b and device.fake_used() == 7 * GB + 3 * (GB // 4)
+    device.scratch_free(b)
+    assert not device.scratch(8 * GB + 1)  # more than there is
+    assert device.fake_last_error() == 0  # nothing left for the next call to find
+    device.end()
     device.end()
     assert device.fake_used() == 0
