@@ -156,8 +156,9 @@ int svo_scene_build_mesh(const float* h_vertices, uint64_t num_vertices,
  * 150-258) and the insertion loop (src/TreeletMemoryManager.cpp:518-545).
  * The slot size is always the automatic one (largest treelet + 8 nodes).
  * Blocks until the pool is built.  Up to 1 GB of scratch, and up to 1 GB of
- * destroyed scenes' pools, is kept on the device for the next build; all of it
- * is given back when the last scene is destroyed. */
+ * destroyed scenes' pools, is kept on the device for the next build while a
+ * scene is alive; all of it is given back when the last one is destroyed, or
+ * where an allocation of the library's does not fit. */
 typedef struct svo_device_scene svo_device_scene;
 int svo_device_scene_build_mesh(const float* h_vertices, uint64_t num_vertices,
                                 const uint32_t* h_triangles, uint64_t num_triangles,

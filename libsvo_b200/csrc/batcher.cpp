@@ -7,6 +7,7 @@
 #include "../../include/libsvo_b200.h"
 #include "batch.h"
 #include "errors.h"
+#include "kept_memory.h"
 
 namespace svo {
 
@@ -159,10 +160,9 @@ int svo_batcher_create(uint32_t max_views, uint32_t max_octrees, svo_batcher** o
   b->max_views = max_views;
   b->max_octrees = max_octrees;
   int rc = SVO_OK;
-  if (rc == SVO_OK) rc = svo::cuda_status(cudaMalloc(&b->d_views, max_views * sizeof(svo::BatchView)));
-  if (rc == SVO_OK)
-    rc = svo::cuda_status(cudaMalloc(&b->d_octrees, max_octrees * sizeof(svo::BatchOctree)));
-  if (rc == SVO_OK) rc = svo::cuda_status(cudaMalloc(&b->d_counter, sizeof(unsigned long long)));
+  if (rc == SVO_OK) rc = svo::cuda_status(svo::device_array(&b->d_views, max_views));
+  if (rc == SVO_OK) rc = svo::cuda_status(svo::device_array(&b->d_octrees, max_octrees));
+  if (rc == SVO_OK) rc = svo::cuda_status(svo::device_array(&b->d_counter, 1));
   if (rc == SVO_OK)
     rc = svo::cuda_status(cudaMallocHost(&b->h_views, max_views * sizeof(svo::BatchView)));
   if (rc == SVO_OK)

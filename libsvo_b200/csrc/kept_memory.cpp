@@ -38,14 +38,6 @@ void give_back(const std::vector<KeptPool>& pools, cudaMemPool_t scratch) {
   if (scratch) cudaMemPoolTrimTo(scratch, 0);
 }
 
-void give_back(Kept& k) {
-  std::unique_lock<std::mutex> lock(k.mu);
-  const std::vector<KeptPool> pools = take_pools(k);
-  cudaMemPool_t scratch = k.scratch;
-  lock.unlock();
-  give_back(pools, scratch);
-}
-
 }  // namespace
 
 void user_begins(int dev) {
@@ -127,14 +119,7 @@ cudaError_t pool_alloc(int dev, uint64_t bytes, void** out, uint64_t* got) {
     }
   }
   *got = bytes;
-  cudaError_t e = cudaMalloc(out, bytes);
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    give_back(k);
-    e = cudaMalloc(out, bytes);
-  }
-  if (e != cudaSuccess) cudaGetLastError();
-  return e;
+  return device_alloc(out, bytes);
 }
 
 void pool_free(int dev, void* p, uint64_t bytes) {
@@ -162,7 +147,26 @@ void pool_free(int dev, void* p, uint64_t bytes) {
 void give_back_kept_memory() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return;
-  give_back(g_kept[dev]);
+  Kept& k = g_kept[dev];
+  std::unique_lock<std::mutex> lock(k.mu);
+  const std::vector<KeptPool> pools = take_pools(k);
+  cudaMemPool_t scratch = k.scratch;
+  lock.unlock();
+  give_back(pools, scratch);
+}
+
+cudaError_t device_alloc(void** out, uint64_t bytes) {
+  cudaError_t e = cudaMalloc(out, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    give_back_kept_memory();
+    e = cudaMalloc(out, bytes);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    *out = nullptr;
+  }
+  return e;
 }
 
 }  // namespace svo

@@ -36,8 +36,15 @@ cudaError_t pool_alloc(int dev, uint64_t bytes, void** out, uint64_t* got);
 // ... and its end, from a user of the device; waits until nothing reads it.
 void pool_free(int dev, void* p, uint64_t bytes);
 
-// Gives what is kept on the current device back to it; called where a large
-// allocation of the library's fails, before it is tried again.
+// Gives what is kept on the current device back to it.
 void give_back_kept_memory();
+
+// Every other allocation of device memory in the library: on the current device;
+// where it does not fit, what builds keep is given back and it is tried once more.
+cudaError_t device_alloc(void** out, uint64_t bytes);
+template <class T>
+cudaError_t device_array(T** out, uint64_t count) {
+  return device_alloc((void**)out, count * sizeof(T));
+}
 
 }  // namespace svo

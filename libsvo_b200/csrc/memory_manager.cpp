@@ -399,7 +399,7 @@ int TreeletMemoryManagerCuda::init_transfer() {
     SVO_CUDA_TRY(cudaEventCreateWithFlags(&stage_evt_[i], cudaEventDisableTiming));
     SVO_CUDA_TRY(cudaMallocHost(&stage_[i], kStageBytes));
   }
-  SVO_CUDA_TRY(cudaMalloc(&d_stats_, sizeof(svo_stats)));
+  SVO_CUDA_TRY(device_array(&d_stats_, 1));
   SVO_CUDA_TRY(cudaMemsetAsync(d_stats_, 0, sizeof(svo_stats), copy_stream_));
   return SVO_OK;
 }
@@ -431,15 +431,7 @@ int TreeletMemoryManagerCuda::init_device_buffer() {
   int rc = init_transfer();
   if (rc != SVO_OK) return rc;
   const uint64_t n = incore_nodes();
-  auto alloc = [&](void** p, uint64_t bytes) {
-    if (cudaMalloc(p, bytes) == cudaSuccess) return true;
-    cudaGetLastError();
-    give_back_kept_memory();
-    return cudaMalloc(p, bytes) == cudaSuccess;
-  };
-  if (!alloc((void**)&d_nodes_, n * sizeof(svo_node)) ||
-      !alloc((void**)&d_attribs_, n * sizeof(svo_attrib))) {
-    cudaGetLastError();
+  if (device_array(&d_nodes_, n) != cudaSuccess || device_array(&d_attribs_, n) != cudaSuccess) {
     cudaFree(d_nodes_);
     cudaFree(d_attribs_);
     d_nodes_ = nullptr;
@@ -590,9 +582,9 @@ int TreeletMemoryManagerCuda::upload_packed(uint32_t* copy_calls) {
   const uint64_t chunk = std::min<uint64_t>(kStageBytes, std::max<uint64_t>(slot_bytes, 4ull << 20));
   const uint64_t per_half = chunk / slot_bytes;
   for (int i = 0; i < 2; ++i) {
-    if (!d_stage_[i]) SVO_CUDA_TRY(cudaMalloc(&d_stage_[i], kStageBytes));
+    if (!d_stage_[i]) SVO_CUDA_TRY(device_alloc(&d_stage_[i], kStageBytes));
     if (!h_ids_[i]) SVO_CUDA_TRY(cudaMallocHost(&h_ids_[i], per_half * sizeof(uint32_t)));
-    if (!d_ids_[i]) SVO_CUDA_TRY(cudaMalloc(&d_ids_[i], per_half * sizeof(uint32_t)));
+    if (!d_ids_[i]) SVO_CUDA_TRY(device_array(&d_ids_[i], per_half));
   }
   uint32_t calls = 0;
   auto it = upload_.begin();
@@ -703,7 +695,7 @@ int TreeletMemoryManagerCuda::rgba_scratch(uint64_t pixels, uint32_t** out) {
     cudaFree(d_rgba_);
     d_rgba_ = nullptr;
     d_rgba_pixels_ = 0;
-    SVO_CUDA_TRY(cudaMalloc(&d_rgba_, pixels * sizeof(uint32_t)));
+    SVO_CUDA_TRY(device_array(&d_rgba_, pixels));
     d_rgba_pixels_ = pixels;
   }
   *out = d_rgba_;
@@ -731,7 +723,7 @@ int TreeletMemoryManagerCuda::render_to_host_async(const svo_frame_params& p,
     cudaFree(d_img_[k]);
     d_img_[k] = nullptr;
     d_img_pixels_[k] = 0;
-    SVO_CUDA_TRY(cudaMalloc(&d_img_[k], pixels * sizeof(uint32_t)));
+    SVO_CUDA_TRY(device_array(&d_img_[k], pixels));
     d_img_pixels_[k] = pixels;
   }
   // the cast may overwrite image k once its previous copy has left
@@ -775,10 +767,10 @@ int TreeletMemoryManagerCuda::init_analysis() {
     if (h_keys) cudaFreeHost(h_keys);
     return cuda_status(e);
   };
-  cudaError_t e = cudaMalloc(&d_slot, (size_t)S * sizeof(int32_t));
+  cudaError_t e = device_array(&d_slot, S);
   if (e == cudaSuccess) e = cudaMallocHost(&h_slot, (size_t)S * sizeof(int32_t));
-  if (e == cudaSuccess) e = cudaMalloc(&d_par, parent.size() * sizeof(int32_t));
-  if (e == cudaSuccess) e = cudaMalloc(&d_keys, key_words * sizeof(uint32_t));
+  if (e == cudaSuccess) e = device_array(&d_par, parent.size());
+  if (e == cudaSuccess) e = device_array(&d_keys, key_words);
   if (e == cudaSuccess) e = cudaMallocHost(&h_keys, key_words * sizeof(uint32_t));
   if (e == cudaSuccess)
     e = cudaMemcpy(d_par, parent.data(), parent.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
@@ -859,7 +851,7 @@ int TreeletMemoryManagerCuda::feedback_scratch(uint64_t records, svo_feedback** 
     cudaFree(d_feedback_);
     d_feedback_ = nullptr;
     d_feedback_records_ = 0;
-    SVO_CUDA_TRY(cudaMalloc(&d_feedback_, grow * sizeof(svo_feedback)));
+    SVO_CUDA_TRY(device_array(&d_feedback_, grow));
     d_feedback_records_ = grow;
   }
   *out = d_feedback_;

@@ -63,11 +63,7 @@ class DevicePool {
   int init(uint64_t bytes) {
     size_ = bytes & ~255ull;
     if (size_ == 0) return SVO_ERR_RANGE;
-    if (cudaMalloc(&base_, size_) != cudaSuccess) {
-      cudaGetLastError();
-      svo::give_back_kept_memory();
-      SVO_CUDA_TRY(cudaMalloc(&base_, size_));
-    }
+    SVO_CUDA_TRY(svo::device_alloc(&base_, size_));
     free_.clear();
     free_[0] = size_;
     return SVO_OK;

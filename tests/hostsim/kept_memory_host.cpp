@@ -180,6 +180,10 @@ uint64_t scratch(uint64_t bytes) {
   return svo::scratch_alloc(pool, bytes, nullptr, &p) == cudaSuccess ? (uint64_t)p : 0u;
 }
 void scratch_free(uint64_t p) { cudaFreeAsync((void*)p, nullptr); }
+uint64_t words(uint64_t n) {
+  uint32_t* p = nullptr;
+  return svo::device_array(&p, n) == cudaSuccess ? (uint64_t)p : 0u;
+}
 void begin() { svo::user_begins(0); }
 void end() { svo::user_ends(0); }
 

@@ -28,6 +28,7 @@ def load(path, tag):
     lib.block_free.argtypes = [u64, u64]
     lib.scratch.argtypes, lib.scratch.restype = [u64], u64
     lib.scratch_free.argtypes = [u64]
+    lib.words.argtypes, lib.words.restype = [u64], u64
     return lib
 
 
@@ -98,3 +99,24 @@ def test_scratch_takes_what_is_kept(device):
     device.end()
     device.end()
     assert device.fake_used() == 0
+
+
+def test_any_allocation_takes_what_is_kept(device):
+    device.begin()
+    device.begin()
+    p, got = block(device, GB)
+    device.block_free(p, got)
+    assert device.words((7 * GB + GB // 2) // 4)
+    assert device.fake_used() == 7 * GB + GB // 2
+    assert not device.words(GB // 4)
+    assert device.fake_last_error() == 0
+
+
+def test_every_allocation_of_the_library_can():
+    """Device memory is asked for in kept_memory.cpp alone, which has what is kept
+    given back where it does not fit.  (The ordering's scratch and the ray counter,
+    small pieces of a stream-ordered pool, do without.)"""
+    for f in sorted(SOURCE.parent.iterdir()):
+        if f.suffix in (".cpp", ".cu", ".cuh", ".h") and f != SOURCE:
+            for call in ("cudaMalloc(", "cudaMallocAsync(", "cudaMallocManaged(", "cudaMallocPitch("):
+                assert call not in f.read_text(), f"{f.name}: {call}"
