@@ -36,13 +36,15 @@
 //     and the treelet ids are range offsets of the boundary levels; one block
 //     per treelet writes its slot, with every sub-treelet root patched into
 //     its parent's leaf as insert_all does.
-// Octrees whose keys would not fit 64 bits, or whose columns number more than
-// kMaxColumns, run 2 to 4 once per spatial chunk (a cell of a top level).
+// Octrees whose keys would not fit 64 bits, whose columns number more than
+// kMaxColumns or whose scratch does not fit run 2 to 4 once per spatial chunk: cells
+// of the top levels, split further where one has too much (for_each_chunk), and
+// chunks that still have too many columns are walked pass by pass.
 //
 // Scratch comes from a stream-ordered memory pool of the library's own; the host
-// waits four times a chunk for a size.  An 81,920-triangle icosphere at depth 11
-// (13 M leaves, 17.3 M nodes, a 628 MB pool) takes 3.2 ms (69.7 before), a 131,072-triangle
-// terrain at depth 9 0.95 ms (22.7), the 5.2 M-triangle depth-14 octree 0.70 s (1.61).
+// waits three times a chunk for a size, and once more for the slots' size.  An
+// 81,920-triangle icosphere at depth 11 (13 M leaves, 17.3 M nodes, a 628 MB pool)
+// takes 3.2 ms (69.7 before), a 131,072-triangle terrain at depth 9 0.95 ms (22.7), the 5.2 M-triangle depth-14 octree 0.70 s (1.61).
 //
 // FP32 arithmetic uses explicit round-to-nearest intrinsics in the host
 // builder's operation order (the library is built with -fmad=false), so the
@@ -58,6 +60,7 @@
 #include <vector>
 
 #include "../../include/libsvo_b200.h"
+#include "chunk_plan.h"
 #include "errors.h"
 #include "gpu_builder.h"
 #include "kept_memory.h"
@@ -419,6 +422,12 @@ __device__ __forceinline__ uint64_t last_at_most(const uint64_t* __restrict__ of
 }
 
 constexpr int kColThreads = 256;
+
+// The columns first .. first + count - 1 of a chunk, of one pass over them.
+struct ColumnWindow {
+  uint64_t first, count;
+};
+
 // A column's hits: bit i of the low byte for the voxel i above the first
 // candidate, whose w is in the bits above; columns of more than eight candidates
 // (a triangle without a dominant axis) are tested again where they are emitted.
@@ -427,11 +436,11 @@ constexpr uint32_t kTestAgain = 0xFFFFFFFFu;
 // block_tri[b]: the triangle of the first column of block b, and of the last
 // column behind the last block.  (Looked up by one thread of each block, the
 // search was a third of the test and half of the emission.)
-__global__ void block_triangles_kernel(const uint64_t* __restrict__ off, uint64_t nt, uint64_t columns,
+__global__ void block_triangles_kernel(const uint64_t* __restrict__ off, uint64_t nt, ColumnWindow win,
                                        uint64_t blocks, uint32_t* __restrict__ block_tri) {
   const uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (b <= blocks)
-    block_tri[b] = (uint32_t)last_at_most(off, 0, nt - 1, min(b * kColThreads, columns - 1));
+    block_tri[b] = (uint32_t)last_at_most(off, 0, nt - 1, win.first + min(b * kColThreads, win.count - 1));
 }
 
 // The triangle of column c, and the column's place (iu, iv) in it.
@@ -451,11 +460,11 @@ __device__ __forceinline__ void column_place(const TriWalk& s, uint64_t k, int* 
 
 __global__ void __launch_bounds__(kColThreads) column_test_kernel(
     const TriWalk* __restrict__ walks, uint32_t depth, Chunk ch,
-    const uint64_t* __restrict__ off, const uint32_t* __restrict__ block_tri, uint64_t columns,
+    const uint64_t* __restrict__ off, const uint32_t* __restrict__ block_tri, ColumnWindow win,
     uint32_t* __restrict__ rec, uint64_t* __restrict__ block_hits) {
-  const uint64_t c = (uint64_t)blockIdx.x * kColThreads + threadIdx.x;
+  const uint64_t i = (uint64_t)blockIdx.x * kColThreads + threadIdx.x, c = win.first + i;
   uint32_t hits = 0;
-  if (c < columns) {
+  if (i < win.count) {
     const uint64_t t = column_triangle(off, block_tri, c);
     const TriWalk s = walks[t];
     int iu, iv;
@@ -470,7 +479,7 @@ __global__ void __launch_bounds__(kColThreads) column_test_kernel(
           mask |= 1u << ((iw - wlo) & 31);
         }
     }
-    rec[c] = hits == 0 ? 0u : (whi - wlo >= 8 ? kTestAgain : ((uint32_t)wlo << 8) | mask);
+    rec[i] = hits == 0 ? 0u : (whi - wlo >= 8 ? kTestAgain : ((uint32_t)wlo << 8) | mask);
   }
   __shared__ uint32_t warp_hits[kColThreads / 32];
   const uint32_t sum = __reduce_add_sync(0xFFFFFFFFu, hits);
@@ -486,11 +495,11 @@ __global__ void __launch_bounds__(kColThreads) column_test_kernel(
 
 __global__ void __launch_bounds__(kColThreads) column_emit_kernel(
     const TriWalk* __restrict__ walks, uint32_t depth, Chunk ch,
-    const uint64_t* __restrict__ off, const uint32_t* __restrict__ block_tri, uint64_t columns,
+    const uint64_t* __restrict__ off, const uint32_t* __restrict__ block_tri, ColumnWindow win,
     const uint32_t* __restrict__ rec,
     const uint64_t* __restrict__ block_off, uint64_t* __restrict__ keys) {
-  const uint64_t c = (uint64_t)blockIdx.x * kColThreads + threadIdx.x;
-  const uint32_t r = c < columns ? rec[c] : 0u;
+  const uint64_t i = (uint64_t)blockIdx.x * kColThreads + threadIdx.x, c = win.first + i;
+  const uint32_t r = i < win.count ? rec[i] : 0u;
   uint64_t t = 0;
   int w = 0, iu = 0, iv = 0, wlo = 0, whi = -1;
   uint32_t n = 0;
@@ -976,8 +985,11 @@ __global__ void __launch_bounds__(256) cut_kernel(LevelPtrs L, CutParams cp,
 
 // ---- host side -----------------------------------------------------------------------
 
-// Columns of one chunk: 2 GB of records, about 5 GB of keys.
+// Columns of one pass, at most: 2 GB of records.  A chunk of more is split while it
+// can be (for_each_chunk), then taken in several passes.
 constexpr uint64_t kMaxColumns = 1ull << 29;
+static_assert(kMaxColumns % kColThreads == 0 && kMaxColumns / kColThreads <= 0x7FFFFFFF, "whole blocks, one grid");
+
 // Scratch of one build, ordered on its stream.
 struct Scratch {
   cudaMemPool_t pool = nullptr;
@@ -1068,21 +1080,17 @@ int sort_keys(const Scratch& sc, cub::DoubleBuffer<uint64_t>& kb, Count n, int l
   return SVO_OK;
 }
 
-Chunk chunk_of(uint32_t ci, uint32_t chunk_levels, uint32_t depth, uint32_t tri_bits) {
-  // chunk ci in Morton order: its code prefix is ci
+Chunk chunk_of(const Cell& cell, uint32_t depth, uint32_t tri_bits) {
   uint32_t cxyz[3] = {0, 0, 0};
-  for (uint32_t b = 0; b < chunk_levels; ++b) {
-    cxyz[0] |= ((ci >> (3 * b + 2)) & 1u) << b;
-    cxyz[1] |= ((ci >> (3 * b + 1)) & 1u) << b;
-    cxyz[2] |= ((ci >> (3 * b)) & 1u) << b;
-  }
-  const uint32_t cs = (1u << depth) >> chunk_levels;  // voxels per chunk per axis
+  for (uint32_t b = 0; b < cell.level; ++b)
+    for (int k = 0; k < 3; ++k) cxyz[k] |= (uint32_t)((cell.index >> (3 * b + 2 - k)) & 1u) << b;
+  const uint32_t cs = (1u << depth) >> cell.level;  // voxels per chunk per axis
   Chunk ch;
   for (int k = 0; k < 3; ++k) {
     ch.lo[k] = (int)(cxyz[k] * cs);
     ch.hi[k] = (int)((cxyz[k] + 1) * cs) - 1;
   }
-  ch.shift = 3 * (depth - chunk_levels);
+  ch.shift = 3 * (depth - cell.level);
   ch.tri_bits = tri_bits;
   return ch;
 }
@@ -1148,57 +1156,60 @@ int DeviceScene::build_mesh(const float* h_vertices, const float* h_normals,
   GB_TRY(cudaMemsetAsync(d_totals.p, 0, kMaxLevels * sizeof(uint64_t), st));
   std::vector<Levels> parts;
   uint64_t totals[kMaxLevels] = {};
-  auto count_columns = [&](const Chunk& ch, uint64_t* n) -> int {
-    column_count_kernel<<<grid_of(nt + 1, 128), 128, 0, st>>>(dV.p, dT.p, nt, depth, ch, walks.p, cols.p);
+  auto count_columns = [&](const Cell& cell, uint64_t* n) -> int {
+    column_count_kernel<<<grid_of(nt + 1, 128), 128, 0, st>>>(dV.p, dT.p, nt, depth,
+                                                              chunk_of(cell, depth, tri_bits), walks.p, cols.p);
     GB_TRY(cudaGetLastError());
     return sum_counts(sc, cols.p, nt, n);
   };
-  uint64_t columns = 0;
-  Chunk ch = chunk_of(0, chunk_levels, depth, tri_bits);
-  int rc = count_columns(ch, &columns);
-  if (rc != SVO_OK) return rc;
-  if (chunk_levels == 0 && columns > kMaxColumns && depth > 1) {
-    // the columns spread over 8^levels cells, about half of them empty
-    while (chunk_levels < std::min(depth - 1, 3u) && (columns >> (2 * chunk_levels)) > kMaxColumns)
-      ++chunk_levels;
-    ch = chunk_of(0, chunk_levels, depth, tri_bits);
-    rc = count_columns(ch, &columns);
-    if (rc != SVO_OK) return rc;
-  }
-  const uint32_t num_chunks = 1u << (3 * chunk_levels);
-  uint32_t last_chunk = 0;  // the last chunk with leaves
-  for (uint32_t ci = 0; ci < num_chunks; ++ci) {
-    if (ci > 0) {
-      ch = chunk_of(ci, chunk_levels, depth, tri_bits);
-      rc = count_columns(ch, &columns);
-      if (rc != SVO_OK) return rc;
-    }
-    if (columns == 0) continue;
-    const uint64_t col_blocks = (columns + kColThreads - 1) / kColThreads;
-    if (col_blocks > 0x7FFFFFFFull) return SVO_ERR_RANGE;
+  Cell last_cell = {0, 0};  // the last one with leaves
+  auto build_chunk = [&](const Cell& cell, uint64_t columns, bool* began) -> int {
+    const Chunk ch = chunk_of(cell, depth, tri_bits);
+    int rc = SVO_OK;
     DevBuf<uint64_t> keys, keys2;
     uint64_t P = 0;
     {
+      // pass by pass over the columns where they are more than a pass may have:
+      // the overlaps are counted first, and each pass's test made again for them
+      const uint64_t pass = std::min(columns, kMaxColumns);
+      const uint64_t col_blocks = (pass + kColThreads - 1) / kColThreads;
       DevBuf<uint32_t> rec;
       DevBuf<uint64_t> block_hits;
       DevBuf<uint32_t> block_tri;
-      GB_TRY(rec.alloc(sc, columns));
+      GB_TRY(rec.alloc(sc, pass));
       GB_TRY(block_hits.alloc(sc, col_blocks + 1));
       GB_TRY(block_tri.alloc(sc, col_blocks + 1));
-      block_triangles_kernel<<<grid_of(col_blocks + 1, 256), 256, 0, st>>>(cols.p, nt, columns, col_blocks,
-                                                                          block_tri.p);
-      GB_TRY(cudaGetLastError());
-      column_test_kernel<<<(unsigned)col_blocks, kColThreads, 0, st>>>(
-          walks.p, depth, ch, cols.p, block_tri.p, columns, rec.p, block_hits.p);
-      GB_TRY(cudaGetLastError());
-      rc = sum_counts(sc, block_hits.p, col_blocks, &P);
-      if (rc != SVO_OK) return rc;
-      pairs += P;
-      if (P == 0) continue;
+      ColumnWindow win = {0, 0};
+      unsigned blocks = 0;
+      auto test_columns = [&](uint64_t first, uint64_t* hits) -> int {
+        win = {first, std::min(pass, columns - first)};
+        blocks = grid_of(win.count, kColThreads);
+        block_triangles_kernel<<<grid_of(blocks + 1, 256), 256, 0, st>>>(cols.p, nt, win, blocks, block_tri.p);
+        GB_TRY(cudaGetLastError());
+        column_test_kernel<<<blocks, kColThreads, 0, st>>>(walks.p, depth, ch, cols.p, block_tri.p, win, rec.p,
+                                                           block_hits.p);
+        GB_TRY(cudaGetLastError());
+        return sum_counts(sc, block_hits.p, blocks, hits);
+      };
+      uint64_t hits = 0;
+      for (uint64_t first = 0; first < columns; first += pass) {
+        rc = test_columns(first, &hits);
+        if (rc != SVO_OK) return rc;
+        P += hits;
+      }
+      if (P == 0) return SVO_OK;
       GB_TRY(keys.alloc(sc, P));
-      column_emit_kernel<<<(unsigned)col_blocks, kColThreads, 0, st>>>(
-          walks.p, depth, ch, cols.p, block_tri.p, columns, rec.p, block_hits.p, keys.p);
-      GB_TRY(cudaGetLastError());
+      uint64_t at = 0;
+      for (uint64_t first = 0; first < columns; first += pass) {
+        if (pass < columns) {
+          rc = test_columns(first, &hits);
+          if (rc != SVO_OK) return rc;
+        }
+        column_emit_kernel<<<blocks, kColThreads, 0, st>>>(walks.p, depth, ch, cols.p, block_tri.p, win, rec.p,
+                                                           block_hits.p, keys.p + at);
+        GB_TRY(cudaGetLastError());
+        at += hits;
+      }
     }
     // stable, by code alone: the triangles of a code are ascending already
     GB_TRY(keys2.alloc(sc, P));
@@ -1216,12 +1227,7 @@ int DeviceScene::build_mesh(const float* h_vertices, const float* h_normals,
     kl.tri_bits = tri_bits;
     kl.depth = depth;
     kl.first_level = 0;
-    if (!parts.empty()) {  // the chunk's prefix against the last one's
-      uint32_t digit = 0;
-      while ((last_chunk ^ ci) >> (3 * (digit + 1))) ++digit;
-      kl.first_level = chunk_levels - digit;
-    }
-    last_chunk = ci;
+    if (!parts.empty()) kl.first_level = first_new_level(last_cell, cell, depth);
     const uint64_t key_blocks = (P + kKeyBlock - 1) / kKeyBlock;
     if (key_blocks > 0x7FFFFFFFull) return SVO_ERR_RANGE;
     DevBuf<uint32_t> counts;
@@ -1234,26 +1240,40 @@ int DeviceScene::build_mesh(const float* h_vertices, const float* h_normals,
     GB_TRY(cudaMemcpyAsync(now, d_totals.p, sizeof(now), cudaMemcpyDeviceToHost, st));
     GB_TRY(cudaStreamSynchronize(st));
     if (now[depth] > 0xFFFFFFFFull) return SVO_ERR_RANGE;
-    parts.emplace_back();
-    Levels& lv = parts.back();
+    Levels lv;
     LevelOut out = {};
-    for (uint32_t d = 0; d <= depth; ++d) {
-      lv.size[d] = now[d] - totals[d];
-      out.base[d] = (uint32_t)totals[d];
-      totals[d] = now[d];
-      GB_TRY(lv.octant[d].alloc(sc, lv.size[d]));
-      out.octant[d] = lv.octant[d].p;
-      if (d == depth) continue;
-      GB_TRY(lv.first[d].alloc(sc, lv.size[d]));
-      out.first[d] = lv.first[d].p;
+    auto alloc_levels = [&]() -> int {
+      for (uint32_t d = 0; d <= depth; ++d) {
+        lv.size[d] = now[d] - totals[d];
+        out.base[d] = (uint32_t)totals[d];
+        GB_TRY(lv.octant[d].alloc(sc, lv.size[d]));
+        out.octant[d] = lv.octant[d].p;
+        if (d == depth) continue;
+        GB_TRY(lv.first[d].alloc(sc, lv.size[d]));
+        out.first[d] = lv.first[d].p;
+      }
+      GB_TRY(lv.leaf_attribs.alloc(sc, lv.size[depth]));
+      out.leaf_attribs = lv.leaf_attribs.p;
+      return SVO_OK;
+    };
+    rc = alloc_levels();
+    if (rc != SVO_OK) {  // the totals as they were, for the cell's children
+      GB_TRY(cudaMemcpyAsync(d_totals.p, totals, sizeof(totals), cudaMemcpyHostToDevice, st));
+      return rc;
     }
-    GB_TRY(lv.leaf_attribs.alloc(sc, lv.size[depth]));
-    out.leaf_attribs = lv.leaf_attribs.p;
-    leaf_in.chunk_base = (uint64_t)ci << ch.shift;
+    *began = true;
+    std::copy(now, now + kMaxLevels, totals);
+    last_cell = cell;
+    pairs += P;
+    parts.push_back(std::move(lv));
+    leaf_in.chunk_base = cell_code(cell, depth);
     level_write_kernel<<<(unsigned)key_blocks, kKeyThreads, 0, st>>>(kl, leaf_in, key_blocks, counts.p,
                                                                     out);
     GB_TRY(cudaGetLastError());
-  }
+    return SVO_OK;
+  };
+  int rc = for_each_chunk(depth, chunk_levels, kMaxColumns, count_columns, build_chunk);
+  if (rc != SVO_OK) return rc;
   cols.reset();
   walks.reset();
   dV.reset();
