@@ -15,6 +15,7 @@
 #include "errors.h"
 #include "feedback.h"
 #include "gpu_builder.h"
+#include "host_image.h"
 #include "memory_manager.h"
 #include "render.h"
 #include "scene.h"
@@ -43,21 +44,6 @@ int guarded(Fn&& fn) {
   } catch (...) {
     return SVO_ERR_INVALID;
   }
-}
-
-// The device-side address of a host image that is page-locked and mapped from
-// its first to its last pixel and lies at a pixel's alignment; else null.
-uint32_t* mapped_image(uint32_t* h, uint64_t pixels) {
-  cudaPointerAttributes first, last;
-  if (((uintptr_t)h & 3u) != 0u || cudaPointerGetAttributes(&first, h) != cudaSuccess ||
-      cudaPointerGetAttributes(&last, h + (pixels - 1)) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  if (first.type != cudaMemoryTypeHost || last.type != cudaMemoryTypeHost || !first.devicePointer ||
-      (uint32_t*)last.devicePointer != (uint32_t*)first.devicePointer + (pixels - 1))
-    return nullptr;
-  return (uint32_t*)first.devicePointer;
 }
 
 int check_cfg(const svo_trace_cfg* cfg) {
@@ -621,7 +607,7 @@ int svo_mm_render_host(svo_mm* mm, const svo_frame_params* params, const svo_tra
   cudaStream_t s = stream ? (cudaStream_t)stream : mm->impl.render_stream();
   const uint64_t pixels = (uint64_t)params->width * params->height;
   if (pixels == 0) return SVO_OK;
-  uint32_t* d_rgba = mapped_image(h_rgba, pixels);
+  uint32_t* d_rgba = svo::mapped_image(h_rgba, pixels);
   if (d_rgba) {
     // page-locked: the cast writes the image there itself, so its blocks' pixels
     // cross PCIe while others are cast (a 1280x720 frame 186 ->
