@@ -384,19 +384,20 @@ constexpr uint32_t kGridRows = 65535u;
 
 namespace {
 
-// The scratch of longest-first dispatch (196 bytes per block) comes from a
-// memory pool of the library's own, one per device, in stream order: calls
-// on different streams get different scratch, and the pool keeps up to 64 MB
-// between calls instead of returning it at every synchronisation.
+// The scratch of a cast -- longest-first dispatch's lists, 196 bytes per block,
+// and the ray counter of stream_rays_kernel -- comes from a memory pool of the
+// library's own, one per device, in stream order: calls on different streams get
+// different scratch, and the pool keeps up to 64 MB between calls instead of
+// returning it at every synchronisation.
 constexpr int kMaxDevices = 64;
-cudaMemPool_t g_order_pool[kMaxDevices] = {};
-std::mutex g_order_pool_mu;
+cudaMemPool_t g_scratch_pool[kMaxDevices] = {};
+std::mutex g_scratch_pool_mu;
 
-cudaMemPool_t order_pool() {
+cudaMemPool_t scratch_pool() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
-  std::lock_guard<std::mutex> lock(g_order_pool_mu);
-  if (!g_order_pool[dev]) {
+  std::lock_guard<std::mutex> lock(g_scratch_pool_mu);
+  if (!g_scratch_pool[dev]) {
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -405,9 +406,9 @@ cudaMemPool_t order_pool() {
     if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) return nullptr;
     uint64_t keep = 64ull << 20;
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    g_order_pool[dev] = pool;
+    g_scratch_pool[dev] = pool;
   }
-  return g_order_pool[dev];
+  return g_scratch_pool[dev];
 }
 
 // Longest-first order of the frame's blocks into *order (stream-ordered
@@ -418,7 +419,7 @@ bool order_blocks(const uint2* nodes, uint64_t num_nodes, const svo_frame_params
                   bool flat, uint32_t gx, uint32_t nblocks, cudaStream_t stream, BlockOrder* order) {
   const uint64_t pixels = (uint64_t)p.width * p.height;
   if (pixels < kOrderMinPixels || pixels > kOrderMaxPixels) return false;
-  cudaMemPool_t pool = order_pool();
+  cudaMemPool_t pool = scratch_pool();
   if (!pool) {
     cudaGetLastError();
     return false;
@@ -556,7 +557,7 @@ int stream_rays(const uint2* nodes, uint64_t num_nodes, const float* origins, co
   const size_t smem = render_smem_bytes(S);
   int dev = 0, sms = 0, per_sm = 0;
   uint32_t* next = nullptr;
-  cudaMemPool_t pool = order_pool();
+  cudaMemPool_t pool = scratch_pool();
   if (!pool || cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, smem) != cudaSuccess || per_sm < 1 ||

@@ -84,11 +84,6 @@ __device__ __forceinline__ float cl_sign(float v) {
 // 2^e for -126 <= e <= 0, exact.
 __device__ __forceinline__ float pow2i(int e) { return __int_as_float((127 + e) << 23); }
 
-// Centre coordinate of lattice cell i at depth k: -0.5 + (2i+1) * 2^-(k+1).
-__device__ __forceinline__ float cell_center(uint32_t i, int k) {
-  return __fadd_rn(-0.5f, __fmul_rn((float)(2u * i + 1u), pow2i(-(k + 1))));
-}
-
 // intersectAABB (opencl/treeletRenderer_rgba.cl:100-178) against [-0.5,0.5]^3.
 __device__ __forceinline__ bool root_slab(const float o[3], const float d[3], float& t_min,
                                           float& t_max) {
