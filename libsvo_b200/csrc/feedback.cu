@@ -13,6 +13,7 @@
 
 #include "feedback.h"
 #include "render.h"
+#include "row_bands.h"
 #include "shade.cuh"
 #include "traverse.cuh"
 
@@ -67,15 +68,12 @@ int launch_feedback(const svo_node* nodes, uint64_t num_nodes, const svo_frame_p
   if (p.height > 0xFFFFFFF0u) return SVO_ERR_RANGE;  // row indices stay below 2^32
   const size_t smem = (size_t)S * kThreads * sizeof(uint2);
   const uint32_t rays = rays_per_warp((uint64_t)p.width * p.height), block_h = rays / kBlockW;
-  const uint32_t per_launch = 65535u * block_h;  // grid rows are at most 65535
-  for (uint32_t y0 = 0; y0 < p.height; y0 += per_launch) {
-    const uint32_t rows = p.height - y0 < per_launch ? p.height - y0 : per_launch;
-    const dim3 grid((p.width + kBlockW - 1) / kBlockW, (rows + block_h - 1) / block_h);
-    feedback_kernel<<<grid, kThreads, smem, stream>>>(reinterpret_cast<const uint2*>(nodes),
-                                                       num_nodes, p, S, out, rgba, y0, rays);
-    if (cudaGetLastError() != cudaSuccess) return SVO_ERR_CUDA;
-  }
-  return SVO_OK;
+  const uint32_t gx = (p.width + kBlockW - 1) / kBlockW;
+  return for_each_band(p.height, block_h, [&](uint32_t y0, uint32_t, uint32_t gy) -> int {
+    feedback_kernel<<<dim3(gx, gy), kThreads, smem, stream>>>(reinterpret_cast<const uint2*>(nodes),
+                                                              num_nodes, p, S, out, rgba, y0, rays);
+    return cudaGetLastError() == cudaSuccess ? SVO_OK : SVO_ERR_CUDA;
+  });
 }
 
 }  // namespace svo

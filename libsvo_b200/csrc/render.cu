@@ -13,6 +13,7 @@
 #include <mutex>
 
 #include "render.h"
+#include "row_bands.h"
 #include "shade.cuh"
 #include "traverse.cuh"
 
@@ -379,9 +380,6 @@ __global__ void __launch_bounds__(kThreads) stream_rays_kernel(
 
 size_t render_smem_bytes(int S) { return (size_t)S * kThreads * sizeof(uint2); }
 
-// Blocks along y of one launch.
-constexpr uint32_t kGridRows = 65535u;
-
 namespace {
 
 // The scratch of a cast -- longest-first dispatch's lists, 196 bytes per block,
@@ -497,14 +495,11 @@ int launch_render(const svo_node* nodes, const svo_attrib* attribs, uint64_t num
     return e == cudaSuccess ? SVO_OK : SVO_ERR_CUDA;
   }
   const uint32_t rays = rays_per_warp((uint64_t)p.width * p.height), block_h = kBlockH / 4 * rays / 8;
-  for (uint32_t y0 = 0; y0 < p.height; y0 += kGridRows * block_h) {
-    const uint32_t rows = std::min(p.height - y0, kGridRows * block_h);
-    const dim3 grid(gx, (rows + block_h - 1) / block_h);
-    fn<<<grid, kThreads, smem, stream>>>(n2, a2, num_nodes, p, S, rgba, hits, stats, y0,
-                                         BlockOrder{nullptr, nullptr, 0u}, gx, rays);
-    if (cudaGetLastError() != cudaSuccess) return SVO_ERR_CUDA;
-  }
-  return SVO_OK;
+  return for_each_band(p.height, block_h, [&](uint32_t y0, uint32_t, uint32_t gy) -> int {
+    fn<<<dim3(gx, gy), kThreads, smem, stream>>>(n2, a2, num_nodes, p, S, rgba, hits, stats, y0,
+                                                 BlockOrder{nullptr, nullptr, 0u}, gx, rays);
+    return cudaGetLastError() == cudaSuccess ? SVO_OK : SVO_ERR_CUDA;
+  });
 }
 
 int launch_render_shadow(const svo_node* nodes, const svo_attrib* attribs, uint64_t num_nodes,
@@ -526,14 +521,11 @@ int launch_render_shadow(const svo_node* nodes, const svo_attrib* attribs, uint6
   // descent in L1; cast in a later pass it reads them from L2 again.
   const uint32_t gx = (p.width + kBlockW - 1) / kBlockW;
   const uint32_t rays = rays_per_warp((uint64_t)p.width * p.height), block_h = kBlockH / 4 * rays / 8;
-  for (uint32_t y0 = 0; y0 < p.height; y0 += kGridRows * block_h) {
-    const uint32_t rows = std::min(p.height - y0, kGridRows * block_h);
-    const dim3 grid(gx, (rows + block_h - 1) / block_h);
-    render_shadow_kernel<<<grid, kThreads, render_smem_bytes(S), stream>>>(
+  return for_each_band(p.height, block_h, [&](uint32_t y0, uint32_t, uint32_t gy) -> int {
+    render_shadow_kernel<<<dim3(gx, gy), kThreads, render_smem_bytes(S), stream>>>(
         n2, a2, num_nodes, p, sc, S, rgba, hits, shadow_hits, stats, y0, rays);
-    if (cudaGetLastError() != cudaSuccess) return SVO_ERR_CUDA;
-  }
-  return SVO_OK;
+    return cudaGetLastError() == cudaSuccess ? SVO_OK : SVO_ERR_CUDA;
+  });
 }
 
 namespace {
