@@ -13,6 +13,7 @@
 #include <mutex>
 
 #include "render.h"
+#include "ray_order.cuh"
 #include "row_bands.h"
 #include "shade.cuh"
 #include "traverse.cuh"
@@ -289,12 +290,35 @@ __global__ void __launch_bounds__(kThreads) render_shadow_kernel(
   count_stats(stats, h);
 }
 
-template <bool kFlat>
-__global__ void __launch_bounds__(kThreads) trace_rays_kernel(
+// Whether a set's rays come in order (ray_order.cuh): every block asks the same
+// eight pairs, which its SM then has in L1.  Called by the whole block.
+__device__ __forceinline__ bool rays_in_order(const float* origins, const float* dirs, uint64_t n) {
+  __shared__ bool in_order;
+  if (threadIdx.x < 32) {
+    const bool close = threadIdx.x < kOrderPairs && pair_close(origins, dirs, order_pair(threadIdx.x, n));
+    const uint32_t pairs = __ballot_sync(0xFFFFFFFFu, close);
+    if (threadIdx.x == 0) in_order = (uint32_t)__popc(pairs) >= kOrderClose;
+  }
+  __syncthreads();
+  return in_order;
+}
+
+// kAsk: casts the rays only if they come in order; launched as a programmatic
+// dependent of stream_rays_kernel, which casts them if they do not.  Behind it, not
+// ahead of it: the blocks that find nothing to cast come and go while the last rays
+// end (ahead of it a million rays without order took 267 against 260 us, four
+// million 883 against 854).  Held to the 10 blocks an SM of the plain kernel.
+template <bool kFlat, bool kAsk>
+__global__ void __launch_bounds__(kThreads, kAsk ? 10 : 0) trace_rays_kernel(
     const uint2* __restrict__ nodes, uint64_t num_nodes, const float* __restrict__ origins,
     const float* __restrict__ dirs, uint64_t n, float tsr, int S, svo_hit* __restrict__ hits,
     svo_stats* __restrict__ stats, uint32_t rays) {
   extern __shared__ uint2 stack_smem[];
+  if (kAsk) {
+    // what comes behind this grid waits for it, and so for the grids before it
+    if (blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!rays_in_order(origins, dirs, n)) return;
+  }
   const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const uint64_t i = ((uint64_t)blockIdx.x * (kThreads / 32) + warp) * rays + lane;
   if (lane >= rays || i >= n) return;
@@ -305,22 +329,37 @@ __global__ void __launch_bounds__(kThreads) trace_rays_kernel(
   count_stats(stats, h);
 }
 
+// The ray counter of stream_rays_kernel, which need not wait for it until it casts
+// (a cleared counter by cudaMemsetAsync: 256,000 pixel rays over a terrain 46 us,
+// so 43).
+__global__ void clear_kernel(uint32_t* next) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  *next = 0u;
+}
+
 // The same rays with lanes that take the next ray as soon as enough of their
-// warp's have ended (kKeepLanes or fewer still run).  Explicit rays come in any
-// order, so the rays of a warp differ in length by an order of magnitude, and
-// lanes of ended rays idled through two thirds of the warp's passes.  `next` is
-// the next ray to take, 0 at launch.  A million rays without order over the
-// depth-11 icosphere 441 -> 326 us, over a depth-10 terrain 365 -> 244 us; two
-// million pixel rays in raster order, which end together anyway, 295 -> 324 us
-// (8 lanes kept: 335, 272 and 304 us; 14: 338, 252, 324; 26: 346, 264, 361).  72
-// registers; bounded to 64 for an eighth block an SM it is slower (336 us).
+// warp's have ended (kKeepLanes or fewer still run).  Rays without order differ in
+// length by an order of magnitude within a warp, and lanes of ended rays idled
+// through two thirds of the warp's passes.  `next` is the next ray to take, 0 at
+// launch.  A million rays without order, a thread a ray against this (us): depth-9
+// icosphere 341 -> 258, depth-11 icosphere 399 -> 302, depth-10 terrain 342 -> 237;
+// with 8 lanes kept 266, 312, 266, with 14 266, 314, 246, with 26 275, 319, 252.
+// Rays in order end together anyway, and a thread a ray is the faster one by up to
+// a third (921,600 pixel rays 148 against 164 us over the icospheres, 65 against 84
+// over the terrain), so they are left to trace_rays_kernel.  72 registers; bounded to
+// 64 for an eighth block an SM it was slower (336 against 326 us).
 constexpr int kKeepLanes = 20;
 template <bool kFlat>
 __global__ void __launch_bounds__(kThreads) stream_rays_kernel(
     const uint2* __restrict__ nodes, uint64_t num_nodes, const float* __restrict__ origins,
     const float* __restrict__ dirs, uint32_t n, float tsr, int S, svo_hit* __restrict__ hits,
-    svo_stats* __restrict__ stats, uint32_t* __restrict__ next) {
+    svo_stats* __restrict__ stats, uint32_t* next) {
   extern __shared__ uint2 stack_smem[];
+  // trace_rays_kernel may be scheduled once every block of this grid has started
+  asm volatile("griddepcontrol.launch_dependents;");
+  const bool in_order = rays_in_order(origins, dirs, n);
+  if (!in_order || blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");  // for the counter
+  if (in_order) return;
   uint2* stack = stack_smem + threadIdx.x;
   const uint32_t lane = threadIdx.x % 32;
   const GlobalFetch fetch{nodes};
@@ -530,22 +569,27 @@ int launch_render_shadow(const svo_node* nodes, const svo_attrib* attribs, uint6
 
 namespace {
 
-// From here on the rays fill the GPU several times over, and the counter's
-// allocation and clearing are lost in the cast.
-constexpr uint64_t kStreamRays = 1ull << 17;
+// From here on lanes have rays to take: a third more than all lanes of
+// stream_rays_kernel hold at once (us, a thread a ray against it, rays without order
+// over depth-9 and depth-11 icospheres and a depth-10 terrain: 131,072 rays 73 / 98 /
+// 79 against 87 / 113 / 89, 170,000 87 / 112 / 97 against 99 / 115 / 104, 200,000 104 /
+// 133 / 108 against 102 / 126 / 105, 262,144 121 / 146 / 127 against 114 / 140 / 119).
+constexpr uint64_t kStreamRays = 3ull << 16;
 
-// stream_rays_kernel, as many blocks as are resident at once.  SVO_ERR_NOTSUP,
-// with nothing launched, where there is no scratch for its counter or the stream
-// is being captured.
-int stream_rays(const uint2* nodes, uint64_t num_nodes, const float* origins, const float* dirs,
-                uint32_t n, float tsr, int S, bool flat, svo_hit* hits, svo_stats* stats,
-                cudaStream_t stream) {
+// A set of rays whose order is not known: stream_rays_kernel, as many blocks as are
+// resident at once, and behind it trace_rays_kernel; one of them casts the set, the
+// other finds that it need not.  SVO_ERR_NOTSUP, with nothing launched, where there
+// is no scratch for the counter or the stream is being captured.
+int stream_or_trace(const uint2* nodes, uint64_t num_nodes, const float* origins, const float* dirs,
+                    uint32_t n, float tsr, int S, bool flat, svo_hit* hits, svo_stats* stats,
+                    cudaStream_t stream) {
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
     cudaGetLastError();
     return SVO_ERR_NOTSUP;
   }
   auto* fn = flat ? stream_rays_kernel<true> : stream_rays_kernel<false>;
+  auto* trace = flat ? trace_rays_kernel<true, true> : trace_rays_kernel<false, true>;
   const size_t smem = render_smem_bytes(S);
   int dev = 0, sms = 0, per_sm = 0;
   uint32_t* next = nullptr;
@@ -557,12 +601,27 @@ int stream_rays(const uint2* nodes, uint64_t num_nodes, const float* origins, co
     cudaGetLastError();
     return SVO_ERR_NOTSUP;
   }
-  cudaError_t e = cudaMemsetAsync(next, 0, sizeof(uint32_t), stream);
+  const unsigned blocks = (n + kThreads - 1) / kThreads;
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(std::min(blocks, (unsigned)(sms * per_sm)));
+  lc.blockDim = dim3(kThreads);
+  lc.dynamicSmemBytes = smem;
+  lc.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  clear_kernel<<<1, 1, 0, stream>>>(next);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = cudaLaunchKernelEx(&lc, fn, nodes, num_nodes, origins, dirs, n, tsr, S, hits, stats, next);
   if (e == cudaSuccess) {
-    const unsigned blocks = std::min<unsigned>((n + kThreads - 1) / kThreads, (unsigned)(sms * per_sm));
-    fn<<<blocks, kThreads, smem, stream>>>(nodes, num_nodes, origins, dirs, n, tsr, S, hits, stats, next);
-    e = cudaGetLastError();
+    lc.gridDim = dim3(blocks);
+    e = cudaLaunchKernelEx(&lc, trace, nodes, num_nodes, origins, dirs, (uint64_t)n, tsr, S, hits, stats, 32u);
   }
+  const cudaError_t last = cudaGetLastError();  // clears a launch error
+  if (e == cudaSuccess) e = last;
   cudaFreeAsync(next, stream);
   return e == cudaSuccess ? SVO_OK : SVO_ERR_CUDA;
 }
@@ -582,15 +641,15 @@ int launch_trace_rays(const svo_node* nodes, uint64_t num_nodes, const float* or
   const size_t smem = render_smem_bytes(S);
   const uint2* n2 = reinterpret_cast<const uint2*>(nodes);
   if (n >= kStreamRays && n <= 0x7FFFFFFFull) {
-    const int rc = stream_rays(n2, num_nodes, origins, dirs, (uint32_t)n, tsr, S,
-                               cfg.traversal == SVO_TRAVERSAL_FLAT, hits, stats, stream);
+    const int rc = stream_or_trace(n2, num_nodes, origins, dirs, (uint32_t)n, tsr, S,
+                                   cfg.traversal == SVO_TRAVERSAL_FLAT, hits, stats, stream);
     if (rc != SVO_ERR_NOTSUP) return rc;
   }
   if (cfg.traversal == SVO_TRAVERSAL_FLAT)
-    trace_rays_kernel<true><<<(unsigned)blocks, kThreads, smem, stream>>>(
+    trace_rays_kernel<true, false><<<(unsigned)blocks, kThreads, smem, stream>>>(
         n2, num_nodes, origins, dirs, n, tsr, S, hits, stats, rays);
   else
-    trace_rays_kernel<false><<<(unsigned)blocks, kThreads, smem, stream>>>(
+    trace_rays_kernel<false, false><<<(unsigned)blocks, kThreads, smem, stream>>>(
         n2, num_nodes, origins, dirs, n, tsr, S, hits, stats, rays);
   return cudaGetLastError() == cudaSuccess ? SVO_OK : SVO_ERR_CUDA;
 }
