@@ -235,31 +235,30 @@ def reference_parity(nodes, attribs, params, gpu_rgba, gpu_hits, light=None, gpu
     return out
 
 
-def run_reference(args, wl):
+def run_reference(args):
     """The reference arm: the reference's renderToBuffer compiled for the host
-    (oracle/_ref; the oracle port if that is absent), all host threads, on
-    the same workload.  A step is one frame, or an evenly spread band of its
-    rows when whole frames would make the run longer than about two minutes."""
-    import libsvo_b200 as L
+    (oracle/_ref), all host threads, on the same workload.  A step is one frame,
+    or an evenly spread band of its rows when whole frames would make the run
+    longer than about two minutes.  Without that build there is nothing of the
+    reference to run, and the line says so."""
     import oracle
 
+    if oracle.reference_lib() is None:
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's sources are not here to be compiled: "
+                                                              "no oracle/_ref library"}), flush=True)
+        return
+    import libsvo_b200 as L
+
+    wl = make_workload(args.workload)
     info = wl.scene.info
     mm = L.TreeletMemoryManagerCuda(wl.scene, info.treelet_bytes * info.num_treelets)
     mm.insertAll()
     nodes, attribs = mm.getIncoreBuffer()
     threads = os.cpu_count() or 1
-    ref = oracle.reference_lib() is not None
     params = [bytes(c.frame_params()) for c in wl.cameras]
 
     def cast(p, rows):
-        if ref:
-            oracle.reference_render(nodes, attribs, p, threads=threads, rows=rows)
-        else:
-            sub = bytearray(p)  # the port renders whole frames: shrink the frame instead
-            w = int(np.frombuffer(p[:4], dtype=np.uint32)[0])
-            sub[4:8] = np.uint32(rows[1] - rows[0]).tobytes()
-            oracle.render(nodes, attribs, bytes(sub), stack_size=wl.stack_size, threads=threads)
-            del w
+        oracle.reference_render(nodes, attribs, p, threads=threads, rows=rows)
 
     t0 = time.perf_counter()
     for p in params:
@@ -284,18 +283,16 @@ def run_reference(args, wl):
     rays = sum(r for r, _ in per)
     secs = sum(e for _, e in per)
     value = rays / secs / 1e6
-    kind = "reference" if ref else "port"
     sample = (f"{'whole frames' if frac >= 1.0 else f'{frac:.3f} of each frame (row bands)'} per step, "
               f"{rays} rays in {secs:.1f} s; "
-              + ("reference treeletRenderer_rgba.cl renderToBuffer compiled for the host"
-                 if ref else "oracle restatement of sample()"))
+              "reference treeletRenderer_rgba.cl renderToBuffer compiled for the host")
     line = {
         "impl": "reference", "metric": METRIC, "value": value, "unit": METRIC,
         "n_gpus": args.gpus, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": wl.rays_per_step / value / 1e3, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f32", "data": "synthetic (seeded scene generators)",
         "config": {"workload": wl.name, "description": wl.description, "rays_per_step": wl.rays_per_step},
-        "cpu_baseline": {"value": value, "unit": METRIC, "cores": threads, "kind": kind, "sample": sample},
+        "cpu_baseline": {"value": value, "unit": METRIC, "cores": threads, "kind": "reference", "sample": sample},
         "e2e": {"value": value, "unit": METRIC, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
     }
     print(json.dumps(line), flush=True)
@@ -1029,7 +1026,7 @@ def main():
     if args.impl == "reference":
         if rank != 0:
             return
-        run_reference(args, make_workload(args.workload))
+        run_reference(args)
         return
 
     import torch
