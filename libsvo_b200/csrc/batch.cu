@@ -121,10 +121,11 @@ __global__ void batch_kernel(const BatchView* __restrict__ views, uint32_t num_v
                                      top_nodes, rays_per_lane);
 }
 
-// The same kernel for 128-thread blocks, held to 8 resident blocks per SM:
-// 62 registers without spills instead of 65 and 7 blocks (the terrain batch
-// of 64 views: 7.92 against 8.34 ms; at 9 blocks the registers spill and it
-// is slower again).
+// The same kernel for 128-thread blocks, held to 8 resident blocks per SM: 64
+// registers without spills.  Unbounded, the general instantiations take 72, or 64
+// with 28 bytes spilled; the treelet-only ones take 64 either way and come out 1 %
+// faster (64 views of 512x512 over a depth-10 terrain 1,961 against 1,983 us, over a
+// depth-11 icosphere 1,461 against 1,478).  At 9 blocks 2,046 and 1,521 us.
 template <int TW, int TH, bool kExt, bool kTreelet>
 __global__ void __launch_bounds__(128, 8) batch_kernel_128(
     const BatchView* __restrict__ views, uint32_t num_views, const BatchOctree* __restrict__ octrees,

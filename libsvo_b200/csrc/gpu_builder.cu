@@ -44,7 +44,13 @@
 // Scratch comes from a stream-ordered memory pool of the library's own; the host
 // waits three times a chunk for a size, and once more for the slots' size.  An
 // 81,920-triangle icosphere at depth 11 (13 M leaves, 17.3 M nodes, a 628 MB pool)
-// takes 3.2 ms (69.7 before), a 131,072-triangle terrain at depth 9 0.95 ms (22.7), the 5.2 M-triangle depth-14 octree 0.70 s (1.61).
+// takes 3.2 ms while another scene keeps scratch and a destroyed scene's pool on the
+// device (kept_memory.h), 5.5 ms with no other scene alive (69 before the columns);
+// a 131,072-triangle terrain at depth 9 0.9 and 1.7 ms (20); the first build of a
+// process 13 ms (25); the 5.2 M-triangle depth-14 octree 0.70 s (1.61).  A triangle
+// takes 228 bytes of scratch with vertex attributes, 112 without, a column 4 and an
+// overlap 16: 1.0 GB at the peak for the icosphere, its pool among it (0.8 before),
+// 2.1 GB for a depth-12 terrain with a 1.2 GB pool (1.5).
 //
 // FP32 arithmetic uses explicit round-to-nearest intrinsics in the host
 // builder's operation order (the library is built with -fmad=false), so the

@@ -37,20 +37,29 @@ constexpr int kThreads = kBlockW * kBlockH;
 // the same code: only the order the blocks start in changes.
 //
 // The estimate is a chain of dependent node reads per ray, so its time grows
-// with the cap on its passes.  A ray at the cap counts for what its progress
-// says about the rest of its way through the root box, so that the long blocks
-// are told from one another (with the capped counts as they are, the 1920x1080
-// icosphere took 255 us against 226 us, as long as in raster order).  The cap
-// (us, 32 / 40 / 48 / 56 passes): 1920x1080 icospheres 236 / 224 / 229 / 243 and
-// 207 / 201 / 211 / 223, 2560x1440 372 / 353 / 357 / 361, a 1920x1080 terrain 202 /
-// 205 / 207 / 209.  One sample a block: 235 us against 226.  Sixteen of a warp's
-// lanes cast samples: with all 32 the paths of more cells diverge in each of a
-// warp's passes (248 against 241 us, 2560x1440 362 against 357).
+// with the cap on its passes, and a low cap ranks the blocks worse.  A ray at the
+// cap counts for what its progress says about the rest of its way through the root
+// box, so that the long blocks are told from one another (with the capped counts as
+// they are, the 1920x1080 icosphere took 255 us against 226 us, as long as in raster
+// order).  The cap (us, 32 / 40 / 48 / 56 passes, six views each):
+//   depth-9 icosphere   1280x1024 140 / 143 / 146 / 149  1920x1080 155 / 158 / 161 / 164
+//   depth-11 icosphere  1280x1024 180 / 173 / 175 / 177  1920x1080 196 / 194 / 198 / 203
+//   the same, near      1920x1080 255 / 249 / 249 / 252
+//   depth-10 terrain    1280x1024 161 / 162 / 163 / 165  1920x1080 218 / 222 / 224 / 227
+//   depth-12 terrain    1280x1024 182 / 183 / 185 / 188  1920x1080 247 / 252 / 255 / 258
+// so 40 is the lowest that ranks the deep icosphere's blocks, for about 1.5 % of a
+// terrain.  Measured with the loop before the present one: one sample a block 235 us
+// against 226; all 32 of a warp's lanes casting samples instead of 16 (the paths of
+// more cells diverge in each of its passes) 248 against 241 us.
 //
-// The line: the tail that the order removes is a few long rays, so it does not
-// grow with the frame, while the estimate is a share of it.  At 1280x720 the two
-// orders are equal (102 us); at 3840x2160 an icosphere took 761 us either way and
-// a terrain 857 us ordered, 801 us in raster order.
+// The lines: the tail that the order removes is a few long rays, so it does not
+// grow with the frame, while the estimate is a share of it.  In raster order and
+// ordered (us): the depth-11 icosphere 1024x768 148 / 140, 1280x1024 192 / 173,
+// 1920x1080 215 / 194, 2560x1440 366 / 318, 3840x2160 653 / 636; the depth-9 one 113 /
+// 107, 153 / 143, 170 / 158, 252 / 250, 473 / 513; the depth-12 terrain 109 / 124,
+// 162 / 184, 238 / 252, 416 / 436, 918 / 969.  A terrain has no such tail and is
+// faster in raster order throughout, by 5 to 14 %; what a frame will show is not
+// known before it is cast.
 constexpr uint32_t kCostCap = 40;  // passes of an estimate ray
 constexpr uint32_t kCostBuckets = 49;
 constexpr uint32_t kCostTop = kCostBuckets - 1;
@@ -549,15 +558,15 @@ int launch_render_shadow(const svo_node* nodes, const svo_attrib* attribs, uint6
   if (p.height > 0xFFFFFFF0u) return SVO_ERR_RANGE;  // row indices stay below 2^32
   const uint2* n2 = reinterpret_cast<const uint2*>(nodes);
   const uint2* a2 = reinterpret_cast<const uint2*>(attribs);
-  // One pass in raster order: ordering by primary-ray cost made the
-  // 3840x2160 shadow frame slower (2.02 against 1.79 ms), the shadow rays'
-  // cost being unknown to the estimate and neighbouring blocks no longer
-  // sharing the caches.  Two passes (the primary rays longest first, each
-  // hit appended to a job list, then one shadow ray per job in full warps)
-  // were slower still: 2.22 against 1.79 ms, and 0.626 against 0.529 ms at
-  // 1920x1080, where the shadow pass alone took 330 us for 504 k rays.  A
-  // shadow ray cast right after its primary ray finds the nodes of its
-  // descent in L1; cast in a later pass it reads them from L2 again.
+  // One pass in raster order.  Measured with the loop of one event a pass (a
+  // 3840x2160 frame 1.79 ms, 1.07 to 1.21 with the present one): ordered by
+  // primary-ray cost 2.02 ms, the shadow rays' cost being unknown to the estimate
+  // and neighbouring blocks no longer sharing the caches; in two passes (the primary
+  // rays longest first, each hit appended to a job list, then one shadow ray per
+  // job in full warps) 2.22 ms, and 0.626 against 0.529 ms at 1920x1080, where the
+  // shadow pass alone took 330 us for 504 k rays.  A shadow ray cast right after its
+  // primary ray finds the nodes of its descent in L1; cast in a later pass it reads
+  // them from L2 again.
   const uint32_t gx = (p.width + kBlockW - 1) / kBlockW;
   const uint32_t rays = rays_per_warp((uint64_t)p.width * p.height), block_h = kBlockH / 4 * rays / 8;
   return for_each_band(p.height, block_h, [&](uint32_t y0, uint32_t, uint32_t gy) -> int {
@@ -632,8 +641,10 @@ int launch_trace_rays(const svo_node* nodes, uint64_t num_nodes, const float* or
                       const float* dirs, uint64_t n, float tsr, const svo_trace_cfg& cfg,
                       svo_hit* hits, svo_stats* stats, cudaStream_t stream) {
   if (n == 0) return SVO_OK;
-  // (us, 32 / 16 / 8 lanes: 1,000 rays over a depth-10 icosphere 50.5 / 47.8 /
-  // 44.4, 8,000 62.0 / 60.1 / 56.7, 30,000 71.7 / 68.9 / 72.5, 50,000 78 / 85 / 94)
+  // (us, 32 / 16 / 8 lanes, rays without order over the depth-11 icosphere: 1,000
+  // rays 62 / 60 / 56, 8,000 72 / 61 / 58, 16,000 75 / 69 / 69, 30,000 79 / 77 / 85,
+  // 50,000 93 / 84 / 102; over a depth-9 terrain 40 / 36 / 35, 50 / 44 / 44, 50 / 48 /
+  // 49, 54 / 50 / 55, 56 / 57 / 73)
   const uint32_t rays = n <= (1u << 15) ? rays_per_warp(n) : 32u;
   const uint64_t per_block = kThreads / 32 * rays, blocks = (n + per_block - 1) / per_block;
   if (blocks > 0x7FFFFFFFull) return SVO_ERR_RANGE;

@@ -13,9 +13,12 @@ size_t render_smem_bytes(int stack_size);
 // Rays of one warp in a frame, an analysis pass or a set of rays.  A set too
 // small to fill the GPU takes as long as its slowest warp, and a warp with fewer
 // rays takes fewer of the loop's paths in each pass, so it is cast with 8 or 16
-// of a warp's lanes (us, 32 / 16 / 8 lanes): 64x64 icosphere 19.1 / 17.8 / 17.4,
-// with shadow rays 53.3 / 50.5 / 47.1; 128x128 25.9 / 25.3 / 24.6 and 61.5 / 57.7
-// / 52.7; 192x192 34.1 / 32.8 / 34.3; 256x256 39.3 / 41.7 / 46.8.
+// of a warp's lanes (us, 32 / 16 / 8 lanes, eight views each): a depth-11 icosphere
+// 64x64 22.9 / 22.4 / 21.1, with shadow rays 77 / 71 / 63; 128x128 33.6 / 32.4 / 31.1
+// and 105 / 98 / 89; 160x160 40.0 / 38.5 / 38.2; 192x192 43.6 / 42.3 / 44.9 and 110 /
+// 105 / 107; 224x224 47.7 / 47.6 / 50.3; 256x256 55.7 / 55.2 / 62.2 and 125 / 122 /
+// 131; a depth-9 terrain 128x128 25.5 / 24.7 / 24.4, 192x192 32.1 / 31.4 / 33.1,
+// 224x224 33.3 / 33.9 / 37.3.
 inline uint32_t rays_per_warp(uint64_t rays) {
   return rays <= (1u << 14) ? 8u : (rays <= (3u << 14) ? 16u : 32u);
 }
